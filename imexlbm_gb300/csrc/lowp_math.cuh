@@ -140,9 +140,13 @@ struct Storage<IMEX_F16DEV> {
     {
         return weight(a) + (double)__half2float(v) * (1.0 / kScale);
     }
+    // kScale is a power of two: scaling after the rounding to float32 gives
+    // the bits of scaling before it, and leaves the float64 pipe one
+    // operation less.  (A difference of float64 values near w is a multiple
+    // of 2^-61 or zero, far above float32's underflow.)
     static __device__ __forceinline__ __half from_f64(double f, int a)
     {
-        return __float2half_rn((float)((f - weight(a)) * kScale));
+        return __float2half_rn(__double2float_rn(f - weight(a)) * kScale);
     }
 };
 
