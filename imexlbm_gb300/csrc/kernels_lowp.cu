@@ -7,6 +7,7 @@
 
 #include <cuda_fp16.h>
 
+#include "conserved.cuh"
 #include "kernels_lowp.cuh"
 #include "lowp_math.cuh"
 #include "rows.cuh"
@@ -91,62 +92,6 @@ __global__ void __launch_bounds__(kStepBlock) k_to_f64(const typename Storage<P>
     const size_t cell = ((size_t)i * g.ny + j) * g.nz + k;
 #pragma unroll
     for (int a = 0; a < kQ; ++a) out[(size_t)a * g.plane + cell] = Storage<P>::to_f64(src[pi.at_dyn(g, a)], a);
-}
-
-// Partial sums of {mass, px, py, pz, ke} (src/lbm.cpp:271-294), one partial
-// per block.  A cell's moments are float32 sums of its deviations h (the
-// stored values' own precision: float32 f - w is exact, float16 values are
-// exact in float32), pair by pair as the collision forms them: mass =
-// 1 + sum h, momentum = sum h e (sum w = 1, sum w e = 0).  They become
-// float64 for the kinetic energy and the block and global sums.  Float64
-// arithmetic per value would make this reduction bound by the float64 pipe
-// (1.67 op/clk/SM): 5.2 ms at 256^3 instead of a fraction of a step.
-template <int P, bool PULL>
-__global__ void __launch_bounds__(kStepBlock) k_conserved_lowp(const typename Storage<P>::T* __restrict__ src, Geom g,
-                                                               double* __restrict__ partial)
-{
-    using A = lowp::F1;
-    __shared__ double smem[32 * 5];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
-    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (k < g.nz) {
-        const PullIndex pi(g, i, j, k, PULL);
-        float h[kQ];
-#pragma unroll
-        for (int a = 0; a < kQ; ++a) h[a] = Storage<P>::dev(src[pi.at_dyn(g, a)], a);
-        float d[kPairs + 1], sp[kPairs + 1];
-#pragma unroll
-        for (int q = 1; q <= kPairs; ++q) {
-            d[q] = A::sub(h[2 * q - 1], h[2 * q]);
-            sp[q] = A::add(h[2 * q - 1], h[2 * q]);
-        }
-        float sig = h[0];
-#pragma unroll
-        for (int q = 1; q <= kPairs; ++q) sig = A::add(sig, sp[q]);
-        float u[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int dim = 0; dim < 3; ++dim)
-#pragma unroll
-            for (int q = 1; q <= kPairs; ++q) {
-                const int e = ex(2 * q - 1, dim);
-                if (e == 1) u[dim] = A::add(u[dim], d[q]);
-                if (e == -1) u[dim] = A::sub(u[dim], d[q]);
-            }
-        constexpr double inv = 1.0 / Storage<P>::kScale;
-        const double ul = (double)u[0] * inv, vl = (double)u[1] * inv, wl = (double)u[2] * inv;
-        v[0] = 1.0 + (double)sig * inv;
-        v[1] = ul;
-        v[2] = vl;
-        v[3] = wl;
-        v[4] = 0.5 * (ul * ul + vl * vl + wl * wl);
-    }
-    block_sum<5>(v, smem);
-    if (threadIdx.x == 0) {
-        const size_t b = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-#pragma unroll
-        for (int q = 0; q < 5; ++q) partial[b * 5 + q] = v[q];
-    }
 }
 
 // Per-cell p, u, v, w in float64 from the stored values (src/lbm.cpp:218-236).
@@ -328,21 +273,16 @@ cudaError_t launch_macro_lowp(int prec, bool pull, const void* src, const Geom& 
     return cudaGetLastError();
 }
 
-cudaError_t launch_conserved_lowp(int prec, bool pull, const void* src, const Geom& g, double* partial, double* out,
-                                  cudaStream_t s)
+cudaError_t launch_conserved_lowp(int prec, bool pull, const void* src, const Geom& g, void* partial, unsigned* ticket,
+                                  double* out, cudaStream_t s)
 {
-    if (prec == IMEX_F32) {
-        const float* p = static_cast<const float*>(src);
-        if (pull) k_conserved_lowp<IMEX_F32, true><<<step_grid(g), kStepBlock, 0, s>>>(p, g, partial);
-        else k_conserved_lowp<IMEX_F32, false><<<step_grid(g), kStepBlock, 0, s>>>(p, g, partial);
-    } else {
-        const __half* p = static_cast<const __half*>(src);
-        if (pull) k_conserved_lowp<IMEX_F16DEV, true><<<step_grid(g), kStepBlock, 0, s>>>(p, g, partial);
-        else k_conserved_lowp<IMEX_F16DEV, false><<<step_grid(g), kStepBlock, 0, s>>>(p, g, partial);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return launch_reduce_partials(partial, conserved_partials(g), out, s);
+    return prec == IMEX_F32 ? cons::launch<IMEX_F32, 3>(pull, src, g, partial, ticket, out, s)
+                            : cons::launch<IMEX_F16DEV, 3>(pull, src, g, partial, ticket, out, s);
+}
+
+size_t conserved_scratch_bytes(const Geom& g)
+{
+    return cons::blocks_for((size_t)g.nx * g.ny * g.nz, current_sm_count(), cons::kMostPerSm) * sizeof(cons::Partial);
 }
 
 }  // namespace imex

@@ -39,7 +39,10 @@ cudaError_t launch_from_f64(int prec, const double* f, void* out, const Geom& g,
 cudaError_t launch_to_f64(int prec, bool pull, const void* src, const Geom& g, double* out, cudaStream_t s);
 cudaError_t launch_macro_lowp(int prec, bool pull, const void* src, const Geom& g, double* p, double* u, double* v,
                               double* w, cudaStream_t s);
-cudaError_t launch_conserved_lowp(int prec, bool pull, const void* src, const Geom& g, double* partial, double* out,
-                                  cudaStream_t s);
+// Conserved sums (conserved.cuh): partial holds conserved_scratch_bytes(),
+// *ticket is 0 before and after the launch.
+cudaError_t launch_conserved_lowp(int prec, bool pull, const void* src, const Geom& g, void* partial, unsigned* ticket,
+                                  double* out, cudaStream_t s);
+size_t conserved_scratch_bytes(const Geom& g);
 
 }  // namespace imex

@@ -503,10 +503,11 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaGetDevice"));
 
     const size_t arr = (size_t)kQ * h->ncells * elem_size(precision);
-    const size_t nparts = conserved_partials(h->g);
-    // scratch: conserved partials, 5 reduced values, fallback counter, error
-    // flag, fixed-point run flag
-    const size_t scratch = nparts * 5 * sizeof(double) + 5 * sizeof(double) + 3 * sizeof(unsigned long long);
+    // scratch: conserved partials (the native engine's: 5 doubles per
+    // 128-cell row segment), 5 reduced values, fallback counter, error flag,
+    // fixed-point run flag, the conserved kernel's ticket
+    const size_t parts = std::max(conserved_partials(h->g) * 5 * sizeof(double), conserved_scratch_bytes(h->g));
+    const size_t scratch = parts + 5 * sizeof(double) + 4 * sizeof(unsigned long long);
     const size_t need = 2 * arr + scratch;
     // Device memory comes from the device's stream-ordered pool: creating
     // and destroying lattices (a server does it per request) then neither
@@ -539,11 +540,12 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     }
     h->scratch = s;
     h->d_partial = reinterpret_cast<double*>(s);
-    h->d_out = h->d_partial + nparts * 5;
+    h->d_out = reinterpret_cast<double*>(s + parts);
     h->d_fallback = reinterpret_cast<unsigned long long*>(h->d_out + 5);
     h->d_err = reinterpret_cast<unsigned*>(h->d_fallback + 1);
     h->d_fail = reinterpret_cast<int*>(h->d_fallback + 2);
-    e = cudaMemsetAsync(h->d_fallback, 0, 3 * sizeof(unsigned long long), h->stream);
+    h->d_ticket = reinterpret_cast<unsigned*>(h->d_fallback + 3);
+    e = cudaMemsetAsync(h->d_fallback, 0, 4 * sizeof(unsigned long long), h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);  // usable from any stream from here on
     if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "imex_create"));
     h->bytes = need;
@@ -764,20 +766,28 @@ int imex_conserved(imex_lattice* h, double out[5])
     const bool pull = h->tag == kPendingStream;
     int timed = h->prof.start(IMEX_PHASE_CONSERVED, h->stream);
     cudaError_t e =
-        is_lowp(h) ? launch_conserved_lowp(h->precision, pull, h->buf[h->cur], h->g, h->d_partial, h->d_out, h->stream)
-        : use_fixed(h) ? launch_conserved_fx(pull, dbuf(h, h->cur), h->g, h->fx, h->d_partial, h->d_out, h->stream)
-                       : launch_conserved_f64(pull, dbuf(h, h->cur), h->g, h->d_partial, h->d_out, h->stream);
+        is_lowp(h) ? launch_conserved_lowp(h->precision, pull, h->buf[h->cur], h->g, h->d_partial, h->d_ticket, h->d_out,
+                                           h->stream)
+        : use_fixed(h)
+            ? launch_conserved_fx(pull, dbuf(h, h->cur), h->g, h->d_partial, h->d_ticket, h->d_out, h->stream)
+            : launch_conserved_f64(pull, dbuf(h, h->cur), h->g, h->d_partial, h->d_out, h->stream);
     h->prof.stop(timed, h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "conserved kernel launch");
-    h->launches += 2;
-    double res[5];
-    IMEX_CUDA(h, cudaMemcpyAsync(res, h->d_out, 5 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "cudaMemcpy");
+    h->launches += is_lowp(h) || use_fixed(h) ? 1 : 2;
+    // the 5 sums, the fallback counter and the error flag lie in a row: one copy
+    struct {
+        double sums[5];
+        unsigned long long fallback, err;
+    } res;
+    IMEX_CUDA(h, cudaMemcpyAsync(&res, h->d_out, sizeof res, cudaMemcpyDeviceToHost, h->stream), "cudaMemcpy");
     IMEX_CUDA(h, cudaStreamSynchronize(h->stream), "imex_conserved");
-    rc = check_kernel_error(h);
-    if (rc) return rc;
+    if (res.err) {
+        rc = check_kernel_error(h);  // reports it and clears the flag
+        if (rc) return rc;
+    }
     bool finite = true;
     for (int q = 0; q < 5; ++q) {
-        out[q] = res[q];
+        out[q] = res.sums[q];
         finite = finite && std::isfinite(out[q]);
     }
     if (!finite) return fail(h, IMEX_ERR_NONFINITE, "imex_conserved: non-finite diagnostics (the run diverged)");

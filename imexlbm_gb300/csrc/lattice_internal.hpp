@@ -37,8 +37,9 @@ struct imex_lattice {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     int device = 0;
-    unsigned char* scratch = nullptr;  // one allocation holding d_partial .. d_fail
-    double* d_partial = nullptr;  // conserved partials (5 per block)
+    unsigned char* scratch = nullptr;  // one allocation holding d_partial .. d_ticket
+    double* d_partial = nullptr;  // conserved partials
+    unsigned* d_ticket = nullptr;  // conserved kernel: blocks done (0 between launches)
     double* d_out = nullptr;      // 5 reduced values
     unsigned long long* d_fallback = nullptr;  // fixed-point engine fallback counter
     size_t bytes = 0;

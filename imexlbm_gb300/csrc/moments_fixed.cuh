@@ -1,0 +1,151 @@
+// A cell's mass and momentum as exact 64-bit fixed point (units of 2^-61),
+// for the diagnostics.  The float64 pipe issues 1.67 operations per clock
+// per SM against ~64 on the integer pipes, so moments formed and summed in
+// float64 bound every diagnostic; formed in integers they leave it idle.
+//
+//   float64 storage   the 27 values converted exactly (fx_math.cuh) and
+//                     summed exactly.
+//   reduced precision the deviations h = kScale (f - w) summed in float32,
+//                     pair by pair as the collision sums them; mass = 1 +
+//                     sum h, momentum = sum h e.  The float32 sums are
+//                     multiples of 2^-37 or more for stored values of the
+//                     weights' size, so their conversion drops nothing.
+//
+// Outside the range (|u| >= 1, 3p outside (0, 2), a float64 value not in
+// [2^-9, 1), NaN, Inf) `ok` is false and the caller uses moments_f64_of.
+#pragma once
+
+#include "fx_math.cuh"
+#include "imexlbm.h"
+#include "kernels_common.cuh"
+#include "lowp_math.cuh"
+
+namespace imex {
+namespace mom {
+
+constexpr int kBits = fx::kFrac;  // 61
+static_assert(kBits == 61, "the shifts below assume units of 2^-61");
+
+template <int P>
+struct Elem {
+    using T = typename lowp::Storage<P>::T;
+    static constexpr int kScaleLog2 = P == IMEX_F16DEV ? 12 : 0;
+    static_assert(lowp::Storage<P>::kScale == (float)(1 << kScaleLog2), "kScale is 2^kScaleLog2");
+};
+template <>
+struct Elem<IMEX_F64> {
+    using T = double;
+};
+
+// x / 2^S in units of 2^-61, bits below dropped; clears ok for |x| >= 2^S
+// (NaN and Inf included).
+template <int S>
+__device__ __forceinline__ int64_t fixed_of_float(float x, bool& ok)
+{
+    const uint32_t b = __float_as_uint(x);
+    const int e = (int)((b >> 23) & 255u);
+    ok = ok && e <= 126 + S;
+    // mantissa * 2^(e - 150) * 2^61 / 2^S = (mantissa << 37) >> (126 + S - e)
+    const int sh = 126 + S - e;
+    const uint64_t v = ((uint64_t)((b & 0x007FFFFFu) | 0x00800000u) << 37) >> (sh < 63 ? sh : 63);
+    return (b >> 31) ? -(int64_t)v : (int64_t)v;
+}
+
+// One cell: M = {3p, u, v, w} 2^61 and u, v, w again as numbers in units of
+// 2^-kVelBits<P> (vel), the form whose squares make the kinetic energy.
+template <int P>
+struct Cell {
+    int64_t M[4];
+    double vel[3];
+};
+template <int P>
+inline constexpr int kVelBits = P == IMEX_F64 ? kBits : P == IMEX_F16DEV ? 12 : 0;
+
+template <int P, bool VEL>
+__device__ __forceinline__ bool moments(const typename Elem<P>::T* __restrict__ src, const Geom& g, const PullIndex& pi,
+                                        Cell<P>& c)
+{
+    bool ok = true;
+    if constexpr (P == IMEX_F64) {
+        double f[kQ];
+        gather27<double>(src, g, pi, f);
+        uint64_t S = 0, A[3] = {0, 0, 0}, B[3] = {0, 0, 0};
+#pragma unroll
+        for (int a = 0; a < kQ; ++a) {  // f_0 < 1, others < 1/8: every sum below 2^64
+            const uint64_t X = fx::to_fixed(f[a], a == 0 ? 8u : 5u, ok);
+            S += X;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                if (ex(a, d) == 1) A[d] += X;
+                if (ex(a, d) == -1) B[d] += X;
+            }
+        }
+        ok = ok && (S >> 62) == 0;
+        c.M[0] = (int64_t)S;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            c.M[1 + d] = (int64_t)(A[d] - B[d]);
+            if (VEL) c.vel[d] = __ll2double_rn(c.M[1 + d]);
+        }
+    } else {
+        using A = lowp::F1;
+        constexpr int S = Elem<P>::kScaleLog2;
+        float h[kQ];
+#pragma unroll
+        for (int a = 0; a < kQ; ++a) h[a] = lowp::Storage<P>::dev(src[pi.at_dyn(g, a)], a);
+        float d[kPairs + 1], sig = h[0];
+#pragma unroll
+        for (int q = 1; q <= kPairs; ++q) {
+            d[q] = A::sub(h[2 * q - 1], h[2 * q]);
+            sig = A::add(sig, A::add(h[2 * q - 1], h[2 * q]));
+        }
+        c.M[0] = (int64_t)(1ull << kBits) + fixed_of_float<S>(sig, ok);
+#pragma unroll
+        for (int dim = 0; dim < 3; ++dim) {
+            float u = 0.f;
+#pragma unroll
+            for (int q = 1; q <= kPairs; ++q) {
+                const int e = ex(2 * q - 1, dim);
+                if (e == 1) u = A::add(u, d[q]);
+                if (e == -1) u = A::sub(u, d[q]);
+            }
+            c.M[1 + dim] = fixed_of_float<S>(u, ok);
+            if (VEL) c.vel[dim] = (double)u;
+        }
+    }
+    return ok;
+}
+
+// The same moments in float64, for a cell outside the range.
+template <int P>
+__device__ __noinline__ void moments_f64_of(const typename Elem<P>::T* src, Geom g, int i, int j, int k, bool pull,
+                                            double* out)
+{
+    const PullIndex pi(g, i, j, k, pull);
+    for (int q = 0; q < 4; ++q) out[q] = 0.0;
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+        double f;
+        if constexpr (P == IMEX_F64) f = src[pi.at_dyn(g, a)];
+        else f = lowp::Storage<P>::to_f64(src[pi.at_dyn(g, a)], a);
+        out[0] += f;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (ex(a, d) == 1) out[1 + d] += f;
+            if (ex(a, d) == -1) out[1 + d] -= f;
+        }
+    }
+}
+
+// (x, y, z) of a flat cell index (z fastest); lattices in device memory
+// hold fewer than 2^32 cells.
+__device__ __forceinline__ void cell_of(const Geom& g, unsigned idx, int& i, int& j, int& k)
+{
+    const unsigned row = idx / (unsigned)g.nz;
+    k = (int)(idx - row * (unsigned)g.nz);
+    i = (int)(row / (unsigned)g.ny);
+    j = (int)(row - (unsigned)i * (unsigned)g.ny);
+}
+
+}  // namespace mom
+}  // namespace imex
