@@ -72,26 +72,53 @@ __global__ void __launch_bounds__(kStepBlock) k_init_lowp(typename Storage<P>::T
     for (int a = 0; a < kQ; ++a) f[(size_t)a * g.plane + cell] = Storage<P>::from_f64(fe[a], a);
 }
 
-// Conversions between float64 reference-order f and the storage format.
+// Conversions between float64 reference-order f and the storage format,
+// bound by memory (10 or 12 bytes a value).  From float64: one direction per
+// grid row, so its weight is uniform over the CTA and no thread divides by
+// the plane's size.
+constexpr int kConvThreads = 256, kConvPer = 4;
 template <int P>
-__global__ void k_from_f64(const double* __restrict__ f, typename Storage<P>::T* __restrict__ out, size_t plane)
+__global__ void __launch_bounds__(kConvThreads) k_from_f64(const double* __restrict__ f,
+                                                           typename Storage<P>::T* __restrict__ out, size_t plane)
 {
-    const size_t n = (size_t)kQ * plane;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-        out[q] = Storage<P>::from_f64(f[q], (int)(q / plane));
+    const int a = blockIdx.y;
+    f += (size_t)a * plane;
+    out += (size_t)a * plane;
+    const size_t q0 = (size_t)blockIdx.x * (kConvThreads * kConvPer) + threadIdx.x;
+    double v[kConvPer];
+#pragma unroll
+    for (int c = 0; c < kConvPer; ++c) v[c] = q0 + c * kConvThreads < plane ? __ldg(f + q0 + c * kConvThreads) : 1.0;
+#pragma unroll
+    for (int c = 0; c < kConvPer; ++c)
+        if (q0 + c * kConvThreads < plane) out[q0 + c * kConvThreads] = Storage<P>::from_f64(v[c], a);
 }
 
-template <int P, bool PULL>
-__global__ void __launch_bounds__(kStepBlock) k_to_f64(const typename Storage<P>::T* __restrict__ src, Geom g,
-                                                       double* __restrict__ out)
+// One cell again in float64, for values off the exact integer grid.
+template <int P>
+__device__ __noinline__ void to_f64_cell_wide(const typename Storage<P>::T* src, Geom g, int i, int j, int k, bool pull,
+                                              unsigned cell, double* out)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
-    if (k >= g.nz) return;
-    const PullIndex pi(g, i, j, k, PULL);
-    const size_t cell = ((size_t)i * g.ny + j) * g.nz + k;
+    const PullIndex pi(g, i, j, k, pull);
 #pragma unroll
     for (int a = 0; a < kQ; ++a) out[(size_t)a * g.plane + cell] = Storage<P>::to_f64(src[pi.at_dyn(g, a)], a);
+}
+
+// To float64: a thread per cell in flat order (a row's end leaves no thread
+// idle), pulling through a pending streaming.
+template <int P, bool PULL>
+__global__ void __launch_bounds__(kStepBlock) k_to_f64(const typename Storage<P>::T* __restrict__ src, Geom g,
+                                                         unsigned cells, double* __restrict__ out)
+{
+    const unsigned cell = blockIdx.x * kStepBlock + threadIdx.x;
+    if (cell >= cells) return;
+    int i, j, k;
+    mom::cell_of(g, cell, i, j, k);
+    const PullIndex pi(g, i, j, k, PULL);
+    bool ok = true;
+#pragma unroll
+    for (int a = 0; a < kQ; ++a)
+        out[(size_t)a * g.plane + cell] = Storage<P>::to_f64_exact(__ldg(src + pi.at_dyn(g, a)), a, ok);
+    if (!ok) to_f64_cell_wide<P>(src, g, i, j, k, PULL, cell, out);
 }
 
 // Per-cell p, u, v, w in float64 from the stored values (src/lbm.cpp:218-236).
@@ -236,24 +263,26 @@ size_t rows_lowp_stage_bytes(int prec, int nz) { return (size_t)kQ * nz * (prec 
 
 cudaError_t launch_from_f64(int prec, const double* f, void* out, const Geom& g, cudaStream_t s)
 {
-    const int blocks = current_sm_count() * 8;
+    const dim3 grid((unsigned)((g.plane + kConvThreads * kConvPer - 1) / (kConvThreads * kConvPer)), kQ);
     if (prec == IMEX_F32)
-        k_from_f64<IMEX_F32><<<blocks, 256, 0, s>>>(f, static_cast<float*>(out), g.plane);
+        k_from_f64<IMEX_F32><<<grid, kConvThreads, 0, s>>>(f, static_cast<float*>(out), g.plane);
     else
-        k_from_f64<IMEX_F16DEV><<<blocks, 256, 0, s>>>(f, static_cast<__half*>(out), g.plane);
+        k_from_f64<IMEX_F16DEV><<<grid, kConvThreads, 0, s>>>(f, static_cast<__half*>(out), g.plane);
     return cudaGetLastError();
 }
 
 cudaError_t launch_to_f64(int prec, bool pull, const void* src, const Geom& g, double* out, cudaStream_t s)
 {
+    if (g.plane > 0xffffffffull - kStepBlock) return cudaErrorInvalidValue;  // above device memory
+    const unsigned cells = (unsigned)g.plane, grid = (cells + kStepBlock - 1) / kStepBlock;
     if (prec == IMEX_F32) {
         const float* p = static_cast<const float*>(src);
-        if (pull) k_to_f64<IMEX_F32, true><<<step_grid(g), kStepBlock, 0, s>>>(p, g, out);
-        else k_to_f64<IMEX_F32, false><<<step_grid(g), kStepBlock, 0, s>>>(p, g, out);
+        if (pull) k_to_f64<IMEX_F32, true><<<grid, kStepBlock, 0, s>>>(p, g, cells, out);
+        else k_to_f64<IMEX_F32, false><<<grid, kStepBlock, 0, s>>>(p, g, cells, out);
     } else {
         const __half* p = static_cast<const __half*>(src);
-        if (pull) k_to_f64<IMEX_F16DEV, true><<<step_grid(g), kStepBlock, 0, s>>>(p, g, out);
-        else k_to_f64<IMEX_F16DEV, false><<<step_grid(g), kStepBlock, 0, s>>>(p, g, out);
+        if (pull) k_to_f64<IMEX_F16DEV, true><<<grid, kStepBlock, 0, s>>>(p, g, cells, out);
+        else k_to_f64<IMEX_F16DEV, false><<<grid, kStepBlock, 0, s>>>(p, g, cells, out);
     }
     return cudaGetLastError();
 }

@@ -31,6 +31,7 @@
 #include <cuda_fp16.h>
 
 #include "d3q27.cuh"
+#include "fx_math.cuh"
 #include "imexlbm.h"
 #include "kernels_lowp.cuh"
 
@@ -39,6 +40,32 @@ namespace lowp {
 
 template <int P>
 struct Storage;
+
+// Weight class of direction a by its place in the direction order: rest,
+// axis, face diagonal, corner.  A few instructions where a is uniform but not
+// a compile-time constant (weight216 walks the direction table there, which
+// held the float16 conversion from float64 at 3.7 ms per 256^3 lattice).
+__host__ __device__ __forceinline__ constexpr int weight_class(int a) { return (a > 0) + (a > 6) + (a > 18); }
+__host__ __device__ __forceinline__ constexpr double class_weight(int c)
+{
+    return c == 0 ? 8.0 / 27.0 : c == 1 ? 2.0 / 27.0 : c == 2 ? 1.0 / 54.0 : 1.0 / 216.0;
+}
+// weight(a) 2^61, an integer: the weights are float64 values above 2^-8.
+__host__ __device__ __forceinline__ constexpr uint64_t weight_fixed(int a)
+{
+    const int c = weight_class(a);
+    return c == 0 ? (uint64_t)(8.0 / 27.0 * 0x1p61)
+         : c == 1 ? (uint64_t)(2.0 / 27.0 * 0x1p61)
+         : c == 2 ? (uint64_t)(1.0 / 54.0 * 0x1p61)
+                  : (uint64_t)(1.0 / 216.0 * 0x1p61);
+}
+constexpr bool weight_classes_ok()
+{
+    for (int a = 0; a < kQ; ++a)
+        if (class_weight(weight_class(a)) != weight(a)) return false;
+    return true;
+}
+static_assert(weight_classes_ok(), "weight_class follows the direction order");
 
 // 32-bit hash of (cell index, step seed) for stochastic rounding: the
 // murmur3 finaliser of their combination.
@@ -125,6 +152,7 @@ struct Storage<IMEX_F32> {
     static __device__ __forceinline__ float dev(float v, int a) { return v - (float)weight(a); }
     static __device__ __forceinline__ float store(float h, int a) { return (float)weight(a) + h; }
     static __device__ __forceinline__ double to_f64(float v, int) { return (double)v; }
+    static __device__ __forceinline__ double to_f64_exact(float v, int, bool&) { return (double)v; }
     static __device__ __forceinline__ float from_f64(double f, int) { return __double2float_rn(f); }
 };
 
@@ -136,18 +164,61 @@ struct Storage<IMEX_F16DEV> {
     static __device__ __forceinline__ float load_plain(const __half* p, int) { return __half2float(*p); }
     static __device__ __forceinline__ float dev(__half v, int) { return __half2float(v); }
     static __device__ __forceinline__ __half store(float h, int) { return __float2half_rn(h); }
+    // Conversions between the stored value and f: weight(a) + v / 2^12
+    // rounded once to float64, and float16(float32(f - weight(a)) 2^12).  In
+    // float64 arithmetic they took 1.67 ms (two operations a value on a pipe
+    // of 1.67 a clock and SM) and 3.66 ms per 256^3 lattice; in integers, on
+    // the exact grid of fx_math.cuh, 1.09 and 1.11 (memory alone: 0.68), and
+    // the initialisation that ends in the second fell from 3.54 to 2.49.
+    // Values off the grid (f outside [2^-9, 1), |f - w| >= 1, NaN, Inf)
+    // clear ok and go through float64, a cell at a time or out of line: with
+    // the float64 form inline the compiler computes it for every value.
+    static __device__ __forceinline__ double to_f64_exact(__half v, int a, bool& ok)
+    {
+        const float x = __half2float(v);
+        const uint32_t b = __float_as_uint(x);
+        const uint32_t e = (b >> 23) & 255u;
+        // x 2^49 = (mantissa << 37) >> (138 - e), exact: a float16 is a multiple of 2^-24
+        const uint32_t sh = 138u - e;
+        const uint64_t m = ((uint64_t)((b & 0x007FFFFFu) | 0x00800000u) << 37) >> (sh < 63u ? sh : 63u);
+        const uint64_t X = weight_fixed(a) + ((b >> 31) ? 0ull - m : m);
+        const uint32_t hi = (uint32_t)(X >> 32), r = 11u - fx::clz32(hi);  // bits below the 53-bit mantissa
+        ok = ok && e <= 138u && r <= 10u;
+        // to nearest, ties to even, as the float64 addition rounds
+        const uint32_t odd = (uint32_t)(X >> r) & 1u;
+        const uint64_t t = X + ((fx::fshl(0u, 1u, r) >> 1) + odd) - (r ? 1u : odd);
+        const uint32_t tl = (uint32_t)t, th = (uint32_t)(t >> 32);
+        return fx::double_of(fx::fshr(th, 0u, r) + (r << 20) + fx::kOutExp, fx::fshr(tl, th, r));
+    }
     static __device__ __forceinline__ double to_f64(__half v, int a)
     {
-        return weight(a) + (double)__half2float(v) * (1.0 / kScale);
+        bool ok = true;
+        const double d = to_f64_exact(v, a, ok);
+        return ok ? d : to_f64_wide(__half2float(v), class_weight(weight_class(a)));
     }
-    // kScale is a power of two: scaling after the rounding to float32 gives
-    // the bits of scaling before it, and leaves the float64 pipe one
-    // operation less.  (A difference of float64 values near w is a multiple
-    // of 2^-61 or zero, far above float32's underflow.)
+    // Scaling by the power of two after the rounding to float32 gives the
+    // bits of scaling before it.  f - w is exact in float64 for f in [w / 2,
+    // 2 w] (Sterbenz), so there the exact integer difference is rounded to
+    // float32 directly.
     static __device__ __forceinline__ __half from_f64(double f, int a)
     {
-        return __float2half_rn(__double2float_rn(f - weight(a)) * kScale);
+        bool ok = true;
+        const uint64_t X = fx::to_fixed(f, 8u, ok), W = weight_fixed(a);
+        ok = ok && X - (W >> 1) <= W + (W >> 1);
+        if (!ok) return __float2half_rn(from_f64_wide(f, class_weight(weight_class(a))));
+        const uint64_t D = X - W, mag = (long long)D < 0 ? 0ull - D : D;
+        // float32 of mag: its top 32 bits with the rest as a sticky bit round
+        // as all 64 would; the shift and the scale 2^-49 go into the exponent
+        const int lz = __clzll((long long)mag);
+        const uint64_t n = mag << (lz & 63);
+        const float m = __uint2float_rn((uint32_t)(n >> 32) | ((uint32_t)n != 0u ? 1u : 0u));
+        const uint32_t bits = mag ? __float_as_uint(m) + ((uint32_t)(32 - 49 - lz) << 23) : 0u;
+        return __float2half_rn(__uint_as_float(bits | ((uint32_t)(D >> 32) & 0x80000000u)));
     }
+    // The float64 forms, out of line: inlined, the compiler computes both
+    // sides of the choice for every value and the float64 pipe binds again.
+    static __device__ __noinline__ double to_f64_wide(float x, double w) { return w + (double)x * (1.0 / kScale); }
+    static __device__ __noinline__ float from_f64_wide(double f, double w) { return __double2float_rn(f - w) * kScale; }
 };
 
 // Arithmetic of one float32 lane (float) or of two cells in lock step
