@@ -721,6 +721,33 @@ int step_fixed_run(imex_lattice* h, int n)
     return step_each(h, n - failed + 1);
 }
 
+// Whether the fused steps of imex_step go two per launch: a float32 lattice
+// large enough (two::worth_alone), unless a launch shape is pinned or the
+// per-phase timer counts single steps.
+bool use_pairs(imex_lattice* h)
+{
+    if (h->precision != IMEX_F32 || h->shape_pinned || h->prof.enabled()) return false;
+    if (h->pairs_worth < 0) h->pairs_worth = two::worth_alone(h->g, current_sm_count());
+    return h->pairs_worth != 0;
+}
+
+// n / 2 launches of two fused float32 steps each, from the steady state.
+int step_pairs(imex_lattice* h, int n)
+{
+    if (!h->pairs)
+        IMEX_CUDA(h, two::make_lattice(static_cast<float*>(h->buf[0]), static_cast<float*>(h->buf[1]), h->g, &h->pairs),
+                  "two-step kernel set-up");
+    for (int s = 0; s + 2 <= n; s += 2) {
+        IMEX_CUDA(h, two::launch(*h->pairs, h->cur, static_cast<const float*>(h->buf[h->cur]),
+                                 static_cast<float*>(h->buf[1 - h->cur]), h->g, h->cf32, h->d_err, h->stream),
+                  "step kernel launch");
+        ++h->launches;
+        h->cur = 1 - h->cur;
+        h->steps += 2;
+    }
+    return IMEX_OK;
+}
+
 bool capturing(imex_lattice* h)
 {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -754,6 +781,16 @@ int imex_step(imex_lattice* h, int nsteps)
             }
             return step_fixed_run(h, nsteps);
         }
+    }
+    if (use_pairs(h) && nsteps >= 3) {
+        if (h->tag != kPendingStream) {
+            rc = step_each(h, 1);
+            if (rc) return rc;
+            --nsteps;
+        }
+        rc = step_pairs(h, nsteps);
+        if (rc) return rc;
+        nsteps &= 1;
     }
     return step_each(h, nsteps);
 }

@@ -12,6 +12,7 @@
 #include "kernels_lowp.cuh"
 #include "phase_timer.hpp"
 #include "rows.cuh"
+#include "two_f32.hpp"
 
 using imex::CollideF32;
 using imex::CollideF64;
@@ -62,6 +63,8 @@ struct imex_lattice {
     RowConfig rows{};           // launch shape of the fused step (stages 0: one thread per cell)
     int shape_mode = -1;        // -1 autotune on first use, 0 one thread per cell, 1 row-staged
     bool shape_pinned = false;  // shape set by imex_set_launch rather than the autotuner
+    imex::two::LatticePtr pairs;  // two float32 steps per launch (two_f32.hpp), made on first use
+    int pairs_worth = -1;         // whether they pay for this lattice alone (-1: not asked yet)
     imex::PhaseTimer prof;      // per-phase device time (imex_profile_*)
     std::string err;
 };

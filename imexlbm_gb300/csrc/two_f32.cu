@@ -1,0 +1,152 @@
+// Two float32 steps per launch (two_f32.cuh): plans, tensor maps and the
+// one-lattice kernel.
+#include <algorithm>
+#include <atomic>
+#include <new>
+
+#include "two_f32.cuh"
+#include "two_f32.hpp"
+
+namespace imex {
+namespace two {
+
+namespace {
+
+__global__ void __launch_bounds__(kThreads, 1)
+    k_two_f32(const __grid_constant__ Maps maps, const float* __restrict__ src, float* __restrict__ dst, Geom g, Plan p,
+              CollideF32 cp, WaitCtl wc)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    run_box(&maps, src, dst, g.nx, g.ny, g.nz, g.plane, box_of(p, g.nx, g.ny, g.nz, blockIdx.x), cp, smem, wc);
+}
+
+using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                            const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                            CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// cuTensorMapEncodeTiled of the driver, through the runtime (the library
+// links no driver library).
+Encode encode_fn()
+{
+    static std::atomic<void*> fn{nullptr};
+    void* f = fn.load();
+    if (!f) {
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        fn.store(f);
+    }
+    return reinterpret_cast<Encode>(f);
+}
+
+// Iterations a CTA spends beside its planes: the pipeline's 3 and the set-up.
+constexpr int kExtra = 5;
+
+// Iterations of the busiest SM (one CTA each at a time).
+long long iterations(const Geom& g, const Plan& p, int sms)
+{
+    return ((long long)p.nty * p.ntz * p.chunks + sms - 1) / sms * ((g.nx + p.chunks - 1) / p.chunks + kExtra);
+}
+
+Plan tiles_of(const Geom& g)
+{
+    Plan p;
+    p.ntz = (g.nz + kTileZ - 1) / kTileZ;
+    p.tz = ((g.nz + p.ntz - 1) / p.ntz + 3) / 4 * 4;  // tiles start on 16-byte boundaries
+    p.ntz = (g.nz + p.tz - 1) / p.tz;
+    p.nty = (g.ny + kTileY - 1) / kTileY;
+    p.ty = (g.ny + p.nty - 1) / p.nty;
+    p.chunks = 1;
+    return p;
+}
+
+}  // namespace
+
+bool eligible(const Geom& g)
+{
+    return g.nz % 4 == 0 && g.nz >= kTileZ && g.ny >= 4 && g.nx >= 4 && g.plane < (1ull << 32) / kQ;
+}
+
+Plan plan_for(const Geom& g, int sms)
+{
+    Plan p = tiles_of(g);
+    Plan best = p;
+    for (p.chunks = 2; p.chunks <= g.nx; ++p.chunks)
+        if (iterations(g, p, sms) < iterations(g, best, sms)) best = p;
+    return best;
+}
+
+Plan plan_tiles(const Geom& g, int planes)
+{
+    Plan p = tiles_of(g);
+    p.chunks = std::max(1, (g.nx + planes / 2) / planes);
+    return p;
+}
+
+// Measured: a launch takes 4 us and 1.85 us per iteration of its busiest SM
+// (64^3 26 us, 96^3 51, 128^3 113, 256^3 703), two launches of the one-step
+// kernel 2 (2 us + cells / 29 per ns) (64^3 21 us, 96^3 66, 128^3 141, 256^3
+// 1053).  So small lattices, whose tiles leave SMs idle or spend most
+// iterations filling the pipeline, and shapes that fit the tiles badly keep one step per
+// launch; the line lies near 80^3.
+bool worth_alone(const Geom& g, int sms)
+{
+    if (!eligible(g)) return false;
+    const double pair = 4.0 + 1.85 * (double)iterations(g, plan_for(g, sms), sms);
+    const double singles = 2.0 * (2.0 + (double)g.plane / 29000.0);
+    return pair < 0.97 * singles;
+}
+
+cudaError_t encode_maps(const float* buf, const Geom& g, const Plan& p, Maps* out)
+{
+    const Encode f = encode_fn();
+    if (!f) return cudaErrorNotSupported;
+    const cuuint64_t dims[3] = {(cuuint64_t)g.nz, (cuuint64_t)g.ny, (cuuint64_t)kQ * g.nx};
+    const cuuint64_t strides[2] = {(cuuint64_t)g.nz * 4, (cuuint64_t)g.nz * g.ny * 4};
+    const cuuint32_t step[3] = {1, 1, 1};
+    for (int q = 0; q < kMaps; ++q) {
+        // fewer rows than one: never used, a valid box all the same
+        const cuuint32_t box[3] = {(cuuint32_t)kTileZ, (cuuint32_t)std::max(1, p.ty + 2 - q), 1};
+        if (f(&out->m[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(buf), dims, strides, box, step,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t allow_smem(const void* kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+}
+
+struct Lattice {
+    Plan plan;
+    Maps maps[2];
+};
+
+void LatticeDelete::operator()(Lattice* p) const { delete p; }
+
+cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, LatticePtr* out)
+{
+    LatticePtr l(new (std::nothrow) Lattice);
+    if (!l) return cudaErrorMemoryAllocation;
+    l->plan = plan_for(g, current_sm_count());
+    cudaError_t e = encode_maps(buf0, g, l->plan, &l->maps[0]);
+    if (e == cudaSuccess) e = encode_maps(buf1, g, l->plan, &l->maps[1]);
+    if (e == cudaSuccess) e = allow_smem((const void*)k_two_f32);
+    if (e == cudaSuccess) *out = std::move(l);
+    return e;
+}
+
+cudaError_t launch(const Lattice& l, int from, const float* src, float* dst, const Geom& g, const CollideF32& cp,
+                   unsigned* err, cudaStream_t s)
+{
+    const unsigned grid = (unsigned)(l.plan.nty * l.plan.ntz * l.plan.chunks);
+    k_two_f32<<<grid, kThreads, kSmemBytes, s>>>(l.maps[from], src, dst, g, l.plan, cp, make_wait_ctl(err));
+    return cudaGetLastError();
+}
+
+}  // namespace two
+}  // namespace imex
