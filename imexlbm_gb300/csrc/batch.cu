@@ -28,6 +28,13 @@
 // Items of members whose step count for the tick is exhausted are armed
 // with no bytes and skipped, keeping the ring's phases uniform.
 //
+// Float32 members whose rows suit tensor copies step twice per launch in a
+// third kernel, the batched form of two_f32.cuh, when the batch holds enough
+// of them to fill the GPU with its tiles (pick_pairs).  At step s = 0, 2, ..
+// of a tick they read buf[cur ^ (s / 2 & 1)] and write the other buffer; a
+// member with an odd number of steps takes the last one in the cell kernel's
+// one-CTA-per-segment form after the tick.
+//
 // Launch shapes (cell kernel: threads per CTA, cells per thread, CTAs per
 // SM; row kernel: stages, stage size, CTAs per SM) are chosen by an
 // autotuner that times each candidate on the batch itself; timing writes
@@ -45,12 +52,14 @@
 #include "lattice_internal.hpp"
 #include "lowp_math.cuh"
 #include "rows_lowp.cuh"
+#include "two_f32.cuh"
 
 namespace imex {
 
 namespace {
 
 constexpr int kBatchMax = 2048;  // members per batch (shared-memory search table)
+constexpr int kDirectSteps = 16;  // steps of a tick without a graph (one table upload for all of them)
 
 struct BatchEntry {
     unsigned long long begin;  // packed index of the member's first cell
@@ -284,6 +293,49 @@ __global__ void __launch_bounds__(rowslp::kThreads, kMinBlocks)
     rowslp::run_items<kDirBytes, lowp::F2, true>(item_of, my, stages, base, smem, wc);
 }
 
+// A member of the two-steps-per-launch kernel.
+struct PairEntry {
+    float* buf[2];
+    unsigned long long plane;
+    two::Plan plan;
+    int nx, ny, nz;
+    int cur;    // buffer holding the member's state at the start of the tick
+    int steps;  // fused steps this tick
+    float eps;
+    unsigned begin;  // first item of the member
+};
+
+struct PairHeader {
+    unsigned total;  // items of all members
+    int count;
+};
+
+constexpr int kPairGroup = 8;  // items per entry of the member lookup table
+
+// Steps s and s + 1 (s even) of every member: one CTA per item, a tile's
+// part along x (two_f32.cuh).  The item's member is found from group[item /
+// kPairGroup] by stepping forward.  24 float32 lattices of edges 32 to 128,
+// initialised, stepped 96 times and read back: 46.3 -> 37.7 ms against the
+// one-CTA-per-segment kernel (itself at the copy bandwidth); no shapes to
+// tune on the way: the first batch of a program takes 38.5 ms instead of 111.
+__global__ void __launch_bounds__(two::kThreads, 1)
+    k_batch_pairs(const PairHeader* __restrict__ hdr, const PairEntry* __restrict__ tab, const two::Maps* __restrict__ maps,
+                  const int* __restrict__ group, int s, CollideF32 base, WaitCtl wc)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    const unsigned item = blockIdx.x;
+    const int count = hdr->count;
+    int m = group[item / kPairGroup];
+    while (m + 1 < count && tab[m + 1].begin <= item) ++m;
+    const PairEntry& e = tab[m];
+    if (s + 1 >= e.steps) return;
+    const int cur = e.cur ^ ((s >> 1) & 1);
+    CollideF32 cp = base;
+    cp.eps = e.eps;
+    two::run_box<true>(&maps[2 * m + cur], e.buf[cur], e.buf[cur ^ 1], e.nx, e.ny, e.nz, e.plane,
+                       two::box_of(e.plan, e.nx, e.ny, e.nz, (int)(item - e.begin)), cp, smem, wc);
+}
+
 }  // namespace
 
 }  // namespace imex
@@ -302,6 +354,35 @@ struct BatchShape {
     int threads = 0, cpt = 0, ctas_per_sm = 0;  // 0: not chosen yet
 };
 
+// A device table and its pinned staging, grown as needed.
+template <class T>
+struct Table {
+    T* d = nullptr;
+    T* h = nullptr;
+    size_t cap = 0;
+    cudaError_t reserve(size_t n, cudaStream_t s)
+    {
+        if (n <= cap) return cudaSuccess;
+        release(s);
+        cudaError_t e = cudaMallocAsync((void**)&d, 2 * n * sizeof(T), s);
+        if (e == cudaSuccess) e = cudaMallocHost((void**)&h, 2 * n * sizeof(T));
+        if (e == cudaSuccess) cap = 2 * n;
+        return e;
+    }
+    cudaError_t upload(size_t n, cudaStream_t s) const
+    {
+        return n ? cudaMemcpyAsync(d, h, n * sizeof(T), cudaMemcpyHostToDevice, s) : cudaSuccess;
+    }
+    void release(cudaStream_t s)
+    {
+        if (d) cudaFreeAsync(d, s);
+        if (h) cudaFreeHost(h);
+        d = nullptr;
+        h = nullptr;
+        cap = 0;
+    }
+};
+
 struct imex_batch {
     std::vector<imex_lattice*> members;
     std::vector<int64_t> limit;  // total reference steps after which a member stops (-1: none)
@@ -318,7 +399,22 @@ struct imex_batch {
     int* d_group = nullptr;     // one-CTA-per-segment cell kernel: member of every kUnitGroup-th segment
     int* h_group = nullptr;
     size_t group_cap = 0;
-    unsigned* d_err = nullptr;  // set by the row kernel when a bounded wait runs out
+    unsigned* d_err = nullptr;  // set by a kernel when a bounded wait runs out
+    // two steps per launch
+    bool cells_pinned = false, rows_pinned = false;  // a launch shape was set: every member keeps one step per launch
+    std::vector<char> pair;          // per member: in the two-step kernel
+    std::vector<two::Plan> pair_plan;
+    Table<PairHeader> phdr;
+    Table<PairEntry> ptab;
+    Table<two::Maps> pmaps;
+    size_t pmaps_up = 0;             // maps of pmaps.h the device holds
+    Table<int> pgroup;
+    Table<BatchHeader> thdr;         // the members' odd last step, in the cell kernel
+    Table<BatchEntry> ttab;
+    Table<int> tgroup;
+    int n_pair = 0;                  // members of the last uploaded table, their items, and the odd steps' segments
+    unsigned pair_items = 0;
+    unsigned tail_units = 0;
     int capacity = 0;
     int device = 0;
     int sms = 0;
@@ -333,7 +429,9 @@ struct imex_batch {
     unsigned long long graph_units = 0;  // segments the captured cell-kernel launches cover
     const int* graph_group = nullptr;    // the group table the captured segment-kernel launches read
     RowShape graph_rshape;
-    int graph_kinds = 0;  // bit 0: cell kernel, bit 1: row kernel, bit 2: cell kernel with float16 members
+    unsigned graph_items = 0;            // items the captured two-step launches cover
+    const void* graph_ptab[4] = {};      // and the tables they read
+    int graph_kinds = 0;  // bit 3: two-step kernel, bit 0: cell kernel, bit 1: row kernel, bit 2: cell kernel with float16 members
     int64_t launches = 0;
     std::string err;
 };
@@ -382,7 +480,7 @@ bool rows_fit(const RowShape& rs, int members)
 
 int kinds(const imex_batch* b)
 {
-    return (b->n_cell > 0 ? 1 : 0) | (b->n_row > 0 ? 2 : 0) | (b->n_cell_f16 > 0 ? 4 : 0);
+    return (b->n_cell > 0 ? 1 : 0) | (b->n_row > 0 ? 2 : 0) | (b->n_cell_f16 > 0 ? 4 : 0) | (b->n_pair > 0 ? 8 : 0);
 }
 
 // One step (index s of the tick) of every member: the cell kernel over its
@@ -477,6 +575,178 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
     return cudaSuccess;
 }
 
+// Steps s and s + 1 of the two-step kernel's members.
+cudaError_t launch_pairs(imex_batch* b, int s)
+{
+    k_batch_pairs<<<b->pair_items, two::kThreads, two::kSmemBytes, b->stream>>>(b->phdr.d, b->ptab.d, b->pmaps.d, b->pgroup.d, s,
+                                                                               base_constants(), make_wait_ctl(b->d_err));
+    return cudaGetLastError();
+}
+
+// The odd last step of its members, after their pairs.
+cudaError_t launch_tail(imex_batch* b)
+{
+    k_batch_units<IMEX_F32><<<b->tail_units, kUnitCells, 0, b->stream>>>(b->thdr.d, b->ttab.d, b->tgroup.d, 0,
+                                                                        base_constants());
+    return cudaGetLastError();
+}
+
+// Step s of the tick of every member (a pair of steps at even s).
+cudaError_t launch_all(imex_batch* b, int s, int K)
+{
+    cudaError_t e = launch_step(b, b->shape, b->rshape, s);
+    if (e == cudaSuccess && b->n_pair > 0 && s % 2 == 0 && s + 1 < K) e = launch_pairs(b, s);
+    return e;
+}
+
+// Whether a member steps once per launch (in the cell or the row kernel).
+bool single(const imex_batch* b, size_t m) { return m >= b->pair.size() || !b->pair[m]; }
+
+// Choose the members of the two-step kernel: float32 lattices that can take
+// it and whose tiles fit it well enough (a 32^3 lattice fills 8 of 10 tile
+// rows and spends 5 of 37 iterations starting up, and still gains 1.25), cut
+// along x so that the SMs' work evens out; none if all of them together
+// leave the GPU too empty to gain.  Estimated from the measured costs of
+// two_f32.hpp: an SM works its share of all items and, in the end, about half
+// the longest one alone.  Pinned launch shapes keep one step per launch.
+void pick_pairs(imex_batch* b)
+{
+    const size_t n = b->members.size();
+    b->pair.assign(n, 0);
+    b->pair_plan.assign(n, two::Plan{});
+    if (b->cells_pinned || b->rows_pinned) return;
+    double singles = 0;
+    std::vector<size_t> cand;
+    for (size_t m = 0; m < n; ++m) {
+        const imex_lattice* h = b->members[m];
+        if (h->precision != IMEX_F32 || !two::eligible(h->g)) continue;
+        const two::Plan p = two::plan_tiles(h->g, h->g.nx);
+        const double one = 2.0 * (double)h->ncells * two::kCellUs;
+        if ((double)p.items() * two::item_iterations(h->g, p) * two::kIterationUs / b->sms > 0.97 * one) continue;
+        cand.push_back(m);
+        singles += one;
+    }
+    double best = 0.97 * (singles + two::kLaunchUs);
+    int best_planes = 0;
+    for (int planes : {16, 24, 32, 48, 64, 96, 128, 192, 256}) {
+        double all = 0;
+        int longest = 0;
+        for (size_t m : cand) {
+            const Geom& g = b->members[m]->g;
+            const two::Plan p = two::plan_tiles(g, planes);
+            all += (double)p.items() * two::item_iterations(g, p);
+            longest = std::max(longest, two::item_iterations(g, p));
+        }
+        const double us = two::kLaunchUs + two::kIterationUs * std::max((double)longest, all / b->sms + 0.5 * longest);
+        if (!cand.empty() && us < best) {
+            best = us;
+            best_planes = planes;
+        }
+    }
+    if (!best_planes) return;
+    for (size_t m : cand) {
+        b->pair[m] = 1;
+        b->pair_plan[m] = two::plan_tiles(b->members[m]->g, best_planes);
+    }
+}
+
+// Upload the two-step kernel's tables for a tick of steps[m] steps: members
+// with the longest items first, so that the last items to finish are short.
+int upload_pairs(imex_batch* b, const std::vector<int>& steps)
+{
+    std::vector<size_t> order;
+    for (size_t m = 0; m < b->members.size(); ++m)
+        if (!single(b, m)) order.push_back(m);
+    b->n_pair = (int)order.size();
+    b->pair_items = b->tail_units = 0;
+    if (order.empty()) return IMEX_OK;
+    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) {
+        return two::item_iterations(b->members[x]->g, b->pair_plan[x]) > two::item_iterations(b->members[y]->g, b->pair_plan[y]);
+    });
+    const size_t n = order.size();
+    size_t items = 0, units = 0;
+    for (size_t m : order) {
+        items += b->pair_plan[m].items();
+        const Geom& g = b->members[m]->g;
+        if (steps[m] & 1) units += (size_t)g.nx * g.ny * ((g.nz + kUnitCells - 1) / kUnitCells);
+    }
+    if (items > 0x7fffffffu || units > 0x7fffffffu)
+        return bfail(b, IMEX_ERR_ARG, "imex_batch_step: too many work items for one launch");
+    const void* maps_at = b->pmaps.d;
+    const size_t pgroups = (items + kPairGroup - 1) / kPairGroup, tgroups = (units + kUnitGroup - 1) / kUnitGroup;
+    cudaError_t e = b->phdr.reserve(1, b->stream);
+    if (e == cudaSuccess) e = b->ptab.reserve(n, b->stream);
+    if (e == cudaSuccess) e = b->pmaps.reserve(2 * n, b->stream);
+    if (e == cudaSuccess) e = b->pgroup.reserve(pgroups, b->stream);
+    if (e == cudaSuccess) e = b->thdr.reserve(1, b->stream);
+    if (e == cudaSuccess) e = b->ttab.reserve(n, b->stream);
+    if (e == cudaSuccess) e = b->tgroup.reserve(tgroups, b->stream);
+    if (e != cudaSuccess) return bcuda(b, e, "batch tables");
+    if (b->pmaps.d != maps_at) b->pmaps_up = 0;
+    size_t begin = 0, ubegin = 0;
+    int tails = 0;
+    bool new_maps = b->pmaps_up < 2 * n;
+    for (size_t q = 0; q < n; ++q) {
+        imex_lattice* h = b->members[order[q]];
+        if (!h->pairs)
+            B_CUDA(b, two::make_lattice(static_cast<float*>(h->buf[0]), static_cast<float*>(h->buf[1]), h->g, &h->pairs),
+                   "two-step kernel set-up");
+        const int k = steps[order[q]];
+        PairEntry& p = b->ptab.h[q];
+        p.buf[0] = static_cast<float*>(h->buf[0]);
+        p.buf[1] = static_cast<float*>(h->buf[1]);
+        p.plane = h->ncells;
+        p.plan = b->pair_plan[order[q]];
+        p.nx = h->g.nx;
+        p.ny = h->g.ny;
+        p.nz = h->g.nz;
+        p.cur = h->cur;
+        p.steps = k;
+        p.eps = h->cf32.eps;
+        p.begin = (unsigned)begin;
+        for (size_t c = begin; c < begin + p.plan.items(); ++c)
+            if (c % kPairGroup == 0) b->pgroup.h[c / kPairGroup] = (int)q;
+        begin += p.plan.items();
+        // the maps change with the members only: uploaded when they differ
+        if (new_maps || std::memcmp(&b->pmaps.h[2 * q], h->pairs->maps, sizeof h->pairs->maps)) {
+            std::memcpy(&b->pmaps.h[2 * q], h->pairs->maps, sizeof h->pairs->maps);
+            new_maps = true;
+        }
+        if (!(k & 1)) continue;
+        BatchEntry& t = b->ttab.h[tails];
+        t = BatchEntry{};
+        t.begin = ubegin;
+        t.plane = h->ncells;
+        t.buf[0] = h->buf[0];
+        t.buf[1] = h->buf[1];
+        t.nx = h->g.nx;
+        t.ny = h->g.ny;
+        t.nz = h->g.nz;
+        t.prec = IMEX_F32;
+        t.cur = h->cur ^ ((k / 2) & 1);
+        t.steps = 1;
+        t.eps = h->cf32.eps;
+        const size_t mine = (size_t)h->g.nx * h->g.ny * ((h->g.nz + kUnitCells - 1) / kUnitCells);
+        for (size_t c = (ubegin + kUnitGroup - 1) / kUnitGroup; c * kUnitGroup < ubegin + mine; ++c) b->tgroup.h[c] = tails;
+        ubegin += mine;
+        ++tails;
+    }
+    *b->phdr.h = PairHeader{(unsigned)begin, (int)n};
+    *b->thdr.h = BatchHeader{ubegin, tails, 0};
+    b->pair_items = (unsigned)begin;
+    b->tail_units = (unsigned)ubegin;
+    e = b->phdr.upload(1, b->stream);
+    if (e == cudaSuccess) e = b->ptab.upload(n, b->stream);
+    if (e == cudaSuccess && new_maps) e = b->pmaps.upload(2 * n, b->stream);
+    if (e == cudaSuccess) e = b->pgroup.upload(pgroups, b->stream);
+    if (e == cudaSuccess && tails) e = b->thdr.upload(1, b->stream);
+    if (e == cudaSuccess && tails) e = b->ttab.upload(tails, b->stream);
+    if (e == cudaSuccess && tails) e = b->tgroup.upload(tgroups, b->stream);
+    if (e != cudaSuccess) return bcuda(b, e, "batch tables");
+    b->pmaps_up = std::max(b->pmaps_up, 2 * n);
+    return IMEX_OK;
+}
+
 // Steps a member still owes before its limit.
 int64_t owed(const imex_batch* b, size_t m, int64_t want)
 {
@@ -509,6 +779,7 @@ int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& r
     unsigned ibegin = 0;
     int n = 0, nr = 0, n16 = 0;
     for (size_t m = 0; m < b->members.size(); ++m) {
+        if (!single(b, m)) continue;
         imex_lattice* h = b->members[m];
         const int B = rows_per_item(h, rs);
         if (!B && h->precision != IMEX_F32) ++n16;
@@ -732,7 +1003,7 @@ int capture_graph(imex_batch* b, int K)
     cudaGraph_t g = nullptr;
     B_CUDA(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
     cudaError_t e = cudaSuccess;
-    for (int s = 0; s < K && e == cudaSuccess; ++s) e = launch_step(b, b->shape, b->rshape, s);
+    for (int s = 0; s < K && e == cudaSuccess; ++s) e = launch_all(b, s, K);
     cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
     if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph, g, 0);
@@ -744,7 +1015,19 @@ int capture_graph(imex_batch* b, int K)
     b->graph_kinds = kinds(b);
     b->graph_units = b->h_hdr->total;
     b->graph_group = b->d_group;
+    b->graph_items = b->pair_items;
+    const void* tabs[4] = {b->phdr.d, b->ptab.d, b->pmaps.d, b->pgroup.d};
+    std::copy(tabs, tabs + 4, b->graph_ptab);
     return IMEX_OK;
+}
+
+// Whether the captured two-step launches still cover the members' items and
+// read the tables in use.
+bool graph_pairs_valid(const imex_batch* b)
+{
+    return b->n_pair == 0 || (b->graph_items == b->pair_items && b->graph_ptab[0] == b->phdr.d &&
+                              b->graph_ptab[1] == b->ptab.d && b->graph_ptab[2] == b->pmaps.d &&
+                              b->graph_ptab[3] == b->pgroup.d);
 }
 
 // Whether the captured graph still describes the launches: the same shapes
@@ -753,7 +1036,7 @@ int capture_graph(imex_batch* b, int K)
 // moves the table when a tick or a tuning candidate needs a larger one).
 bool graph_valid(const imex_batch* b, int K)
 {
-    return b->graph && b->graph_k == K && b->graph_shape.threads == b->shape.threads &&
+    return b->graph && b->graph_k == K && graph_pairs_valid(b) && b->graph_shape.threads == b->shape.threads &&
            b->graph_shape.cpt == b->shape.cpt && b->graph_shape.ctas_per_sm == b->shape.ctas_per_sm &&
            b->graph_rshape.stages == b->rshape.stages && b->graph_rshape.dir_kb == b->rshape.dir_kb &&
            b->graph_rshape.f32 == b->rshape.f32 &&
@@ -788,6 +1071,8 @@ int imex_batch_create(int max_members, imex_batch** out)
     if (e == cudaSuccess) e = cudaMalloc(&b->d_err, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(b->d_err, 0, sizeof(unsigned));
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_batch_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)two::kSmemBytes);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_batch_rows<1024, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_batch_rows<1024, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -812,6 +1097,13 @@ void imex_batch_destroy(imex_batch* b)
     if (!b) return;
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
+    b->phdr.release(b->stream);
+    b->ptab.release(b->stream);
+    b->pmaps.release(b->stream);
+    b->pgroup.release(b->stream);
+    b->thdr.release(b->stream);
+    b->ttab.release(b->stream);
+    b->tgroup.release(b->stream);
     if (b->d_hdr) cudaFree(b->d_hdr);
     if (b->d_tab) cudaFree(b->d_tab);
     if (b->h_hdr) cudaFreeHost(b->h_hdr);
@@ -881,7 +1173,10 @@ int imex_batch_step(imex_batch* b, int nsteps)
     }
     int rc = join_members(b);
     if (rc) return rc;
-    if (!b->shape.threads || !b->rshape.stages) {
+    pick_pairs(b);
+    bool singles = false;  // members that step once per launch
+    for (size_t m = 0; m < b->members.size(); ++m) singles = singles || single(b, m);
+    if (singles && (!b->shape.threads || !b->rshape.stages)) {
         rc = tune_batch(b, !b->shape.threads, !b->rshape.stages);
         if (rc) return rc;
     }
@@ -890,10 +1185,11 @@ int imex_batch_step(imex_batch* b, int nsteps)
         int64_t most = 0;
         for (size_t m = 0; m < left.size(); ++m) most = std::max(most, left[m]);
         if (most == 0) break;
-        const int K = b->graph_steps > 0 ? b->graph_steps : 1;
+        const int K = b->graph_steps > 0 ? b->graph_steps : kDirectSteps;
         const int k = (int)std::min<int64_t>(most, K);
         for (size_t m = 0; m < left.size(); ++m) tick[m] = (int)std::min<int64_t>(left[m], k);
-        rc = upload_table(b, tick, b->rshape, b->shape);
+        rc = upload_pairs(b, tick);
+        if (!rc) rc = upload_table(b, tick, b->rshape, b->shape);
         if (rc) return rc;
         if (b->graph_steps > 0 && k == b->graph_steps) {
             if (!graph_valid(b, k)) {
@@ -902,14 +1198,16 @@ int imex_batch_step(imex_batch* b, int nsteps)
             }
             B_CUDA(b, cudaGraphLaunch(b->graph, b->stream), "cudaGraphLaunch");
         } else {
-            for (int s = 0; s < k; ++s) B_CUDA(b, launch_step(b, b->shape, b->rshape, s), "batch kernel launch");
+            for (int s = 0; s < k; ++s) B_CUDA(b, launch_all(b, s, k), "batch kernel launch");
         }
-        b->launches += (int64_t)k * ((b->n_cell > 0) + (b->n_row > 0));
+        if (b->tail_units) B_CUDA(b, launch_tail(b), "batch kernel launch");
+        b->launches += (int64_t)k * ((b->n_cell > 0) + (b->n_row > 0)) + (b->n_pair > 0 ? k / 2 : 0) + (b->tail_units > 0);
         for (size_t m = 0; m < left.size(); ++m) {
             imex_lattice* h = b->members[m];
-            h->cur ^= tick[m] & 1;
+            const int writes = single(b, m) ? tick[m] : tick[m] / 2 + (tick[m] & 1);
+            h->cur ^= writes & 1;
             h->steps += tick[m];
-            h->launches += tick[m];
+            h->launches += writes;
             left[m] -= tick[m];
         }
     }
@@ -935,6 +1233,7 @@ int imex_batch_synchronize(imex_batch* b)
 int imex_batch_set_launch(imex_batch* b, int threads, int cells_per_thread, int ctas_per_sm)
 {
     if (!b) return set_thread_error(IMEX_ERR_ARG, "imex_batch_set_launch: null batch");
+    b->cells_pinned = threads != 0;
     if (threads == 0) {
         b->shape = BatchShape{};
         return IMEX_OK;
@@ -968,6 +1267,7 @@ int imex_batch_get_launch(imex_batch* b, int out[3])
 int imex_batch_set_row_launch(imex_batch* b, int stages, int dir_kb, int ctas_per_sm, int float32_members)
 {
     if (!b) return set_thread_error(IMEX_ERR_ARG, "imex_batch_set_row_launch: null batch");
+    b->rows_pinned = stages != 0;
     if (stages == 0 || stages == -1) {  // 0: autotune, -1: row kernel off
         b->rshape = RowShape{stages, 0, 0, 1};
         return IMEX_OK;

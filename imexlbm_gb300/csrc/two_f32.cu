@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               CollideF32 cp, WaitCtl wc)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    run_box(&maps, src, dst, g.nx, g.ny, g.nz, g.plane, box_of(p, g.nx, g.ny, g.nz, blockIdx.x), cp, smem, wc);
+    run_box<false>(&maps, src, dst, g.nx, g.ny, g.nz, g.plane, box_of(p, g.nx, g.ny, g.nz, blockIdx.x), cp, smem, wc);
 }
 
 using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -46,7 +46,7 @@ constexpr int kExtra = 5;
 // Iterations of the busiest SM (one CTA each at a time).
 long long iterations(const Geom& g, const Plan& p, int sms)
 {
-    return ((long long)p.nty * p.ntz * p.chunks + sms - 1) / sms * ((g.nx + p.chunks - 1) / p.chunks + kExtra);
+    return (long long)((p.items() + sms - 1) / sms) * item_iterations(g, p);
 }
 
 Plan tiles_of(const Geom& g)
@@ -61,13 +61,7 @@ Plan tiles_of(const Geom& g)
     return p;
 }
 
-}  // namespace
-
-bool eligible(const Geom& g)
-{
-    return g.nz % 4 == 0 && g.nz >= kTileZ && g.ny >= 4 && g.nx >= 4 && g.plane < (1ull << 32) / kQ;
-}
-
+// The tiles cut along x so that the busiest SM has least to do.
 Plan plan_for(const Geom& g, int sms)
 {
     Plan p = tiles_of(g);
@@ -75,27 +69,6 @@ Plan plan_for(const Geom& g, int sms)
     for (p.chunks = 2; p.chunks <= g.nx; ++p.chunks)
         if (iterations(g, p, sms) < iterations(g, best, sms)) best = p;
     return best;
-}
-
-Plan plan_tiles(const Geom& g, int planes)
-{
-    Plan p = tiles_of(g);
-    p.chunks = std::max(1, (g.nx + planes / 2) / planes);
-    return p;
-}
-
-// Measured: a launch takes 4 us and 1.85 us per iteration of its busiest SM
-// (64^3 26 us, 96^3 51, 128^3 113, 256^3 703), two launches of the one-step
-// kernel 2 (2 us + cells / 29 per ns) (64^3 21 us, 96^3 66, 128^3 141, 256^3
-// 1053).  So small lattices, whose tiles leave SMs idle or spend most
-// iterations filling the pipeline, and shapes that fit the tiles badly keep one step per
-// launch; the line lies near 80^3.
-bool worth_alone(const Geom& g, int sms)
-{
-    if (!eligible(g)) return false;
-    const double pair = 4.0 + 1.85 * (double)iterations(g, plan_for(g, sms), sms);
-    const double singles = 2.0 * (2.0 + (double)g.plane / 29000.0);
-    return pair < 0.97 * singles;
 }
 
 cudaError_t encode_maps(const float* buf, const Geom& g, const Plan& p, Maps* out)
@@ -116,17 +89,36 @@ cudaError_t encode_maps(const float* buf, const Geom& g, const Plan& p, Maps* ou
     return cudaSuccess;
 }
 
-cudaError_t allow_smem(const void* kernel)
+}  // namespace
+
+bool eligible(const Geom& g)
 {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    return g.nz % 4 == 0 && g.nz >= kTileZ && g.ny >= 4 && g.nx >= 4 && g.plane < (1ull << 32) / kQ;
 }
 
-struct Lattice {
-    Plan plan;
-    Maps maps[2];
-};
 
-void LatticeDelete::operator()(Lattice* p) const { delete p; }
+int item_iterations(const Geom& g, const Plan& p) { return (g.nx + p.chunks - 1) / p.chunks + kExtra; }
+
+Plan plan_tiles(const Geom& g, int planes)
+{
+    Plan p = tiles_of(g);
+    p.chunks = std::max(1, (g.nx + planes / 2) / planes);
+    return p;
+}
+
+// Measured: a launch takes 4 us and 1.85 us per iteration of its busiest SM
+// (64^3 26 us, 96^3 51, 128^3 113, 256^3 703), two launches of the one-step
+// kernel 2 (2 us + cells / 29 per ns) (64^3 21 us, 96^3 66, 128^3 141, 256^3
+// 1053).  So small lattices, whose tiles leave SMs idle or spend most
+// iterations filling the pipeline, and shapes that fit the tiles badly keep one step per
+// launch; the line lies near 80^3.
+bool worth_alone(const Geom& g, int sms)
+{
+    if (!eligible(g)) return false;
+    const double pair = kLaunchUs + kIterationUs * (double)iterations(g, plan_for(g, sms), sms);
+    const double singles = 2.0 * (kLaunchUs / 2 + (double)g.plane * kCellUs);
+    return pair < 0.97 * singles;
+}
 
 cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, LatticePtr* out)
 {
@@ -135,7 +127,8 @@ cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, La
     l->plan = plan_for(g, current_sm_count());
     cudaError_t e = encode_maps(buf0, g, l->plan, &l->maps[0]);
     if (e == cudaSuccess) e = encode_maps(buf1, g, l->plan, &l->maps[1]);
-    if (e == cudaSuccess) e = allow_smem((const void*)k_two_f32);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_two_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e == cudaSuccess) *out = std::move(l);
     return e;
 }
@@ -143,8 +136,7 @@ cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, La
 cudaError_t launch(const Lattice& l, int from, const float* src, float* dst, const Geom& g, const CollideF32& cp,
                    unsigned* err, cudaStream_t s)
 {
-    const unsigned grid = (unsigned)(l.plan.nty * l.plan.ntz * l.plan.chunks);
-    k_two_f32<<<grid, kThreads, kSmemBytes, s>>>(l.maps[from], src, dst, g, l.plan, cp, make_wait_ctl(err));
+    k_two_f32<<<(unsigned)l.plan.items(), kThreads, kSmemBytes, s>>>(l.maps[from], src, dst, g, l.plan, cp, make_wait_ctl(err));
     return cudaGetLastError();
 }
 

@@ -47,12 +47,12 @@
 // strides), nz >= 32, ny >= 4, nx >= 4, 27 * cells below 2^32.
 #pragma once
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "bulk.cuh"
 #include "kernels_common.cuh"
 #include "lowp_math.cuh"
+#include "two_f32.hpp"
 
 namespace imex {
 namespace two {
@@ -67,7 +67,6 @@ constexpr int kStage = kRows * (kTileZ + 8);  // staged values of a direction: r
 constexpr int kRing = 9 * (1 + 2 + 3);       // ring arrays of kMid values
 constexpr int kSide = 7;                     // side pieces of a loader thread
 constexpr int kLoadWarps = kThreadsL / 32;
-constexpr int kMaps = 4;                     // boxes of ty + 2, ty + 1, ty and ty - 1 rows
 static_assert(kMid / 2 <= kThreadsA && kTileY * kTileZ / 2 <= kThreadsB, "one pair of cells per thread");
 static_assert(36 * kRows <= kSide * kThreadsL, "side pieces");
 static_assert(kStage * 4 % 128 == 0 && kMid % 2 == 0, "128-byte aligned boxes, 8-byte pairs");
@@ -77,16 +76,6 @@ static_assert(kLoadWarps * 32 >= kQ, "a loader thread per direction");
 constexpr size_t kDataBytes = (size_t)(2 * kQ * kStage + kRing * kMid) * sizeof(float);
 constexpr size_t kSmemBytes = kDataBytes + 64;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of a CTA");
-
-struct alignas(64) Maps {
-    CUtensorMap m[kMaps];
-};
-
-// How a lattice is cut: nty x ntz tiles of at most ty x tz destinations, each
-// marched in `chunks` parts along x.
-struct Plan {
-    int ty, tz, nty, ntz, chunks;
-};
 
 // One CTA's destinations.
 struct Box {
@@ -157,10 +146,13 @@ __device__ __forceinline__ void cp16(void* dst, const void* src)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(bulk::smem_u32(dst)), "l"(src) : "memory");
 }
 
-// The two-step march of one box of the lattice at src into dst.  Every wait
+// The two-step march of one box of the lattice at src into dst.  kMapsInMemory:
+// the tensor maps lie in global memory (a batch's table) rather than in the
+// kernel's parameters.  Every wait
 // on an mbarrier is bounded: one that runs out sets wc.err, the loaders stop
 // bringing planes, and the CTA runs to its end on what the stages hold (its
 // results are reported invalid).
+template <bool kMapsInMemory>
 __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const float* __restrict__ src,
                                         float* __restrict__ dst, int nx, int ny, int nz, size_t plane, const Box& b,
                                         const CollideF32& cp, unsigned char* smem, const WaitCtl& wc)
@@ -198,6 +190,8 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
         // with the map's otherwise (a tile one row short brings one too many)
         const int rows = bot ? R - top - bot : b.box_rows - top;
         const CUtensorMap* const map = &maps->m[b.box_rows - rows];
+        if constexpr (kMapsInMemory)  // written through the generic proxy (an upload before the launch)
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
         const uint32_t row_bytes = (uint32_t)b.cols * 4u;
         const uint32_t my_bytes = (uint32_t)rows * (kTileZ * 4u) + (uint32_t)(top + bot) * row_bytes;
         unsigned from[kSide], at[kSide];
