@@ -45,10 +45,12 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "imexlbm.h"
 #include "imexlbm_internal.hpp"
+#include "flat_lowp.cuh"
 #include "lattice_internal.hpp"
 #include "lowp_math.cuh"
 #include "rows_lowp.cuh"
@@ -131,26 +133,28 @@ __device__ __forceinline__ void batch_cell(const BatchEntry& e, unsigned local, 
     batch_cell_at<P>(e, i, j, k, local, s, base);
 }
 
-// Cells per row segment of the one-CTA-per-segment cell kernel.
-constexpr int kUnitCells = kStepBlock;
-constexpr int kUnitGroup = 256;  // row segments per entry of the member lookup table
+// Cells per segment of the one-CTA-per-segment cell kernel.
+constexpr int kUnitCells = flat::kCells, kUnitThreads = flat::kThreads;
+constexpr int kUnitGroup = 256;  // segments per entry of the member lookup table
 
-// One CTA per row segment: the grid of the one-lattice kernel (k_step_lowp:
-// 128 threads per CTA, each CTA kUnitCells consecutive z-cells of one (x, y)
-// row), over every member of the cell kernel.  Segment u belongs to the
-// member whose first segment index `begin` is the largest not above u; the
-// member is found from group[u / kUnitGroup] (the member holding segment
-// u - u mod kUnitGroup) by stepping forward, the same for every thread of
-// the CTA, and the segment's (x, y, z block) is decoded once per CTA, so a
-// thread's cell costs what it costs in the one-lattice kernel.  The grid
-// covers the segments of the tick's members; a CUDA graph of these
-// launches is captured again when that count changes.  The float32-only
-// instantiation fits 48 registers (10 CTAs, 40 warps per SM, as the one-
-// lattice kernel); with the float16 path too it needs 64.
-template <int PF, int MINB = PF == IMEX_F32 ? 10 : 0>
-__global__ void __launch_bounds__(kUnitCells, MINB) k_batch_units(const BatchHeader* __restrict__ hdr,
-                                                            const BatchEntry* __restrict__ tab,
-                                                            const int* __restrict__ group, int s, CollideF32 base)
+// Segments of a member.
+__host__ __device__ inline unsigned long long unit_count(unsigned long long cells)
+{
+    return (cells + kUnitCells - 1) / kUnitCells;
+}
+
+// One CTA per segment of kUnitCells cells in a member's flat order, two
+// cells per thread (flat_lowp.cuh, the one-lattice kernel's cell pairs).
+// Segment u belongs to the member whose first segment index `begin` is the
+// largest not above u; the member is found from group[u / kUnitGroup] (the
+// member holding segment u - u mod kUnitGroup) by stepping forward, the same
+// for every thread of the CTA.  The grid covers the segments of the tick's
+// members; a CUDA graph of these launches is captured again when that count
+// changes.  PF = IMEX_F32: every member is float32.
+template <int PF>
+__global__ void __launch_bounds__(kUnitThreads) k_batch_units(const BatchHeader* __restrict__ hdr,
+                                                              const BatchEntry* __restrict__ tab,
+                                                              const int* __restrict__ group, int s, CollideF32 base)
 {
     const unsigned u = blockIdx.x;
     const int count = hdr->count;
@@ -158,17 +162,28 @@ __global__ void __launch_bounds__(kUnitCells, MINB) k_batch_units(const BatchHea
     while (m + 1 < count && tab[m + 1].begin <= u) ++m;
     const BatchEntry& e = tab[m];
     if (s >= e.steps) return;
-    const unsigned zbs = ((unsigned)e.nz + kUnitCells - 1) / kUnitCells;
     const unsigned seg = u - (unsigned)e.begin;
-    const unsigned row = seg / zbs;
-    const int k = (int)(seg - row * zbs) * kUnitCells + (int)threadIdx.x;
-    if (k >= e.nz) return;
-    const int i = (int)(row / (unsigned)e.ny);
-    const int j = (int)(row - (unsigned)i * (unsigned)e.ny);
-    const unsigned local = row * (unsigned)e.nz + (unsigned)k;
-    if constexpr (PF == IMEX_F32) batch_cell_at<IMEX_F32>(e, i, j, k, local, s, base);
-    else if (e.prec == IMEX_F32) batch_cell_at<IMEX_F32>(e, i, j, k, local, s, base);
-    else batch_cell_at<IMEX_F16DEV>(e, i, j, k, local, s, base);
+    const void* src = e.buf[e.cur ^ (s & 1)];
+    void* dst = e.buf[e.cur ^ (s & 1) ^ 1];
+    CollideF32 cp = base;
+    cp.eps = e.eps;
+    auto run = [&](auto prec, auto near_) {
+        constexpr int P = decltype(prec)::value;
+        constexpr bool kNear = decltype(near_)::value;
+        using T = typename lowp::Storage<P>::T;
+        const unsigned c = flat::first_cell<kNear>(seg, threadIdx.x);
+        if (c < (unsigned)e.plane)
+            flat::step_pair<P, kNear>(static_cast<const T*>(src), static_cast<T*>(dst), e.nx, e.ny, e.nz, e.plane, c, cp);
+    };
+    if (PF != IMEX_F32 && e.prec == IMEX_F16DEV) {
+        cp.sr = e.sr;
+        cp.seed = e.seed + (uint32_t)s;
+        run(std::integral_constant<int, IMEX_F16DEV>{}, std::true_type{});
+    } else if (e.plane & 1) {
+        run(std::integral_constant<int, IMEX_F32>{}, std::false_type{});
+    } else {
+        run(std::integral_constant<int, IMEX_F32>{}, std::true_type{});
+    }
 }
 
 // CPT cells per thread, strided by blockDim within a chunk of CPT*blockDim.
@@ -528,14 +543,14 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
     if (b->n_cell > 0) {
         const bool f32 = b->n_cell_f16 == 0;
         cudaError_t e;
-        if (sh.cpt == 0) {  // one CTA per row segment
+        if (sh.cpt == 0) {  // one CTA per segment
             const unsigned long long units = b->h_hdr->total;
             if (units == 0 || units > 0x7fffffffull) return cudaErrorInvalidValue;
             if (f32)
-                k_batch_units<IMEX_F32><<<(unsigned)units, kUnitCells, 0, b->stream>>>(b->d_hdr, b->d_tab, b->d_group, s,
+                k_batch_units<IMEX_F32><<<(unsigned)units, kUnitThreads, 0, b->stream>>>(b->d_hdr, b->d_tab, b->d_group, s,
                                                                                      base);
             else
-                k_batch_units<0><<<(unsigned)units, kUnitCells, 0, b->stream>>>(b->d_hdr, b->d_tab, b->d_group, s, base);
+                k_batch_units<0><<<(unsigned)units, kUnitThreads, 0, b->stream>>>(b->d_hdr, b->d_tab, b->d_group, s, base);
             e = cudaGetLastError();
         } else if (f32 && sh.cpt == 1 && sh.threads == 128) e = launch_cells<1, IMEX_F32, 128, 9>(b, sh, s, base);
         else if (sh.cpt == 1) e = f32 ? launch_cells<1, IMEX_F32>(b, sh, s, base) : launch_cells<1, 0>(b, sh, s, base);
@@ -586,7 +601,7 @@ cudaError_t launch_pairs(imex_batch* b, int s)
 // The odd last step of its members, after their pairs.
 cudaError_t launch_tail(imex_batch* b)
 {
-    k_batch_units<IMEX_F32><<<b->tail_units, kUnitCells, 0, b->stream>>>(b->thdr.d, b->ttab.d, b->tgroup.d, 0,
+    k_batch_units<IMEX_F32><<<b->tail_units, kUnitThreads, 0, b->stream>>>(b->thdr.d, b->ttab.d, b->tgroup.d, 0,
                                                                         base_constants());
     return cudaGetLastError();
 }
@@ -667,8 +682,7 @@ int upload_pairs(imex_batch* b, const std::vector<int>& steps)
     size_t items = 0, units = 0;
     for (size_t m : order) {
         items += b->pair_plan[m].items();
-        const Geom& g = b->members[m]->g;
-        if (steps[m] & 1) units += (size_t)g.nx * g.ny * ((g.nz + kUnitCells - 1) / kUnitCells);
+        if (steps[m] & 1) units += unit_count(b->members[m]->ncells);
     }
     if (items > 0x7fffffffu || units > 0x7fffffffu)
         return bfail(b, IMEX_ERR_ARG, "imex_batch_step: too many work items for one launch");
@@ -726,7 +740,7 @@ int upload_pairs(imex_batch* b, const std::vector<int>& steps)
         t.cur = h->cur ^ ((k / 2) & 1);
         t.steps = 1;
         t.eps = h->cf32.eps;
-        const size_t mine = (size_t)h->g.nx * h->g.ny * ((h->g.nz + kUnitCells - 1) / kUnitCells);
+        const size_t mine = unit_count(h->ncells);
         for (size_t c = (ubegin + kUnitGroup - 1) / kUnitGroup; c * kUnitGroup < ubegin + mine; ++c) b->tgroup.h[c] = tails;
         ubegin += mine;
         ++tails;
@@ -773,7 +787,7 @@ int rows_per_item(const imex_lattice* h, const RowShape& rs)
 // on a boundary of sh's chunk (threads x cells per thread).
 int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& rs, const BatchShape& sh)
 {
-    const bool units = sh.cpt == 0;  // one CTA per row segment: the index counts segments
+    const bool units = sh.cpt == 0;  // one CTA per segment: the index counts segments
     const unsigned long long chunk = (unsigned long long)(sh.threads > 0 ? sh.threads : 256) * (sh.cpt > 0 ? sh.cpt : 1);
     unsigned long long begin = 0;
     unsigned ibegin = 0;
@@ -806,7 +820,7 @@ int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& r
             e.begin = begin;
             e.ibegin = 0;
             if (units)
-                begin += (unsigned long long)h->g.nx * h->g.ny * ((h->g.nz + kUnitCells - 1) / kUnitCells);
+                begin += unit_count(h->ncells);
             else
                 begin += (h->ncells + chunk - 1) / chunk * chunk;
         }
@@ -814,7 +828,7 @@ int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& r
     b->h_hdr->total = begin;
     b->h_hdr->count = n;
     if (units && n > 0) {
-        if (begin > 0x7fffffffull) return bfail(b, IMEX_ERR_ARG, "imex_batch_step: too many row segments for one launch");
+        if (begin > 0x7fffffffull) return bfail(b, IMEX_ERR_ARG, "imex_batch_step: too many segments for one launch");
         const size_t groups = (size_t)((begin + kUnitGroup - 1) / kUnitGroup);
         if (groups > b->group_cap) {
             if (b->d_group) cudaFreeAsync(b->d_group, b->stream);
@@ -873,26 +887,6 @@ int release_members(imex_batch* b)
     return IMEX_OK;
 }
 
-std::vector<BatchShape> candidates()
-{
-    std::vector<BatchShape> out;
-    out.push_back(BatchShape{kUnitCells, 0, 0});  // one CTA per row segment
-    const int threads[2] = {128, 256};
-    const int cpts[3] = {1, 2, 4};
-    const int ctas[4] = {2, 4, 8, 9};
-    for (int t : threads)
-        for (int c : cpts)
-            for (int k : ctas) {
-                if (t * k > 2048 || (k == 9 && (t != 128 || c != 1))) continue;  // 9: the lean kernel's residency
-                BatchShape s;
-                s.threads = t;
-                s.cpt = c;
-                s.ctas_per_sm = k;
-                out.push_back(s);
-            }
-    return out;
-}
-
 // Row-kernel shapes (stages, KiB per direction, CTAs per SM); those whose
 // CTAs do not fit an SM's shared memory with the batch's table are skipped.
 std::vector<RowShape> row_candidates()
@@ -935,61 +929,37 @@ int time_step(imex_batch* b, const BatchShape& sh, const RowShape& rs, float* ms
     return IMEX_OK;
 }
 
-// Pick the launch shapes.  First the row kernel's: each shape, with and
-// without the float32 members, against the row kernel off, the members it
-// leaves in the cell kernel at the cell kernel's current (or default)
-// shape; then the cell kernel's shapes - only if the chosen split leaves it
-// members, and timed on that split.  Shapes pinned by imex_batch_set_launch
-// / imex_batch_set_row_launch are kept.  Each timing is one warm-up and
-// three steps of the whole batch, so the order matters for a large batch:
-// float16-deviation members usually go to the row kernel and float32 ones
-// to the one-CTA-per-segment cell kernel, and the cell kernel's other
-// shapes are timed only on what is left to it.
-int tune_batch(imex_batch* b, bool tune_cells, bool tune_rows)
+// Pick the launch shapes.  The cell kernel's is one CTA per segment: its
+// other shapes (k_batch: pinned by imex_batch_set_launch) were slower on every
+// batch timed, float32 28-30 against 30-32 GLUPS, and timing 18 of them was most of a
+// batch's first call.  The row kernel's shapes are timed, with and without
+// the float32 members, against the row kernel off, the members it leaves in
+// the cell kernel.  Shapes pinned by imex_batch_set_launch /
+// imex_batch_set_row_launch are kept.  Each timing is one warm-up and three
+// steps of the members that step once per launch.
+int tune_batch(imex_batch* b)
 {
+    if (!b->shape.threads) b->shape = BatchShape{kUnitThreads, 0, 0};
+    if (b->rshape.stages) return IMEX_OK;
     const RowShape off{-1, 0, 0, 1};
-    // the row kernel's shapes are weighed against the cell kernel's usual
-    // best, one CTA per row segment
-    if (!b->shape.threads) b->shape = BatchShape{kUnitCells, 0, 0};
-    if (tune_rows) {
-        float best = 0.f;
-        int rc = time_step(b, b->shape, off, &best);
-        if (rc) return rc;
-        RowShape best_rs = off;
-        for (RowShape rs : row_candidates()) {
-            if (!rows_fit(rs, b->capacity)) continue;
-            for (int f32 = 1; f32 >= 0; --f32) {
-                rs.f32 = f32;
-                float ms = 0.f;
-                rc = time_step(b, b->shape, rs, &ms);
-                if (rc) return rc;
-                if (b->n_row > 0 && ms < best) {
-                    best = ms;
-                    best_rs = rs;
-                }
+    float best = 0.f;
+    int rc = time_step(b, b->shape, off, &best);
+    if (rc) return rc;
+    RowShape best_rs = off;
+    for (RowShape rs : row_candidates()) {
+        if (!rows_fit(rs, b->capacity)) continue;
+        for (int f32 = 1; f32 >= 0; --f32) {
+            rs.f32 = f32;
+            float ms = 0.f;
+            rc = time_step(b, b->shape, rs, &ms);
+            if (rc) return rc;
+            if (b->n_row > 0 && ms < best) {
+                best = ms;
+                best_rs = rs;
             }
         }
-        b->rshape = best_rs;
     }
-    if (tune_cells) {
-        std::vector<int> one(b->members.size(), 1);
-        int rc = upload_table(b, one, b->rshape, b->shape);
-        if (rc) return rc;
-        if (b->n_cell > 0) {
-            float best = 0.f;
-            BatchShape best_shape;
-            for (const BatchShape& sh : candidates()) {
-                float ms = 0.f;
-                rc = time_step(b, sh, b->rshape, &ms);
-                if (rc) return rc;
-                if (!best_shape.threads || ms < best) {
-                    best = ms;
-                    best_shape = sh;
-                }
-            }
-            b->shape = best_shape;
-        }
-    }
+    b->rshape = best_rs;
     return IMEX_OK;
 }
 
@@ -1177,7 +1147,7 @@ int imex_batch_step(imex_batch* b, int nsteps)
     bool singles = false;  // members that step once per launch
     for (size_t m = 0; m < b->members.size(); ++m) singles = singles || single(b, m);
     if (singles && (!b->shape.threads || !b->rshape.stages)) {
-        rc = tune_batch(b, !b->shape.threads, !b->rshape.stages);
+        rc = tune_batch(b);
         if (rc) return rc;
     }
     std::vector<int> tick(b->members.size());
@@ -1238,11 +1208,11 @@ int imex_batch_set_launch(imex_batch* b, int threads, int cells_per_thread, int 
         b->shape = BatchShape{};
         return IMEX_OK;
     }
-    if (cells_per_thread == 0) {  // one CTA of 128 threads per row segment
-        if (threads != kUnitCells)
-            return bfail(b, IMEX_ERR_ARG, "imex_batch_set_launch: cells_per_thread 0 (one CTA per row segment) "
+    if (cells_per_thread == 0) {  // one CTA of 128 threads per segment
+        if (threads != kUnitThreads)
+            return bfail(b, IMEX_ERR_ARG, "imex_batch_set_launch: cells_per_thread 0 (one CTA per segment) "
                                           "takes 128 threads");
-        b->shape = BatchShape{kUnitCells, 0, 0};
+        b->shape = BatchShape{kUnitThreads, 0, 0};
         return IMEX_OK;
     }
     if ((threads != 128 && threads != 256) || (cells_per_thread != 1 && cells_per_thread != 2 && cells_per_thread != 4) ||

@@ -1,0 +1,135 @@
+// Fused step of the reduced-precision formats over flat cell pairs: a thread
+// takes cells 2 p and 2 p + 1 of the lattice's flat order (z fastest),
+// whatever row they lie in, straight from global memory.  Any sizes; the
+// row-staged kernel (rows_lowp.cuh) takes float16 rows that are whole 16-byte
+// pieces, the two-step kernel (two_f32.cuh) most large float32 lattices, this one the
+// rest.
+//
+// Why pairs in flat order.  One thread per cell and 128 of them per row
+// segment (the form before) leaves the threads behind a row's end idle and
+// spends ~815 instructions on a float16 cell: issue-bound.  Two cells go
+// through the packed f32x2 collision together; pairs of the flat order are
+// the pairs that share a random word (sr_word), so one cvt.rs rounds
+// both; no thread is idle whatever nz is.  The two cells' sources are
+// separate sums of an x, a y and a z offset, so a pair may lie across a
+// row's end.
+// Measured per step, before -> now: float16 131 x 77 x 90 37.0 -> 21.3 us, 107 x
+// 99 x 84 33.0 -> 20.6, 255^3 469 -> 383, 256^3 468 -> 335 (the row-staged kernel:
+// 281); float32 97 x 150 x 121 69.9 -> 61.7, 255^3 575 -> 547, 256^3 527 -> 520
+// (memory alone: 543 at the copy rate).  Bound: memory for float32, issue for float16.
+#pragma once
+
+#include "kernels_common.cuh"
+#include "lowp_math.cuh"
+
+namespace imex {
+namespace flat {
+
+constexpr int kThreads = 128;
+constexpr int kCells = 2 * kThreads;  // cells of a CTA
+
+// Source offsets of the pull of a cell within a direction's plane: the sum
+// of the parts for ex, ey and ez ([e + 1]).
+struct Pull {
+    unsigned x[3], y[3], z[3];
+    __device__ __forceinline__ Pull(int nx, int ny, int nz, int i, int j, int k)
+    {
+        const unsigned row = (unsigned)nz, sheet = (unsigned)ny * (unsigned)nz;
+        x[0] = (unsigned)(i == nx - 1 ? 0 : i + 1) * sheet;
+        x[1] = (unsigned)i * sheet;
+        x[2] = (unsigned)(i == 0 ? nx - 1 : i - 1) * sheet;
+        y[0] = (unsigned)(j == ny - 1 ? 0 : j + 1) * row;
+        y[1] = (unsigned)j * row;
+        y[2] = (unsigned)(j == 0 ? ny - 1 : j - 1) * row;
+        z[0] = (unsigned)(k == nz - 1 ? 0 : k + 1);
+        z[1] = (unsigned)k;
+        z[2] = (unsigned)(k == 0 ? nz - 1 : k - 1);
+    }
+    __device__ __forceinline__ unsigned at(int a) const { return x[ex(a, 0) + 1] + y[ex(a, 1) + 1] + z[ex(a, 2) + 1]; }
+};
+
+// A thread's pair is two neighbours, cells 2 t and 2 t + 1 of its CTA's
+// kCells (kNear), or cells t and t + kThreads.  Float32 results of an odd number of
+// cells lie off their 8-byte boundary in every other direction: there the
+// second form keeps lanes on consecutive cells, so that the 4-byte accesses
+// coalesce (61 x 65 x 63: 10.3 us against 12.3; 64^3 8.4 in the first form,
+// 10.3 in the second).
+template <bool kNear>
+__device__ __forceinline__ unsigned first_cell(unsigned block, unsigned t)
+{
+    return block * kCells + (kNear ? 2 * t : t);
+}
+
+// Fused step of the pair whose first cell is c < plane (the second may lie
+// beyond the last cell) of a lattice of fewer than 2^32 cells.  kNear as
+// above; float16 pairs are neighbours.
+template <int P, bool kNear>
+__device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __restrict__ src,
+                                          typename lowp::Storage<P>::T* __restrict__ dst, int nx, int ny, int nz,
+                                          size_t plane, unsigned c, const CollideF32& cp)
+{
+    static_assert(kNear || P == IMEX_F32, "float16 pairs share a random word");
+    using S = lowp::Storage<P>;
+    using T = typename S::T;
+    using A = lowp::F2;
+    constexpr unsigned kNext = kNear ? 1 : kThreads;
+    const bool two = c + kNext < (unsigned)plane;
+    auto pull_of = [&](unsigned cell) {
+        const unsigned row = cell / (unsigned)nz, i = row / (unsigned)ny;
+        return Pull(nx, ny, nz, (int)i, (int)(row - i * (unsigned)ny), (int)(cell - row * (unsigned)nz));
+    };
+    const Pull p0 = pull_of(c), p1 = pull_of(two ? c + kNext : c);
+    float2 h[kQ];
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+        const T* p = src + (size_t)a * plane;
+        const T v0 = __ldg(p + p0.at(a)), v1 = __ldg(p + p1.at(a));
+        h[a] = make_float2(S::dev(v0, a), S::dev(v1, a));
+    }
+    lowp::collide_dev<P, A>(h, cp);
+    T* const o = dst + c;
+    if constexpr (P == IMEX_F16DEV) {
+        // an odd number of cells puts every other direction's pairs off their
+        // 4-byte boundary
+        const bool whole = two && !(plane & 1);
+        auto put = [&](int a, __half2 r) {
+            T* const q = o + (size_t)a * plane;
+            if (whole) {
+                *reinterpret_cast<__half2*>(q) = r;
+            } else {
+                q[0] = __low2half(r);
+                if (two) q[1] = __high2half(r);
+            }
+        };
+        if (cp.sr) {
+            const uint32_t ph = lowp::sr_hash(c >> 1, cp.seed), pc = lowp::sr_corner_hash(ph);
+            lowp::round_f16_conserving<A>(h, [&](int a, float2 v) -> float2 {
+                const uint32_t w = lowp::cvt_rs_f16x2(v.y, v.x, lowp::sr_word(ph, pc, a));
+                const __half2 r = *reinterpret_cast<const __half2*>(&w);
+                put(a, r);
+                return make_float2(lowp::sub_f16_f32(__low2half(r), v.x), lowp::sub_f16_f32(__high2half(r), v.y));
+            });
+        } else {
+            lowp::round_f16_conserving<A>(h, [&](int a, float2 v) -> float2 {
+                const __half2 r = __floats2half2_rn(v.x, v.y);
+                put(a, r);
+                return make_float2(lowp::sub_f16_f32(__low2half(r), v.x), lowp::sub_f16_f32(__high2half(r), v.y));
+            });
+        }
+    } else {
+#pragma unroll
+        for (int a = 0; a < kQ; ++a) {
+            T* const q = o + (size_t)a * plane;
+            const float2 v = make_float2(S::store(h[a].x, a), S::store(h[a].y, a));
+            if (kNear && two) {  // plane even: 8-byte aligned
+                *reinterpret_cast<float2*>(q) = v;
+            } else {
+                q[0] = v.x;
+                if (two) q[kNext] = v.y;
+            }
+        }
+    }
+}
+
+}  // namespace flat
+}  // namespace imex

@@ -8,6 +8,7 @@
 #include <cuda_fp16.h>
 
 #include "conserved.cuh"
+#include "flat_lowp.cuh"
 #include "kernels_lowp.cuh"
 #include "lowp_math.cuh"
 #include "rows.cuh"
@@ -21,7 +22,8 @@ namespace {
 using lowp::Storage;
 using lowp::collide_dev_f32;
 
-template <int P, bool PULL, bool COLLIDE>
+// Collision in place (src == dst), or streaming alone.
+template <int P, bool COLLIDE>
 __global__ void __launch_bounds__(kStepBlock) k_step_lowp(const typename Storage<P>::T* src, typename Storage<P>::T* dst,
                                                           Geom g, CollideF32 cp)
 {
@@ -29,22 +31,17 @@ __global__ void __launch_bounds__(kStepBlock) k_step_lowp(const typename Storage
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, i = blockIdx.z;
     if (k >= g.nz) return;
-    const PullIndex pi(g, i, j, k, PULL);
     const size_t cell = ((size_t)i * g.ny + j) * g.nz + k;
     if constexpr (!COLLIDE) {
         // streaming alone moves the stored bits unchanged
+        const PullIndex pi(g, i, j, k, true);
 #pragma unroll
         for (int a = 0; a < kQ; ++a) dst[(size_t)a * g.plane + cell] = src[pi.at_dyn(g, a)];
         return;
     }
     float h[kQ];
-    if constexpr (PULL) {
 #pragma unroll
-        for (int a = 0; a < kQ; ++a) h[a] = S::load(src + pi.at_dyn(g, a), a);
-    } else {
-#pragma unroll
-        for (int a = 0; a < kQ; ++a) h[a] = S::load_plain(src + (size_t)a * g.plane + cell, a);
-    }
+    for (int a = 0; a < kQ; ++a) h[a] = S::load_plain(src + (size_t)a * g.plane + cell, a);
     collide_dev_f32<P>(h, cp);
     if constexpr (P == IMEX_F16DEV) {
         auto at = [&](int a) -> __half& { return dst[(size_t)a * g.plane + cell]; };
@@ -53,6 +50,18 @@ __global__ void __launch_bounds__(kStepBlock) k_step_lowp(const typename Storage
 #pragma unroll
         for (int a = 0; a < kQ; ++a) dst[(size_t)a * g.plane + cell] = S::store(h[a], a);
     }
+}
+
+// The fused step over flat cell pairs (flat_lowp.cuh).
+template <int P, bool kNear, bool SR>
+__global__ void __launch_bounds__(flat::kThreads) k_flat_lowp(const typename Storage<P>::T* __restrict__ src,
+                                                              typename Storage<P>::T* __restrict__ dst, Geom g,
+                                                              CollideF32 cp)
+{
+    const unsigned c = flat::first_cell<kNear>(blockIdx.x, threadIdx.x);
+    if (c >= (unsigned)g.plane) return;
+    cp.sr = SR;
+    flat::step_pair<P, kNear>(src, dst, g.nx, g.ny, g.nz, g.plane, c, cp);
 }
 
 // Taylor-Green initial state (float64 equilibrium, src/lbm.cpp:78-108),
@@ -159,9 +168,20 @@ cudaError_t step_impl(int mode, const void* src, void* dst, const Geom& g, const
     const T* a = static_cast<const T*>(src);
     T* b = static_cast<T*>(dst);
     switch (mode) {
-    case kModeFused: k_step_lowp<P, true, true><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
-    case kModeCollide: k_step_lowp<P, false, true><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
-    case kModeStream: k_step_lowp<P, true, false><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
+    case kModeFused: {
+        if (g.plane > 0xffffffffull - flat::kCells) return cudaErrorInvalidValue;  // above device memory
+        const unsigned grid = (unsigned)((g.plane + flat::kCells - 1) / flat::kCells);
+        if constexpr (P == IMEX_F16DEV) {
+            if (cp.sr) k_flat_lowp<P, true, true><<<grid, flat::kThreads, 0, s>>>(a, b, g, cp);
+            else k_flat_lowp<P, true, false><<<grid, flat::kThreads, 0, s>>>(a, b, g, cp);
+        } else {
+            if (g.plane & 1) k_flat_lowp<P, false, false><<<grid, flat::kThreads, 0, s>>>(a, b, g, cp);
+            else k_flat_lowp<P, true, false><<<grid, flat::kThreads, 0, s>>>(a, b, g, cp);
+        }
+        break;
+    }
+    case kModeCollide: k_step_lowp<P, true><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
+    case kModeStream: k_step_lowp<P, false><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -332,7 +332,7 @@ int imex_batch_synchronize(imex_batch *b);
 /* Pin the launch shape of the one-thread-per-cell kernel: a persistent
  * grid (threads 128|256, cells_per_thread 1|2|4, ctas_per_sm * threads <=
  * 2048; CTAs beyond those that can be resident are not launched), or
- * cells_per_thread 0 with threads 128 - one CTA per 128-cell row segment of
+ * cells_per_thread 0 with threads 128 - one CTA per 256-cell segment of
  * every member, the one-lattice kernel's grid over the whole batch (its
  * CUDA graph is captured again when the members' segment count changes).
  * threads = 0 retunes. */
