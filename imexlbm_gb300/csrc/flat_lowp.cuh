@@ -28,26 +28,6 @@ namespace flat {
 constexpr int kThreads = 128;
 constexpr int kCells = 2 * kThreads;  // cells of a CTA
 
-// Source offsets of the pull of a cell within a direction's plane: the sum
-// of the parts for ex, ey and ez ([e + 1]).
-struct Pull {
-    unsigned x[3], y[3], z[3];
-    __device__ __forceinline__ Pull(int nx, int ny, int nz, int i, int j, int k)
-    {
-        const unsigned row = (unsigned)nz, sheet = (unsigned)ny * (unsigned)nz;
-        x[0] = (unsigned)(i == nx - 1 ? 0 : i + 1) * sheet;
-        x[1] = (unsigned)i * sheet;
-        x[2] = (unsigned)(i == 0 ? nx - 1 : i - 1) * sheet;
-        y[0] = (unsigned)(j == ny - 1 ? 0 : j + 1) * row;
-        y[1] = (unsigned)j * row;
-        y[2] = (unsigned)(j == 0 ? ny - 1 : j - 1) * row;
-        z[0] = (unsigned)(k == nz - 1 ? 0 : k + 1);
-        z[1] = (unsigned)k;
-        z[2] = (unsigned)(k == 0 ? nz - 1 : k - 1);
-    }
-    __device__ __forceinline__ unsigned at(int a) const { return x[ex(a, 0) + 1] + y[ex(a, 1) + 1] + z[ex(a, 2) + 1]; }
-};
-
 // A thread's pair is two neighbours, cells 2 t and 2 t + 1 of its CTA's
 // kCells (kNear), or cells t and t + kThreads.  Float32 results of an odd number of
 // cells lie off their 8-byte boundary in every other direction: there the
@@ -74,11 +54,7 @@ __device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __
     using A = lowp::F2;
     constexpr unsigned kNext = kNear ? 1 : kThreads;
     const bool two = c + kNext < (unsigned)plane;
-    auto pull_of = [&](unsigned cell) {
-        const unsigned row = cell / (unsigned)nz, i = row / (unsigned)ny;
-        return Pull(nx, ny, nz, (int)i, (int)(row - i * (unsigned)ny), (int)(cell - row * (unsigned)nz));
-    };
-    const Pull p0 = pull_of(c), p1 = pull_of(two ? c + kNext : c);
+    const FlatPull p0(nx, ny, nz, c), p1(nx, ny, nz, two ? c + kNext : c);
     float2 h[kQ];
 #pragma unroll
     for (int a = 0; a < kQ; ++a) {

@@ -73,6 +73,29 @@ struct PullIndex {
     }
 };
 
+// The same for a cell given by its flat index (z fastest) in a lattice of
+// fewer than 2^32 cells: the source offset within a direction's plane is the
+// sum of a part for each of ex, ey and ez ([e + 1]).
+struct FlatPull {
+    unsigned x[3], y[3], z[3];
+    __device__ __forceinline__ FlatPull(int nx, int ny, int nz, unsigned cell)
+    {
+        const unsigned row = cell / (unsigned)nz, k = cell - row * (unsigned)nz;
+        const unsigned i = row / (unsigned)ny, j = row - i * (unsigned)ny;
+        const unsigned sheet = (unsigned)ny * (unsigned)nz;
+        x[0] = (i == (unsigned)nx - 1 ? 0 : i + 1) * sheet;
+        x[1] = i * sheet;
+        x[2] = (i == 0 ? (unsigned)nx - 1 : i - 1) * sheet;
+        y[0] = (j == (unsigned)ny - 1 ? 0 : j + 1) * (unsigned)nz;
+        y[1] = j * (unsigned)nz;
+        y[2] = (j == 0 ? (unsigned)ny - 1 : j - 1) * (unsigned)nz;
+        z[0] = k == (unsigned)nz - 1 ? 0 : k + 1;
+        z[1] = k;
+        z[2] = k == 0 ? (unsigned)nz - 1 : k - 1;
+    }
+    __device__ __forceinline__ unsigned at(int a) const { return x[ex(a, 0) + 1] + y[ex(a, 1) + 1] + z[ex(a, 2) + 1]; }
+};
+
 template <int A, typename T>
 __device__ __forceinline__ T ldg_pull(const T* __restrict__ src, const Geom& g, const PullIndex& p)
 {
