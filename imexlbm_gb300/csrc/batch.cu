@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kUnitThreads) k_batch_units(const BatchHeader*
         using T = typename lowp::Storage<P>::T;
         const unsigned c = flat::first_cell<kNear>(seg, threadIdx.x);
         if (c < (unsigned)e.plane)
-            flat::step_pair<P, kNear>(static_cast<const T*>(src), static_cast<T*>(dst), e.nx, e.ny, e.nz, e.plane, c, cp);
+            flat::step_pair<P, kNear, true>(static_cast<const T*>(src), static_cast<T*>(dst), e.nx, e.ny, e.nz, e.plane, c, cp);
     };
     if (PF != IMEX_F32 && e.prec == IMEX_F16DEV) {
         cp.sr = e.sr;
@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(rowslp::kThreads, kMinBlocks)
                  int stages, int table_cap, WaitCtl wc)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    chain_begin<true>();
     const int count = hdr->count;
     if (count > table_cap) {  // the table would not fit the shared memory the launch has
         if (threadIdx.x == 0) atomicOr(wc.err, 2u);
@@ -338,12 +339,16 @@ __global__ void __launch_bounds__(two::kThreads, 1)
                   const int* __restrict__ group, int s, CollideF32 base, WaitCtl wc)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    chain_next();
     const unsigned item = blockIdx.x;
     const int count = hdr->count;
     int m = group[item / kPairGroup];
     while (m + 1 < count && tab[m + 1].begin <= item) ++m;
     const PairEntry& e = tab[m];
-    if (s + 1 >= e.steps) return;
+    if (s + 1 >= e.steps) {
+        chain_wait();
+        return;
+    }
     const int cur = e.cur ^ ((s >> 1) & 1);
     CollideF32 cp = base;
     cp.eps = e.eps;
@@ -546,11 +551,8 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
         if (sh.cpt == 0) {  // one CTA per segment
             const unsigned long long units = b->h_hdr->total;
             if (units == 0 || units > 0x7fffffffull) return cudaErrorInvalidValue;
-            if (f32)
-                k_batch_units<IMEX_F32><<<(unsigned)units, kUnitThreads, 0, b->stream>>>(b->d_hdr, b->d_tab, b->d_group, s,
-                                                                                     base);
-            else
-                k_batch_units<0><<<(unsigned)units, kUnitThreads, 0, b->stream>>>(b->d_hdr, b->d_tab, b->d_group, s, base);
+            auto* fn = f32 ? k_batch_units<IMEX_F32> : k_batch_units<0>;
+            fn<<<(unsigned)units, kUnitThreads, 0, b->stream>>>(b->d_hdr, b->d_tab, b->d_group, s, base);
             e = cudaGetLastError();
         } else if (f32 && sh.cpt == 1 && sh.threads == 128) e = launch_cells<1, IMEX_F32, 128, 9>(b, sh, s, base);
         else if (sh.cpt == 1) e = f32 ? launch_cells<1, IMEX_F32>(b, sh, s, base) : launch_cells<1, 0>(b, sh, s, base);
@@ -571,7 +573,8 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
         const int cap = test_fault_kind() == IMEX_TEST_FAULT_BATCH_TABLE ? b->n_row - 1 : b->capacity;
         const WaitCtl wc = make_wait_ctl(b->d_err);
 #define IMEX_BATCH_ROWS(D, M) \
-    k_batch_rows<D, M><<<grid, rowslp::kThreads, smem, b->stream>>>(b->d_rhdr, b->d_rtab, s, base, rs.stages, cap, wc)
+    return launch_chained(k_batch_rows<D, M>, grid, rowslp::kThreads, smem, b->stream, b->d_rhdr, b->d_rtab, s, base, \
+                          rs.stages, cap, wc)
         switch (rs.dir_kb) {
         case 1:
             if (one) IMEX_BATCH_ROWS(1024, 1);
@@ -585,7 +588,6 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
         default: return cudaErrorInvalidValue;
         }
 #undef IMEX_BATCH_ROWS
-        return cudaGetLastError();
     }
     return cudaSuccess;
 }
@@ -593,9 +595,8 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
 // Steps s and s + 1 of the two-step kernel's members.
 cudaError_t launch_pairs(imex_batch* b, int s)
 {
-    k_batch_pairs<<<b->pair_items, two::kThreads, two::kSmemBytes, b->stream>>>(b->phdr.d, b->ptab.d, b->pmaps.d, b->pgroup.d, s,
-                                                                               base_constants(), make_wait_ctl(b->d_err));
-    return cudaGetLastError();
+    return launch_chained(k_batch_pairs, b->pair_items, two::kThreads, two::kSmemBytes, b->stream, b->phdr.d, b->ptab.d,
+                          b->pmaps.d, b->pgroup.d, s, base_constants(), make_wait_ctl(b->d_err));
 }
 
 // The odd last step of its members, after their pairs.

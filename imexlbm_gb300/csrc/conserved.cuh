@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(kThreads, MINB)
 {
     __shared__ BlockSum s;
     __shared__ int s_last;
+    chain_begin<true>();
     Int128 m[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
     double ke = 0.0, sums[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     int any = 0;
@@ -210,9 +211,8 @@ cudaError_t launch(bool pull, const void* src, const Geom& g, void* part, unsign
     const unsigned grid = blocks_for(cells, current_sm_count(), MINB);
     const auto* p = static_cast<const typename mom::Elem<P>::T*>(src);
     auto* pt = static_cast<Partial*>(part);
-    if (pull) k_conserved<P, true, MINB><<<grid, kThreads, 0, s>>>(p, g, (unsigned)cells, pt, ticket, out);
-    else k_conserved<P, false, MINB><<<grid, kThreads, 0, s>>>(p, g, (unsigned)cells, pt, ticket, out);
-    return cudaGetLastError();
+    return pull ? launch_chained(k_conserved<P, true, MINB>, grid, kThreads, 0, s, p, g, (unsigned)cells, pt, ticket, out)
+                : launch_chained(k_conserved<P, false, MINB>, grid, kThreads, 0, s, p, g, (unsigned)cells, pt, ticket, out);
 }
 
 }  // namespace cons

@@ -42,8 +42,8 @@ __device__ __forceinline__ unsigned first_cell(unsigned block, unsigned t)
 
 // Fused step of the pair whose first cell is c < plane (the second may lie
 // beyond the last cell) of a lattice of fewer than 2^32 cells.  kNear as
-// above; float16 pairs are neighbours.
-template <int P, bool kNear>
+// above; float16 pairs are neighbours.  Ends its kernel's chain (chain_end).
+template <int P, bool kNear, bool kEarly>
 __device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __restrict__ src,
                                           typename lowp::Storage<P>::T* __restrict__ dst, int nx, int ny, int nz,
                                           size_t plane, unsigned c, const CollideF32& cp)
@@ -63,6 +63,7 @@ __device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __
         h[a] = make_float2(S::dev(v0, a), S::dev(v1, a));
     }
     lowp::collide_dev<P, A>(h, cp);
+    chain_end<kEarly>();
     T* const o = dst + c;
     if constexpr (P == IMEX_F16DEV) {
         // an odd number of cells puts every other direction's pairs off their

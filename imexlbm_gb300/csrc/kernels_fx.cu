@@ -111,11 +111,12 @@ __global__ void __launch_bounds__(kStepBlock, 5) k_collide_fx(double* __restrict
 //
 // FLAT: a thread's cell is its place in the flat order (z fastest) instead
 // of a place in the CTA's row segment.
-template <bool OM_GE1, bool IN_FX, bool OUT_FX, bool FLAT>
+template <bool OM_GE1, bool IN_FX, bool OUT_FX, bool FLAT, bool EARLY>
 __global__ void __launch_bounds__(kStepBlock, 5)
     k_step_fxs(const unsigned long long* __restrict__ src, unsigned long long* __restrict__ dst, Geom g, FxConst c,
                int j, int* __restrict__ fail)
 {
+    chain_begin<EARLY>();
     if (*fail < j) return;  // an earlier step of the run failed
     uint64_t in[kQ], out[kQ];
     size_t cell;
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(kStepBlock, 5)
     }
     bool ok = true;
     fx::collide_cell_io<OM_GE1, IN_FX, OUT_FX>(in, out, c, ok);
+    chain_end<EARLY>();
 #pragma unroll
     for (int a = 0; a < kQ; ++a) dst[(size_t)a * g.plane + cell] = out[a];
     if (!ok) atomicMin(fail, j);
@@ -350,18 +352,26 @@ __global__ void k_fx_to_f64(unsigned long long* __restrict__ buf, size_t n)
     }
 }
 
+template <bool OM_GE1, bool FLAT, bool EARLY>
+cudaError_t launch_fxs_as(dim3 grid, unsigned bs, const unsigned long long* src, unsigned long long* dst, const Geom& g,
+                          const FxConst& c, int j, int n, int* fail, cudaStream_t s)
+{
+    const bool in_fx = j > 1, out_fx = j < n;
+    if (in_fx && out_fx) return launch_chained(k_step_fxs<OM_GE1, true, true, FLAT, EARLY>, grid, bs, 0, s, src, dst, g, c, j, fail);
+    if (in_fx) return launch_chained(k_step_fxs<OM_GE1, true, false, FLAT, EARLY>, grid, bs, 0, s, src, dst, g, c, j, fail);
+    if (out_fx) return launch_chained(k_step_fxs<OM_GE1, false, true, FLAT, EARLY>, grid, bs, 0, s, src, dst, g, c, j, fail);
+    return launch_chained(k_step_fxs<OM_GE1, false, false, FLAT, EARLY>, grid, bs, 0, s, src, dst, g, c, j, fail);
+}
+
 template <bool OM_GE1, bool FLAT>
 cudaError_t launch_fxs(const unsigned long long* src, unsigned long long* dst, const Geom& g, const FxConst& c, int j,
                        int n, int* fail, cudaStream_t s)
 {
     const unsigned bs = FLAT ? kStepBlock : row_block(g.nz);
     const dim3 grid = FLAT ? dim3((unsigned)((g.plane + kStepBlock - 1) / kStepBlock)) : dim3((g.nz + bs - 1) / bs, g.ny, g.nx);
-    const bool in_fx = j > 1, out_fx = j < n;
-    if (in_fx && out_fx) k_step_fxs<OM_GE1, true, true, FLAT><<<grid, bs, 0, s>>>(src, dst, g, c, j, fail);
-    else if (in_fx) k_step_fxs<OM_GE1, true, false, FLAT><<<grid, bs, 0, s>>>(src, dst, g, c, j, fail);
-    else if (out_fx) k_step_fxs<OM_GE1, false, true, FLAT><<<grid, bs, 0, s>>>(src, dst, g, c, j, fail);
-    else k_step_fxs<OM_GE1, false, false, FLAT><<<grid, bs, 0, s>>>(src, dst, g, c, j, fail);
-    return cudaGetLastError();
+    return chain_early((unsigned long long)grid.x * grid.y * grid.z)
+               ? launch_fxs_as<OM_GE1, FLAT, true>(grid, bs, src, dst, g, c, j, n, fail, s)
+               : launch_fxs_as<OM_GE1, FLAT, false>(grid, bs, src, dst, g, c, j, n, fail, s);
 }
 
 // Native float64 redo of one cell of a staged row.

@@ -53,15 +53,16 @@ __global__ void __launch_bounds__(kStepBlock) k_step_lowp(const typename Storage
 }
 
 // The fused step over flat cell pairs (flat_lowp.cuh).
-template <int P, bool kNear, bool SR>
+template <int P, bool kNear, bool SR, bool kEarly>
 __global__ void __launch_bounds__(flat::kThreads) k_flat_lowp(const typename Storage<P>::T* __restrict__ src,
                                                               typename Storage<P>::T* __restrict__ dst, Geom g,
                                                               CollideF32 cp)
 {
+    chain_begin<kEarly>();
     const unsigned c = flat::first_cell<kNear>(blockIdx.x, threadIdx.x);
     if (c >= (unsigned)g.plane) return;
     cp.sr = SR;
-    flat::step_pair<P, kNear>(src, dst, g.nx, g.ny, g.nz, g.plane, c, cp);
+    flat::step_pair<P, kNear, kEarly>(src, dst, g.nx, g.ny, g.nz, g.plane, c, cp);
 }
 
 // Taylor-Green initial state (float64 equilibrium, src/lbm.cpp:78-108),
@@ -171,14 +172,15 @@ cudaError_t step_impl(int mode, const void* src, void* dst, const Geom& g, const
     case kModeFused: {
         if (g.plane > 0xffffffffull - flat::kCells) return cudaErrorInvalidValue;  // above device memory
         const unsigned grid = (unsigned)((g.plane + flat::kCells - 1) / flat::kCells);
+        const bool early = chain_early(grid);
+        auto go = [&](auto kernel) { return launch_chained(kernel, grid, flat::kThreads, 0, s, a, b, g, cp); };
         if constexpr (P == IMEX_F16DEV) {
-            if (cp.sr) k_flat_lowp<P, true, true><<<grid, flat::kThreads, 0, s>>>(a, b, g, cp);
-            else k_flat_lowp<P, true, false><<<grid, flat::kThreads, 0, s>>>(a, b, g, cp);
+            if (cp.sr) return early ? go(k_flat_lowp<P, true, true, true>) : go(k_flat_lowp<P, true, true, false>);
+            return early ? go(k_flat_lowp<P, true, false, true>) : go(k_flat_lowp<P, true, false, false>);
         } else {
-            if (g.plane & 1) k_flat_lowp<P, false, false><<<grid, flat::kThreads, 0, s>>>(a, b, g, cp);
-            else k_flat_lowp<P, true, false><<<grid, flat::kThreads, 0, s>>>(a, b, g, cp);
+            if (g.plane & 1) return early ? go(k_flat_lowp<P, false, false, true>) : go(k_flat_lowp<P, false, false, false>);
+            return early ? go(k_flat_lowp<P, true, false, true>) : go(k_flat_lowp<P, true, false, false>);
         }
-        break;
     }
     case kModeCollide: k_step_lowp<P, true><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
     case kModeStream: k_step_lowp<P, false><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
@@ -251,9 +253,8 @@ cudaError_t launch_rows_lowp_d(int prec, const void* src, void* dst, const Geom&
         if (e != cudaSuccess) return e;
         if (dev < 64) allowed[dev].store((int)smem);
     }
-    rowslp::k_rows_lowp<D, MINB><<<grid, rowslp::kThreads, smem, s>>>(src, dst, g, prec, rc.rows, cp, rc.stages,
-                                                                       make_wait_ctl(err));
-    return cudaGetLastError();
+    return launch_chained(rowslp::k_rows_lowp<D, MINB>, grid, rowslp::kThreads, smem, s, src, dst, g, prec, rc.rows, cp,
+                          rc.stages, make_wait_ctl(err));
 }
 
 cudaError_t launch_rows_lowp(int prec, const void* src, void* dst, const Geom& g, const CollideF32& cp,

@@ -315,6 +315,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
                 int stages, WaitCtl wc)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    chain_begin<true>();  // the ring leaves the next launch's CTAs no room before this one's end
     const int yblocks = y_blocks(g.ny, B);
     const int items = g.nx * yblocks;
     const int G = gridDim.x;

@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               CollideF32 cp, WaitCtl wc)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    chain_next();
     run_box<false>(&maps, src, dst, g.nx, g.ny, g.nz, g.plane, box_of(p, g.nx, g.ny, g.nz, blockIdx.x), cp, smem, wc);
 }
 
@@ -136,8 +137,8 @@ cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, La
 cudaError_t launch(const Lattice& l, int from, const float* src, float* dst, const Geom& g, const CollideF32& cp,
                    unsigned* err, cudaStream_t s)
 {
-    k_two_f32<<<(unsigned)l.plan.items(), kThreads, kSmemBytes, s>>>(l.maps[from], src, dst, g, l.plan, cp, make_wait_ctl(err));
-    return cudaGetLastError();
+    return launch_chained(k_two_f32, (unsigned)l.plan.items(), kThreads, kSmemBytes, s, l.maps[from], src, dst, g, l.plan,
+                          cp, make_wait_ctl(err));
 }
 
 }  // namespace two

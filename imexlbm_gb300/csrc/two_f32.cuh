@@ -151,7 +151,9 @@ __device__ __forceinline__ void cp16(void* dst, const void* src)
 // kernel's parameters.  Every wait
 // on an mbarrier is bounded: one that runs out sets wc.err, the loaders stop
 // bringing planes, and the CTA runs to its end on what the stages hold (its
-// results are reported invalid).
+// results are reported invalid).  The set-up before the roles' loops touches
+// no lattice, so each role waits for the kernels before (chain_wait) only then;
+// the caller has let the next kernel in.
 template <bool kMapsInMemory>
 __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const float* __restrict__ src,
                                         float* __restrict__ dst, int nx, int ny, int nz, size_t plane, const Box& b,
@@ -239,6 +241,7 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
                 }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bulk::smem_u32(mb)) : "memory");
         };
+        chain_wait();
         int brought = 0;
         bool good = true;
         for (int i = 0; i < last; ++i) {
@@ -264,6 +267,7 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
             pa = q == 0 ? side0 + r * 8 + 2 : r * kTileZ + 2 * q - 2;
             pb = q == half ? side0 + r * 8 + 4 : r * kTileZ + 2 * q;
         }
+        chain_wait();
         bool good = true;
         int s2 = 0, s3 = 0;  // ring slots of this plane's ex = 0 and ex = +1 values
         for (int i = 0; i < last + 1; ++i) {
@@ -319,6 +323,7 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
         pos = (r + 1) * W + 2 * q;
         to = (unsigned)(b.y0 + r) * (unsigned)nz + (unsigned)(b.z0 + 2 * q);
     }
+    chain_wait();
     int s2 = 0, s3 = 0;  // slots of middle planes i - 2 (ex = 0) and i - 3 (ex = +1): those plane i is about to take
     for (int i = 0; i < last + 1; ++i) {
         float2 h[kQ];
