@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, MINB)
         mom::cell_of(g, (unsigned)q, i, j, k);
         const PullIndex pi(g, i, j, k, PULL);
         mom::Cell<P> c;
-        if (mom::moments<P, true>(src, g, pi, c)) {
+        if (mom::moments<P, false>(src, g, pi, c)) {
 #pragma unroll
             for (int d = 0; d < 4; ++d) m[d].add((long long)c.M[d]);
 #pragma unroll

@@ -121,50 +121,6 @@ __global__ void __launch_bounds__(1024) k_reduce_partials(const double* __restri
         for (int q = 0; q < 5; ++q) out[q] = v[q];
 }
 
-// Per-cell p, u, v, w (src/lbm.cpp:218-236).
-template <bool PULL>
-__global__ void __launch_bounds__(kStepBlock) k_macro_f64(const double* __restrict__ src, Geom g, double* __restrict__ p,
-                                                          double* __restrict__ u, double* __restrict__ v, double* __restrict__ w)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
-    if (k >= g.nz) return;
-    const PullIndex pi(g, i, j, k, PULL);
-    double f[kQ];
-    gather27<double>(src, g, pi, f);
-    double pl, ul, vl, wl;
-    moments_f64(f, pl, ul, vl, wl);
-    const size_t cell = ((size_t)i * g.ny + j) * g.nz + k;
-    if (p) p[cell] = pl * (1.0 / 3.0);
-    u[cell] = ul;
-    v[cell] = vl;
-    w[cell] = wl;
-}
-
-// max over cells of |a - b| and of |b| for three component arrays of n
-// values; results as the bit patterns of non-negative doubles (ordered like
-// unsigned integers), combined with atomicMax.
-__global__ void k_maxdiff3(const double* __restrict__ a, const double* __restrict__ b, size_t n,
-                           unsigned long long* __restrict__ out)
-{
-    double md = 0.0, mb = 0.0;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            md = fmax(md, fabs(a[c * n + q] - b[c * n + q]));
-            mb = fmax(mb, fabs(b[c * n + q]));
-        }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        md = fmax(md, __shfl_down_sync(0xffffffffu, md, o));
-        mb = fmax(mb, __shfl_down_sync(0xffffffffu, mb, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(out, (unsigned long long)__double_as_longlong(md));
-        atomicMax(out + 1, (unsigned long long)__double_as_longlong(mb));
-    }
-}
-
 // ---------------------------------------------------------------- launchers --
 static dim3 step_grid(const Geom& g) { return dim3((g.nz + kStepBlock - 1) / kStepBlock, g.ny, g.nx); }
 
@@ -206,24 +162,6 @@ cudaError_t launch_conserved_f64(bool pull, const double* src, const Geom& g, do
 cudaError_t launch_reduce_partials(const double* partial, size_t n, double* out, cudaStream_t s)
 {
     k_reduce_partials<<<1, 1024, 0, s>>>(partial, n, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_macro_f64(bool pull, const double* src, const Geom& g, double* p, double* u, double* v, double* w,
-                             cudaStream_t s)
-{
-    if (pull)
-        k_macro_f64<true><<<step_grid(g), kStepBlock, 0, s>>>(src, g, p, u, v, w);
-    else
-        k_macro_f64<false><<<step_grid(g), kStepBlock, 0, s>>>(src, g, p, u, v, w);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_maxdiff3(const double* a, const double* b, size_t n, unsigned long long* out, cudaStream_t s)
-{
-    cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
-    k_maxdiff3<<<current_sm_count() * 8, 256, 0, s>>>(a, b, n, out);
     return cudaGetLastError();
 }
 

@@ -11,6 +11,7 @@
 #include "flat_lowp.cuh"
 #include "kernels_lowp.cuh"
 #include "lowp_math.cuh"
+#include "macro.cuh"
 #include "rows.cuh"
 #include "rows_lowp.cuh"
 #include "tg_init.cuh"
@@ -129,35 +130,6 @@ __global__ void __launch_bounds__(kStepBlock) k_to_f64(const typename Storage<P>
     for (int a = 0; a < kQ; ++a)
         out[(size_t)a * g.plane + cell] = Storage<P>::to_f64_exact(__ldg(src + pi.at_dyn(g, a)), a, ok);
     if (!ok) to_f64_cell_wide<P>(src, g, i, j, k, PULL, cell, out);
-}
-
-// Per-cell p, u, v, w in float64 from the stored values (src/lbm.cpp:218-236).
-template <int P, bool PULL>
-__global__ void __launch_bounds__(kStepBlock) k_macro_lowp(const typename Storage<P>::T* __restrict__ src, Geom g,
-                                                           double* __restrict__ p, double* __restrict__ u,
-                                                           double* __restrict__ v, double* __restrict__ w)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
-    if (k >= g.nz) return;
-    const PullIndex pi(g, i, j, k, PULL);
-    double pl = 0.0, ul = 0.0, vl = 0.0, wl = 0.0;
-#pragma unroll
-    for (int a = 0; a < kQ; ++a) {
-        const double fv = Storage<P>::to_f64(src[pi.at_dyn(g, a)], a);
-        pl += fv;
-        if (ex(a, 0) == 1) ul += fv;
-        if (ex(a, 0) == -1) ul -= fv;
-        if (ex(a, 1) == 1) vl += fv;
-        if (ex(a, 1) == -1) vl -= fv;
-        if (ex(a, 2) == 1) wl += fv;
-        if (ex(a, 2) == -1) wl -= fv;
-    }
-    const size_t cell = ((size_t)i * g.ny + j) * g.nz + k;
-    if (p) p[cell] = pl * (1.0 / 3.0);
-    u[cell] = ul;
-    v[cell] = vl;
-    w[cell] = wl;
 }
 
 dim3 step_grid(const Geom& g) { return dim3((g.nz + kStepBlock - 1) / kStepBlock, g.ny, g.nx); }
@@ -308,19 +280,32 @@ cudaError_t launch_to_f64(int prec, bool pull, const void* src, const Geom& g, d
     return cudaGetLastError();
 }
 
-cudaError_t launch_macro_lowp(int prec, bool pull, const void* src, const Geom& g, double* p, double* u, double* v,
-                              double* w, cudaStream_t s)
+cudaError_t launch_macro(int prec, bool pull, const void* src, const Geom& g, double* p, double* u, double* v, double* w,
+                         cudaStream_t s)
 {
-    if (prec == IMEX_F32) {
-        const float* q = static_cast<const float*>(src);
-        if (pull) k_macro_lowp<IMEX_F32, true><<<step_grid(g), kStepBlock, 0, s>>>(q, g, p, u, v, w);
-        else k_macro_lowp<IMEX_F32, false><<<step_grid(g), kStepBlock, 0, s>>>(q, g, p, u, v, w);
-    } else {
-        const __half* q = static_cast<const __half*>(src);
-        if (pull) k_macro_lowp<IMEX_F16DEV, true><<<step_grid(g), kStepBlock, 0, s>>>(q, g, p, u, v, w);
-        else k_macro_lowp<IMEX_F16DEV, false><<<step_grid(g), kStepBlock, 0, s>>>(q, g, p, u, v, w);
+    switch (prec) {
+    case IMEX_F64: return macro::launch<IMEX_F64>(pull, src, g, p, u, v, w, s);
+    case IMEX_F32: return macro::launch<IMEX_F32>(pull, src, g, p, u, v, w, s);
+    default: return macro::launch<IMEX_F16DEV>(pull, src, g, p, u, v, w, s);
     }
-    return cudaGetLastError();
+}
+
+cudaError_t launch_velocity_diff(int prec_a, const void* fa, bool pull_a, int prec_b, const void* fb, bool pull_b,
+                                 const Geom& g, unsigned long long* res, cudaStream_t s)
+{
+    cudaError_t e = cudaMemsetAsync(res, 0, 4 * sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    switch (3 * prec_a + prec_b) {
+    case 3 * IMEX_F64 + IMEX_F64: return macro::launch_diff<IMEX_F64, IMEX_F64>(fa, pull_a, fb, pull_b, g, res, s);
+    case 3 * IMEX_F64 + IMEX_F32: return macro::launch_diff<IMEX_F64, IMEX_F32>(fa, pull_a, fb, pull_b, g, res, s);
+    case 3 * IMEX_F64 + IMEX_F16DEV: return macro::launch_diff<IMEX_F64, IMEX_F16DEV>(fa, pull_a, fb, pull_b, g, res, s);
+    case 3 * IMEX_F32 + IMEX_F64: return macro::launch_diff<IMEX_F32, IMEX_F64>(fa, pull_a, fb, pull_b, g, res, s);
+    case 3 * IMEX_F32 + IMEX_F32: return macro::launch_diff<IMEX_F32, IMEX_F32>(fa, pull_a, fb, pull_b, g, res, s);
+    case 3 * IMEX_F32 + IMEX_F16DEV: return macro::launch_diff<IMEX_F32, IMEX_F16DEV>(fa, pull_a, fb, pull_b, g, res, s);
+    case 3 * IMEX_F16DEV + IMEX_F64: return macro::launch_diff<IMEX_F16DEV, IMEX_F64>(fa, pull_a, fb, pull_b, g, res, s);
+    case 3 * IMEX_F16DEV + IMEX_F32: return macro::launch_diff<IMEX_F16DEV, IMEX_F32>(fa, pull_a, fb, pull_b, g, res, s);
+    default: return macro::launch_diff<IMEX_F16DEV, IMEX_F16DEV>(fa, pull_a, fb, pull_b, g, res, s);
+    }
 }
 
 cudaError_t launch_conserved_lowp(int prec, bool pull, const void* src, const Geom& g, void* partial, unsigned* ticket,

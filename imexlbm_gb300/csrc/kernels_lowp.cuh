@@ -37,8 +37,13 @@ cudaError_t launch_step_lowp(int prec, int mode, const void* src, void* dst, con
 cudaError_t launch_from_f64(int prec, const double* f, void* out, const Geom& g, cudaStream_t s);
 // storage -> float64 reference-order f (pulled through streaming when `pull`)
 cudaError_t launch_to_f64(int prec, bool pull, const void* src, const Geom& g, double* out, cudaStream_t s);
-cudaError_t launch_macro_lowp(int prec, bool pull, const void* src, const Geom& g, double* p, double* u, double* v,
-                              double* w, cudaStream_t s);
+// Per-cell p (optional), u, v, w in any storage precision (macro.cuh).
+cudaError_t launch_macro(int prec, bool pull, const void* src, const Geom& g, double* p, double* u, double* v, double* w,
+                         cudaStream_t s);
+// Largest velocity difference of two lattices of one size: four values in
+// device memory (macro.cuh, k_velocity_diff).
+cudaError_t launch_velocity_diff(int prec_a, const void* fa, bool pull_a, int prec_b, const void* fb, bool pull_b,
+                                 const Geom& g, unsigned long long* res, cudaStream_t s);
 // Conserved sums (conserved.cuh): partial holds conserved_scratch_bytes(),
 // *ticket is 0 before and after the launch.
 cudaError_t launch_conserved_lowp(int prec, bool pull, const void* src, const Geom& g, void* partial, unsigned* ticket,

@@ -6,7 +6,8 @@
 //   float64 storage   the 27 values converted exactly (fx_math.cuh) and
 //                     summed exactly.
 //   reduced precision the deviations h = kScale (f - w) summed in float32,
-//                     pair by pair as the collision sums them; mass = 1 +
+//                     pair by pair as the collision sums them (or, EXACT,
+//                     the stored values exactly); mass = 1 +
 //                     sum h, momentum = sum h e.  The float32 sums are
 //                     multiples of 2^-37 or more for stored values of the
 //                     weights' size, so their conversion drops nothing.
@@ -37,14 +38,14 @@ struct Elem<IMEX_F64> {
     using T = double;
 };
 
-// x / 2^S in units of 2^-61, bits below dropped; clears ok for |x| >= 2^S
-// (NaN and Inf included).
-template <int S>
+// x / 2^S in units of 2^-61, bits below dropped; clears ok for |x| >= 2^(S -
+// LIM) (NaN and Inf included).
+template <int S, int LIM = 0>
 __device__ __forceinline__ int64_t fixed_of_float(float x, bool& ok)
 {
     const uint32_t b = __float_as_uint(x);
     const int e = (int)((b >> 23) & 255u);
-    ok = ok && e <= 126 + S;
+    ok = ok && e <= 126 + S - LIM;
     // mantissa * 2^(e - 150) * 2^61 / 2^S = (mantissa << 37) >> (126 + S - e)
     const int sh = 126 + S - e;
     const uint64_t v = ((uint64_t)((b & 0x007FFFFFu) | 0x00800000u) << 37) >> (sh < 63 ? sh : 63);
@@ -61,7 +62,9 @@ struct Cell {
 template <int P>
 inline constexpr int kVelBits = P == IMEX_F64 ? kBits : P == IMEX_F16DEV ? 12 : 0;
 
-template <int P, bool VEL>
+// EXACT (reduced precision): the stored values summed exactly instead of in
+// float32; the velocities in units of 2^-61.
+template <int P, bool EXACT>
 __device__ __forceinline__ bool moments(const typename Elem<P>::T* __restrict__ src, const Geom& g, const PullIndex& pi,
                                         Cell<P>& c)
 {
@@ -85,7 +88,38 @@ __device__ __forceinline__ bool moments(const typename Elem<P>::T* __restrict__ 
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             c.M[1 + d] = (int64_t)(A[d] - B[d]);
-            if (VEL) c.vel[d] = __ll2double_rn(c.M[1 + d]);
+            c.vel[d] = __ll2double_rn(c.M[1 + d]);
+        }
+    } else if constexpr (EXACT) {
+        // float32: f itself; float16: the deviations, the weights added after
+        int64_t S = 0, U[3] = {0, 0, 0};
+#pragma unroll
+        for (int a = 0; a < kQ; ++a) {
+            const auto v = __ldg(src + pi.at_dyn(g, a));
+            constexpr int S2 = P == IMEX_F32 ? 0 : Elem<P>::kScaleLog2;
+            float x;
+            if constexpr (P == IMEX_F32) x = v;
+            else x = __half2float(v);
+            // below 1/2 (rest) and 1/8: every sum below 2^63
+            const int64_t X = a == 0 ? fixed_of_float<S2, 1>(x, ok) : fixed_of_float<S2, 3>(x, ok);
+            S += X;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                if (ex(a, d) == 1) U[d] += X;
+                if (ex(a, d) == -1) U[d] -= X;
+            }
+        }
+        if constexpr (P == IMEX_F16DEV) {
+            uint64_t w = 0;
+#pragma unroll
+            for (int a = 0; a < kQ; ++a) w += lowp::weight_fixed(a);
+            S += (int64_t)w;
+        }
+        c.M[0] = S;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            c.M[1 + d] = U[d];
+            c.vel[d] = __ll2double_rn(U[d]);
         }
     } else {
         using A = lowp::F1;
@@ -110,7 +144,7 @@ __device__ __forceinline__ bool moments(const typename Elem<P>::T* __restrict__ 
                 if (e == -1) u = A::sub(u, d[q]);
             }
             c.M[1 + dim] = fixed_of_float<S>(u, ok);
-            if (VEL) c.vel[dim] = (double)u;
+            c.vel[dim] = (double)u;
         }
     }
     return ok;
