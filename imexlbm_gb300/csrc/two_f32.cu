@@ -107,17 +107,18 @@ Plan plan_tiles(const Geom& g, int planes)
     return p;
 }
 
-// Measured: a launch takes 4 us and 1.85 us per iteration of its busiest SM
-// (64^3 26 us, 96^3 51, 128^3 113, 256^3 703), two launches of the one-step
-// kernel 2 (2 us + cells / 29 per ns) (64^3 21 us, 96^3 66, 128^3 141, 256^3
-// 1053).  So small lattices, whose tiles leave SMs idle or spend most
-// iterations filling the pipeline, and shapes that fit the tiles badly keep one step per
-// launch; the line lies near 80^3.
+// Measured: two steps in one launch take 1.5 us and 1.65 us per iteration of
+// the busiest SM (96^3 41 us, 128^3 103, 256^3 676), in two launches of the
+// one-step kernel cells / 31 per ns each (96^3 59 us, 128^3 134, 256^3 1034;
+// below 80^3 less, the lattice then stays in L2: 80^3 28 us against 35). So
+// small lattices, whose tiles leave SMs idle or spend most iterations filling
+// the pipeline, and shapes that fit the tiles badly keep one step per launch;
+// the line lies near 85^3.
 bool worth_alone(const Geom& g, int sms)
 {
     if (!eligible(g)) return false;
     const double pair = kLaunchUs + kIterationUs * (double)iterations(g, plan_for(g, sms), sms);
-    const double singles = 2.0 * (kLaunchUs / 2 + (double)g.plane * kCellUs);
+    const double singles = 2.0 * (double)g.plane * kCellUs;
     return pair < 0.97 * singles;
 }
 

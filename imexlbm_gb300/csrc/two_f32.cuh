@@ -10,7 +10,7 @@
 // pair of cells and step) and the latency of a plane's phases.
 //
 // Order.  Iteration i of a tile:
-//   loaders (2 warps)  bring the 27 pulled sources of middle plane i + 2
+//   loaders (3 warps)  bring the 27 pulled sources of middle plane i + 2
 //                      (x = x0 - 1 + i + 2) into one of two stages;
 //   A (7 warps)        collide middle plane i (the tile and one cell around
 //                      it) from its stage: the first step, stored - as the
@@ -28,8 +28,8 @@
 //
 // Tile.  32 z cells x 10 rows of destinations at most: 34 x 12 middle cells,
 // 1.275 times the work of the first step.  12 working warps put 3 on each of the SM's four
-// schedulers; 12 rows (8 + 6 warps, 4 on two of the schedulers) measured 774
-// us, 13 rows with the ex = -1, 0, +1 ring one plane deeper each (no barrier
+// schedulers; 2 loader warps measured 703 us, 4 691; 12 rows (8 + 6 warps, 4 on two
+// of the schedulers) 774, 13 rows with the ex = -1, 0, +1 ring one plane deeper each (no barrier
 // 1) and a single stage 835.  Half the time of the first versions was the
 // loads: 34-float rows through L1 (ld or 4-byte cp.async) have too little of
 // L1 left beside 220 KB of shared memory (1290 us), 16-byte cp.async writes
@@ -57,7 +57,7 @@
 namespace imex {
 namespace two {
 
-constexpr int kThreadsA = 224, kThreadsB = 160, kThreadsL = 64;
+constexpr int kThreadsA = 224, kThreadsB = 160, kThreadsL = 96;
 constexpr int kThreads = kThreadsA + kThreadsB + kThreadsL;
 constexpr int kTileZ = 32;                   // staged values of a row, destination columns at most
 constexpr int kTileY = 10;                   // destination rows of a tile at most
@@ -65,7 +65,7 @@ constexpr int kRows = kTileY + 2;            // middle rows
 constexpr int kMid = kRows * (kTileZ + 2);   // middle cells of a plane
 constexpr int kStage = kRows * (kTileZ + 8);  // staged values of a direction: rows, then 2 x 4 side values a row
 constexpr int kRing = 9 * (1 + 2 + 3);       // ring arrays of kMid values
-constexpr int kSide = 7;                     // side pieces of a loader thread
+constexpr int kSide = 5;                     // side pieces of a loader thread
 constexpr int kLoadWarps = kThreadsL / 32;
 static_assert(kMid / 2 <= kThreadsA && kTileY * kTileZ / 2 <= kThreadsB, "one pair of cells per thread");
 static_assert(36 * kRows <= kSide * kThreadsL, "side pieces");
@@ -346,7 +346,7 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
             float* const d = dst + (size_t)(b.x0 + i - 3) * sheet + to;
 #pragma unroll
             for (int a = 0; a < kQ; ++a)
-                *reinterpret_cast<float2*>(d + (size_t)a * plane) = make_float2(S::store(h[a].x, a), S::store(h[a].y, a));
+                __stcs(reinterpret_cast<float2*>(d + (size_t)a * plane), make_float2(S::store(h[a].x, a), S::store(h[a].y, a)));
         }
         bar_sync<0, kThreadsA + kThreadsB>();
         s2 ^= 1;

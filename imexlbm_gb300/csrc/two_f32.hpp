@@ -43,7 +43,7 @@ Plan plan_tiles(const Geom& g, int planes);
 int item_iterations(const Geom& g, const Plan& p);
 // Microseconds: an SM's iteration, a launch, and a float32 cell's step in the
 // one-step kernels on the whole GPU (see worth_alone).
-constexpr double kIterationUs = 1.85, kLaunchUs = 4.0, kCellUs = 1.0 / 29000.0;
+constexpr double kIterationUs = 1.65, kLaunchUs = 1.5, kCellUs = 1.0 / 31000.0;
 
 cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, LatticePtr* out);
 // Two fused steps of one lattice from buffer `from` into the other one.
