@@ -36,9 +36,8 @@
 // one-CTA-per-segment form after the tick.
 //
 // Launch shapes (cell kernel: threads per CTA, cells per thread, CTAs per
-// SM; row kernel: stages, stage size, CTAs per SM) are chosen by an
-// autotuner that times each candidate on the batch itself; timing writes
-// only the members' spare buffers, so it changes no state.
+// SM; row kernel: stages, stage size, CTAs per SM) follow from the members
+// by rule (pick_pairs, pick_rows) unless they are pinned.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -332,8 +331,7 @@ constexpr int kPairGroup = 8;  // items per entry of the member lookup table
 // part along x (two_f32.cuh).  The item's member is found from group[item /
 // kPairGroup] by stepping forward.  24 float32 lattices of edges 32 to 128,
 // initialised, stepped 96 times and read back: 46.3 -> 37.7 ms against the
-// one-CTA-per-segment kernel (itself at the copy bandwidth); no shapes to
-// tune on the way: the first batch of a program takes 38.5 ms instead of 111.
+// one-CTA-per-segment kernel (itself at the copy bandwidth).
 __global__ void __launch_bounds__(two::kThreads, 1)
     k_batch_pairs(const PairHeader* __restrict__ hdr, const PairEntry* __restrict__ tab, const two::Maps* __restrict__ maps,
                   const int* __restrict__ group, int s, CollideF32 base, WaitCtl wc)
@@ -642,7 +640,7 @@ void pick_pairs(imex_batch* b)
         cand.push_back(m);
         singles += one;
     }
-    double best = 0.97 * (singles + two::kLaunchUs);
+    double best = 0.97 * (singles + two::kLaunchUs);  // a launch either way
     int best_planes = 0;
     for (int planes : {16, 24, 32, 48, 64, 96, 128, 192, 256}) {
         double all = 0;
@@ -888,80 +886,31 @@ int release_members(imex_batch* b)
     return IMEX_OK;
 }
 
-// Row-kernel shapes (stages, KiB per direction, CTAs per SM); those whose
-// CTAs do not fit an SM's shared memory with the batch's table are skipped.
-std::vector<RowShape> row_candidates()
+// The row kernel's shape for the members that step once per launch, from the
+// cells whose rows it can take.  Float16-deviation members only: what is left
+// of float32 here is too little for the two-step kernel, and the segment
+// kernel serves it as well.  Measured, GLUPS of the segment kernel, of two 2 KB
+// stages with two CTAs per SM and of two 4 KB stages with one (the other
+// shapes that fit were slower on every batch): one 32^3 6.7 / 5.1 / 5.1, 4 of
+// them 18.4 / 16.1 / 20.4, 16 33.6 / 36.9 / 31.5, 64 38.6 / 43.3 / 35.9; one 64^3 27.6 / 27.7 / 29.2, 16 42.0
+// / 50.1 / 48.3; 6 of 96^3 42.8 / 49.1 / 50.6; one 128^3 40.9 / 46.7 / 47.6, four 43.8 / 55.3 / 56.4;
+// 256^3 44.9 / 57.7 / 59.9; but 8 of 80^3 41.9 / 47.3 / 42.5.  So: the segment kernel
+// below 0.3 M cells; 4 KB where members of 96-wide rows and wider hold 5 M; else
+// 2 KB.  (Timing every shape on the batch itself chose the same and took most of a batch's
+// first call, and of a server's every time its load doubled.)
+RowShape pick_rows(const imex_batch* b)
 {
-    const int shapes[][3] = {{2, 2, 2}, {2, 1, 2}, {3, 1, 2}, {2, 2, 1}, {3, 2, 1}, {2, 4, 1}};
-    std::vector<RowShape> out;
-    for (const auto& x : shapes) {
-        RowShape r;
-        r.stages = x[0];
-        r.dir_kb = x[1];
-        r.ctas_per_sm = x[2];
-        out.push_back(r);
+    unsigned long long cells = 0, wide = 0;
+    for (size_t m = 0; m < b->members.size(); ++m) {
+        const imex_lattice* h = b->members[m];
+        if (!single(b, m) || h->precision != IMEX_F16DEV || !rows_per_item(h, RowShape{2, 4, 1, 0})) continue;
+        cells += h->ncells;
+        if (h->g.nz >= 96) wide += h->ncells;
     }
-    return out;
-}
-
-// Milliseconds per step of shapes (sh, rs) on the current members: step 0
-// of a one-step tick reads buf[cur] and writes the other buffer, leaving
-// every member's state as it was.
-int time_step(imex_batch* b, const BatchShape& sh, const RowShape& rs, float* ms)
-{
-    std::vector<int> one(b->members.size(), 1);
-    int rc = upload_table(b, one, rs, sh);
-    if (rc) return rc;
-    cudaEvent_t e0, e1;
-    B_CUDA(b, cudaEventCreate(&e0), "cudaEventCreate");
-    B_CUDA(b, cudaEventCreate(&e1), "cudaEventCreate");
-    cudaError_t e = launch_step(b, sh, rs, 0);  // warm-up
-    if (e == cudaSuccess) e = cudaEventRecord(e0, b->stream);
-    for (int r = 0; r < 3 && e == cudaSuccess; ++r) e = launch_step(b, sh, rs, 0);
-    if (e == cudaSuccess) e = cudaEventRecord(e1, b->stream);
-    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-    float t = 0.f;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    if (e != cudaSuccess) return bcuda(b, e, "batch autotune");
-    b->launches += 4 * ((b->n_cell > 0) + (b->n_row > 0));
-    *ms = t / 3;
-    return IMEX_OK;
-}
-
-// Pick the launch shapes.  The cell kernel's is one CTA per segment: its
-// other shapes (k_batch: pinned by imex_batch_set_launch) were slower on every
-// batch timed, float32 28-30 against 30-32 GLUPS, and timing 18 of them was most of a
-// batch's first call.  The row kernel's shapes are timed, with and without
-// the float32 members, against the row kernel off, the members it leaves in
-// the cell kernel.  Shapes pinned by imex_batch_set_launch /
-// imex_batch_set_row_launch are kept.  Each timing is one warm-up and three
-// steps of the members that step once per launch.
-int tune_batch(imex_batch* b)
-{
-    if (!b->shape.threads) b->shape = BatchShape{kUnitThreads, 0, 0};
-    if (b->rshape.stages) return IMEX_OK;
-    const RowShape off{-1, 0, 0, 1};
-    float best = 0.f;
-    int rc = time_step(b, b->shape, off, &best);
-    if (rc) return rc;
-    RowShape best_rs = off;
-    for (RowShape rs : row_candidates()) {
-        if (!rows_fit(rs, b->capacity)) continue;
-        for (int f32 = 1; f32 >= 0; --f32) {
-            rs.f32 = f32;
-            float ms = 0.f;
-            rc = time_step(b, b->shape, rs, &ms);
-            if (rc) return rc;
-            if (b->n_row > 0 && ms < best) {
-                best = ms;
-                best_rs = rs;
-            }
-        }
-    }
-    b->rshape = best_rs;
-    return IMEX_OK;
+    if (cells < 300000) return RowShape{-1, 0, 0, 1};
+    const RowShape large{2, 4, 1, 0}, small{2, 2, 2, 0};
+    if (wide >= 5000000 && rows_fit(large, b->capacity)) return large;
+    return rows_fit(small, b->capacity) ? small : RowShape{-1, 0, 0, 1};
 }
 
 // Capture K steps (s = 0..K-1) of the current shapes into a graph.
@@ -1145,12 +1094,8 @@ int imex_batch_step(imex_batch* b, int nsteps)
     int rc = join_members(b);
     if (rc) return rc;
     pick_pairs(b);
-    bool singles = false;  // members that step once per launch
-    for (size_t m = 0; m < b->members.size(); ++m) singles = singles || single(b, m);
-    if (singles && (!b->shape.threads || !b->rshape.stages)) {
-        rc = tune_batch(b);
-        if (rc) return rc;
-    }
+    if (!b->cells_pinned) b->shape = BatchShape{kUnitThreads, 0, 0};
+    if (!b->rows_pinned) b->rshape = pick_rows(b);
     std::vector<int> tick(b->members.size());
     for (;;) {
         int64_t most = 0;
@@ -1239,7 +1184,7 @@ int imex_batch_set_row_launch(imex_batch* b, int stages, int dir_kb, int ctas_pe
 {
     if (!b) return set_thread_error(IMEX_ERR_ARG, "imex_batch_set_row_launch: null batch");
     b->rows_pinned = stages != 0;
-    if (stages == 0 || stages == -1) {  // 0: autotune, -1: row kernel off
+    if (stages == 0 || stages == -1) {  // 0: by rule, -1: row kernel off
         b->rshape = RowShape{stages, 0, 0, 1};
         return IMEX_OK;
     }

@@ -265,7 +265,7 @@ class Batch:
 
     def set_row_launch(self, stages: int, dir_kb: int = 2, ctas_per_sm: int = 1, float32_members: bool = True) -> None:
         """Row-staged kernel shape (stages, KiB per direction in a stage,
-        CTAs per SM, float32 members in it); stages 0 autotunes, -1 turns
+        CTAs per SM, float32 members in it); stages 0 goes by the members, -1 turns
         the row kernel off."""
         self._check(self._L.imex_batch_set_row_launch(self._b, int(stages), int(dir_kb), int(ctas_per_sm),
                                                       int(bool(float32_members))))

@@ -323,9 +323,9 @@ int imex_batch_remove(imex_batch *b, imex_lattice *h);
 int imex_batch_size(const imex_batch *b);
 
 /* Advance every member nsteps reference steps (Collision then Streaming,
- * as imex_step), or up to its limit.  The first call times the launch
- * shapes (threads per CTA, cells per thread, CTAs per SM) on the batch
- * itself, without changing any member's state, and keeps the fastest. */
+ * as imex_step), or up to its limit.  Which kernel a member runs in and
+ * the launch shapes follow from the members' formats and sizes by rule,
+ * unless they are pinned (below). */
 int imex_batch_step(imex_batch *b, int nsteps);
 int imex_batch_synchronize(imex_batch *b);
 
@@ -335,7 +335,7 @@ int imex_batch_synchronize(imex_batch *b);
  * cells_per_thread 0 with threads 128 - one CTA per 256-cell segment of
  * every member, the one-lattice kernel's grid over the whole batch (its
  * CUDA graph is captured again when the members' segment count changes).
- * threads = 0 retunes. */
+ * threads = 0 leaves it to the rule again. */
 int imex_batch_set_launch(imex_batch *b, int threads, int cells_per_thread, int ctas_per_sm);
 int imex_batch_get_launch(imex_batch *b, int out[3]);
 
@@ -344,11 +344,12 @@ int imex_batch_get_launch(imex_batch *b, int out[3]);
  * dir_kb KiB: ring depth `stages`, `dir_kb` KiB per direction in a stage
  * (1, 2 or 4; a member's work item is the largest block of y-rows that
  * fits), resident CTAs per SM, and whether float32 members join it
- * (float32_members != 0) or stay in the cell kernel.  stages 0 autotunes
- * (default); -1 turns the row kernel off, so every member runs in the cell
- * kernel.  imex_batch_get_row_launch gives {stages, dir_kb, ctas_per_sm,
- * float32_members} (stages -1 when the tuner found the cell kernel
- * faster). */
+ * (float32_members != 0) or stay in the cell kernel.  stages 0 leaves
+ * it to the rule (default); -1 turns the row kernel off, so every member runs in the cell
+ * kernel.  With either shape pinned no member steps twice per launch.
+ * imex_batch_get_row_launch gives {stages, dir_kb, ctas_per_sm,
+ * float32_members} (stages -1 when the rule keeps every member in the cell
+ * kernel). */
 int imex_batch_set_row_launch(imex_batch *b, int stages, int dir_kb, int ctas_per_sm, int float32_members);
 int imex_batch_get_row_launch(imex_batch *b, int out[4]);
 
