@@ -8,12 +8,12 @@
 //   imex_checkpoint_save  the handle's raw device state to a file, and
 //   imex_checkpoint_load  back (no reference counterpart)
 //
-// One kernel serves the min/max and the Tecplot file: per cell it forms p = sum f / 3 and
-// u = sum f e (the ComputeMacroscopic moments, src/lbm.cpp:218-236, pulled
-// through a pending streaming), reduces their minima and maxima, and - for
-// the file - writes the four fields transposed to the file's x-fastest
-// (Fortran) order through a shared-memory tile, so both the reads along z
-// and the writes along x are coalesced.  The file is then streamed to disk
+// The min/max alone is minmax.cuh's.  For the Tecplot file one kernel forms,
+// per cell, p = sum f / 3 and u = sum f e (the ComputeMacroscopic moments,
+// src/lbm.cpp:218-236, pulled through a pending streaming), reduces their
+// minima and maxima, and writes the four fields transposed to the file's
+// x-fastest (Fortran) order through a shared-memory tile, so both the reads
+// along z and the writes along x are coalesced.  The file is then streamed to disk
 // in chunks through two pinned host buffers, copy of one chunk overlapping
 // the write of the other.
 #include <cfloat>
@@ -27,6 +27,7 @@
 #include "kernels_common.cuh"
 #include "lattice_internal.hpp"
 #include "lowp_math.cuh"
+#include "minmax.cuh"
 
 namespace imex {
 namespace {
@@ -68,7 +69,7 @@ inline double order_unkey(unsigned long long k)
 
 // One (32 z) x (32 x) tile of one y row per block.  mm[0..3] = max of u, v,
 // w, p and mm[4..7] = their min, as order keys; NaN values are skipped, as
-// the reference's `if (u > umx)` comparisons skip them.  out (optional) =
+// the reference's `if (u > umx)` comparisons skip them.  out =
 // u, v, w, p blocks of ncells doubles each, index x + nx (y + ny z).
 template <int P, bool PULL>
 __global__ void __launch_bounds__(kFieldThreads) k_fields(const typename Src<P>::T* __restrict__ src, Geom g,
@@ -103,15 +104,13 @@ __global__ void __launch_bounds__(kFieldThreads) k_fields(const typename Src<P>:
             if (val[c] < mn[c]) mn[c] = val[c];
         }
     }
-    if (out) {
-        __syncthreads();
-        for (int r = warp; r < kTile; r += kFieldThreads / 32) {
-            const int k = k0 + r, i = i0 + lane;
-            if (k >= g.nz || i >= g.nx) continue;
-            const size_t o = ((size_t)k * g.ny + j) * g.nx + i;
+    __syncthreads();
+    for (int r = warp; r < kTile; r += kFieldThreads / 32) {
+        const int k = k0 + r, i = i0 + lane;
+        if (k >= g.nz || i >= g.nx) continue;
+        const size_t o = ((size_t)k * g.ny + j) * g.nx + i;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) out[c * g.plane + o] = tile[c][lane][r];
-        }
+        for (int c = 0; c < 4; ++c) out[c * g.plane + o] = tile[c][lane][r];
     }
     // warp, then block, then one atomic per value and block
     __shared__ double red[kFieldThreads / 32][8];
@@ -183,7 +182,7 @@ int ready(imex_lattice* h, const char* what)
     return IMEX_OK;
 }
 
-// Run the field kernel; minmax[8] on return, the fields (if out) queued.
+// Run the field kernel; minmax[8] on return, the fields queued.
 int run_fields(imex_lattice* h, double* out, unsigned long long* d_mm, double minmax[8], const char* what)
 {
     unsigned long long keys[8];
@@ -350,6 +349,9 @@ struct CkptHeader {
 constexpr char kCkptMagic[8] = {'I', 'M', 'E', 'X', 'C', 'K', 'P', 'T'};
 
 }  // namespace
+
+size_t minmax_scratch_bytes(const Geom& g) { return mm::scratch_bytes(g); }
+
 }  // namespace imex
 
 using namespace imex;
@@ -361,12 +363,22 @@ int imex_minmax_uvwp(imex_lattice* h, double out[8])
     int rc = ready(h, "imex_minmax_uvwp");
     if (rc) return rc;
     if (!out) return fail(h, IMEX_ERR_ARG, "imex_minmax_uvwp: null output");
-    unsigned long long* d = nullptr;
-    cudaError_t e = cudaMallocAsync(&d, 8 * sizeof(unsigned long long), h->stream);
+    cudaError_t e;
+    {
+        PhaseScope timed(h->prof, IMEX_PHASE_MACRO, h->stream);
+        e = mm::launch(h->precision, h->tag == kPendingStream, h->buf[h->cur], h->g, h->d_partial, h->stream);
+    }
+    mm::Result r;
+    if (e == cudaSuccess) h->launches += 2;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&r, h->d_partial, sizeof r, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "imex_minmax_uvwp");
-    rc = run_fields(h, nullptr, d, out, "imex_minmax_uvwp");
-    cudaFreeAsync(d, h->stream);
-    return rc;
+    for (int c = 0; c < 4; ++c) {  // p, u, v, w to u, v, w, p; 0: no value compared
+        const int to = c == 0 ? 3 : c - 1;
+        out[to] = r.picked[c] ? order_unkey(r.picked[c]) : -DBL_MAX;
+        out[4 + to] = r.picked[4 + c] ? order_unkey(~r.picked[4 + c]) : DBL_MAX;
+    }
+    return IMEX_OK;
 }
 
 int imex_write_tecplot(imex_lattice* h, const char* path, int n)

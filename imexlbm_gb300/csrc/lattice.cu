@@ -506,7 +506,9 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     // scratch: conserved partials (the native engine's: 5 doubles per
     // 128-cell row segment), 5 reduced values, fallback counter, error flag,
     // fixed-point run flag, the conserved kernel's ticket
-    const size_t parts = std::max(conserved_partials(h->g) * 5 * sizeof(double), conserved_scratch_bytes(h->g));
+    // (the min/max report's chunks lie in the partials' place)
+    const size_t parts = std::max({conserved_partials(h->g) * 5 * sizeof(double), conserved_scratch_bytes(h->g),
+                                   minmax_scratch_bytes(h->g)});
     const size_t scratch = parts + 5 * sizeof(double) + 4 * sizeof(unsigned long long);
     const size_t need = 2 * arr + scratch;
     // Device memory comes from the device's stream-ordered pool: creating

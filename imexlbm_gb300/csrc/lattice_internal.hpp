@@ -74,5 +74,6 @@ namespace imex {
 // Both defined in lattice.cu.
 int lattice_fail(imex_lattice* h, int code, const std::string& msg);
 size_t lattice_elem_size(int precision);
+size_t minmax_scratch_bytes(const Geom& g);  // fields.cu
 
 }  // namespace imex

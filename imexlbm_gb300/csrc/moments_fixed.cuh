@@ -113,6 +113,7 @@ __device__ __forceinline__ bool moments(const typename Elem<P>::T* __restrict__ 
             uint64_t w = 0;
 #pragma unroll
             for (int a = 0; a < kQ; ++a) w += lowp::weight_fixed(a);
+            ok = ok && S < (int64_t)3 << 61;  // the weights' 2^61 more stays below 2^63
             S += (int64_t)w;
         }
         c.M[0] = S;
