@@ -784,7 +784,9 @@ int imex_step(imex_lattice* h, int nsteps)
             return step_fixed_run(h, nsteps);
         }
     }
-    if (use_pairs(h) && nsteps >= 3) {
+    // (a captured run keeps one step per launch: replayed, it must end in the
+    // buffer it began in whenever its number of steps is even)
+    if (use_pairs(h) && nsteps >= 3 && !capturing(h)) {
         if (h->tag != kPendingStream) {
             rc = step_each(h, 1);
             if (rc) return rc;

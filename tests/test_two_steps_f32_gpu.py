@@ -83,3 +83,28 @@ def test_starved_plane_is_reported_and_the_handle_recovers(imex):
         lat.initialize_phase(0.3, 1.1, 2.0)
         lat.step(9)
         assert np.array_equal(lat.get_f(), want)
+
+
+@pytest.mark.parametrize("steps", [4, 6])
+def test_captured_run_replays(imex, steps):
+    """A graph of an even number of steps, replayed, goes on from its own result."""
+    torch = pytest.importorskip("torch")
+    shape = (96, 96, 96)
+    outs = []
+    for captured in (False, True):
+        with imex.LBM(*shape, 0.003, 1.0, 0.06, precision=imex.IMEX_F32) as lat:
+            lat.initialize_phase(0.3, 1.1, 2.0)
+            lat.step(1)
+            if captured:
+                stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+                lat.set_stream(stream.cuda_stream)
+                with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+                    lat.step(steps)
+                graph.replay()
+                graph.replay()
+                torch.cuda.synchronize()
+            else:
+                lat.step(2 * steps)
+            outs.append(lat.get_f())
+            lat.set_stream(None)
+    assert np.array_equal(*outs)
