@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(two::kThreads, 1)
     const int cur = e.cur ^ ((s >> 1) & 1);
     CollideF32 cp = base;
     cp.eps = e.eps;
-    two::run_box<true>(&maps[2 * m + cur], e.buf[cur], e.buf[cur ^ 1], e.nx, e.ny, e.nz, e.plane,
+    two::run_box<true, false>(&maps[2 * m + cur], e.buf[cur], e.buf[cur ^ 1], e.nx, e.ny, e.nz, e.plane,
                        two::box_of(e.plan, e.nx, e.ny, e.nz, (int)(item - e.begin)), cp, smem, wc);
 }
 

@@ -129,17 +129,19 @@ struct PullIndex {
 // sum of a part for each of ex, ey and ez ([e + 1]).
 struct FlatPull {
     unsigned x[3], y[3], z[3];
-    __device__ __forceinline__ FlatPull(int nx, int ny, int nz, unsigned cell)
+    __device__ __forceinline__ FlatPull(int nx, int ny, int nz, unsigned cell) : FlatPull(nx, ny, nz, cell, nz) {}
+    // rows `pitch` values apart
+    __device__ __forceinline__ FlatPull(int nx, int ny, int nz, unsigned cell, int pitch)
     {
         const unsigned row = cell / (unsigned)nz, k = cell - row * (unsigned)nz;
         const unsigned i = row / (unsigned)ny, j = row - i * (unsigned)ny;
-        const unsigned sheet = (unsigned)ny * (unsigned)nz;
+        const unsigned sheet = (unsigned)ny * (unsigned)pitch;
         x[0] = (i == (unsigned)nx - 1 ? 0 : i + 1) * sheet;
         x[1] = i * sheet;
         x[2] = (i == 0 ? (unsigned)nx - 1 : i - 1) * sheet;
-        y[0] = (j == (unsigned)ny - 1 ? 0 : j + 1) * (unsigned)nz;
-        y[1] = j * (unsigned)nz;
-        y[2] = (j == 0 ? (unsigned)ny - 1 : j - 1) * (unsigned)nz;
+        y[0] = (j == (unsigned)ny - 1 ? 0 : j + 1) * (unsigned)pitch;
+        y[1] = j * (unsigned)pitch;
+        y[2] = (j == 0 ? (unsigned)ny - 1 : j - 1) * (unsigned)pitch;
         z[0] = k == (unsigned)nz - 1 ? 0 : k + 1;
         z[1] = k;
         z[2] = k == 0 ? (unsigned)nz - 1 : k - 1;

@@ -502,7 +502,12 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     cudaError_t e = cudaGetDevice(&h->device);
     if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaGetDevice"));
 
-    const size_t arr = (size_t)kQ * h->ncells * elem_size(precision);
+    size_t arr = (size_t)kQ * h->ncells * elem_size(precision);
+    // float32 rows that are no multiple of 4 values: room for the layout of two
+    // steps per launch, where there is any and the lattice is worth it
+    const size_t plain = arr;
+    if (precision == IMEX_F32 && two::padded_eligible(h->g) && two::worth_alone(h->g, current_sm_count()))
+        arr = kQ * two::padded_plane(h->g) * sizeof(float);
     // scratch: conserved partials (the native engine's: 5 doubles per
     // 128-cell row segment), 5 reduced values, fallback counter, error flag,
     // fixed-point run flag, the conserved kernel's ticket
@@ -510,7 +515,7 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     const size_t parts = std::max({conserved_partials(h->g) * 5 * sizeof(double), conserved_scratch_bytes(h->g),
                                    minmax_scratch_bytes(h->g)});
     const size_t scratch = parts + 5 * sizeof(double) + 4 * sizeof(unsigned long long);
-    const size_t need = 2 * arr + scratch;
+    size_t need = 2 * arr + scratch;
     // Device memory comes from the device's stream-ordered pool: creating
     // and destroying lattices (a server does it per request) then neither
     // synchronises the device nor returns memory to the driver.  Memory the
@@ -524,6 +529,10 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
     cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
     const size_t avail = free_b + (reserved > used ? (size_t)(reserved - used) : 0);
+    if (need > avail && arr > plain) {
+        arr = plain;
+        need = 2 * arr + scratch;
+    }
     if (need > avail) {
         char msg[160];
         std::snprintf(msg, sizeof msg, "imex_create: needs %.3f GB of device memory, %.3f GB free", need / 1e9,
@@ -533,7 +542,20 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaStreamCreate"));
     h->stream = h->own_stream;
-    for (int b = 0; b < 2 && e == cudaSuccess; ++b) e = cudaMallocAsync(&h->buf[b], arr, h->stream);
+    h->padded_room = arr > plain;
+    auto buffers = [&](size_t bytes) {
+        for (int b = 0; b < 2 && e == cudaSuccess; ++b) e = cudaMallocAsync(&h->buf[b], bytes, h->stream);
+    };
+    buffers(arr);
+    if (e != cudaSuccess && h->padded_room) {
+        cudaGetLastError();
+        if (h->buf[0]) cudaFreeAsync(h->buf[0], h->stream);
+        h->buf[0] = h->buf[1] = nullptr;
+        h->padded_room = false;
+        need -= 2 * (arr - plain);
+        e = cudaSuccess;
+        buffers(plain);
+    }
     unsigned char* s = nullptr;
     if (e == cudaSuccess) e = cudaMallocAsync((void**)&s, scratch, h->stream);
     if (e != cudaSuccess) {
@@ -729,23 +751,33 @@ int step_fixed_run(imex_lattice* h, int n)
 bool use_pairs(imex_lattice* h)
 {
     if (h->precision != IMEX_F32 || h->shape_pinned || h->prof.enabled()) return false;
-    if (h->pairs_worth < 0) h->pairs_worth = two::worth_alone(h->g, current_sm_count());
+    if (h->pairs_worth < 0)
+        h->pairs_worth = (two::eligible(h->g) || h->padded_room) && two::worth_alone(h->g, current_sm_count());
     return h->pairs_worth != 0;
 }
 
-// n / 2 launches of two fused float32 steps each, from the steady state.
-int step_pairs(imex_lattice* h, int n)
+// Fused float32 steps, n or n - 1 of them, two per launch from the steady
+// state; rows that are no multiple of 4 values: a single step into the padded
+// layout first and one out of it last.  *done: the steps taken.
+int step_pairs(imex_lattice* h, int n, int* done)
 {
     if (!h->pairs)
         IMEX_CUDA(h, two::make_lattice(static_cast<float*>(h->buf[0]), static_cast<float*>(h->buf[1]), h->g, &h->pairs),
                   "two-step kernel set-up");
-    for (int s = 0; s + 2 <= n; s += 2) {
-        IMEX_CUDA(h, two::launch(*h->pairs, h->cur, static_cast<const float*>(h->buf[h->cur]),
-                                 static_cast<float*>(h->buf[1 - h->cur]), h->g, h->cf32, h->d_err, h->stream),
-                  "step kernel launch");
+    const bool padded = h->pairs->padded;
+    *done = padded && n < 4 ? 0 : n & ~1;
+    for (int s = 0; s < *done;) {
+        const float* src = static_cast<const float*>(h->buf[h->cur]);
+        float* dst = static_cast<float*>(h->buf[1 - h->cur]);
+        const bool edge = padded && (s == 0 || s == *done - 1);
+        cudaError_t e = edge ? two::launch_edge(s > 0, src, dst, h->g, h->cf32, h->stream)
+                             : two::launch(*h->pairs, h->cur, src, dst, h->g, h->cf32, h->d_err, h->stream);
+        if (e != cudaSuccess && padded && s > 0) h->tag = kUninit;  // no plain state left
+        IMEX_CUDA(h, e, "step kernel launch");
         ++h->launches;
         h->cur = 1 - h->cur;
-        h->steps += 2;
+        h->steps += edge ? 1 : 2;
+        s += edge ? 1 : 2;
     }
     return IMEX_OK;
 }
@@ -792,9 +824,10 @@ int imex_step(imex_lattice* h, int nsteps)
             if (rc) return rc;
             --nsteps;
         }
-        rc = step_pairs(h, nsteps);
+        int done = 0;
+        rc = step_pairs(h, nsteps, &done);
         if (rc) return rc;
-        nsteps &= 1;
+        nsteps -= done;
     }
     return step_each(h, nsteps);
 }

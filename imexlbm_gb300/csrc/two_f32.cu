@@ -12,13 +12,63 @@ namespace two {
 
 namespace {
 
+template <bool kPadded>
 __global__ void __launch_bounds__(kThreads, 1)
     k_two_f32(const __grid_constant__ Maps maps, const float* __restrict__ src, float* __restrict__ dst, Geom g, Plan p,
               CollideF32 cp, WaitCtl wc)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     chain_next();
-    run_box<false>(&maps, src, dst, g.nx, g.ny, g.nz, g.plane, box_of(p, g.nx, g.ny, g.nz, blockIdx.x), cp, smem, wc);
+    run_box<false, kPadded>(&maps, src, dst, g.nx, g.ny, g.nz, kPadded ? (size_t)g.nx * g.ny * pitch_of(g.nz) : g.plane,
+                           box_of(p, g.nx, g.ny, g.nz, blockIdx.x), cp, smem, wc);
+}
+
+// One fused step between the layouts, two cells a thread (flat_lowp.cuh's
+// separate pairs: neither layout's rows are 8-byte aligned in every direction).
+constexpr int kEdgeThreads = 128;
+template <bool kOut>
+__global__ void __launch_bounds__(kEdgeThreads) k_edge_f32(const float* __restrict__ src, float* __restrict__ dst, Geom g,
+                                                           CollideF32 cp)
+{
+    using S = lowp::Storage<IMEX_F32>;
+    using A = lowp::F2;
+    chain_begin<true>();
+    const unsigned cells = (unsigned)g.plane, c0 = blockIdx.x * (2 * kEdgeThreads) + threadIdx.x;
+    if (c0 >= cells) return;
+    const bool two = c0 + kEdgeThreads < cells;
+    const unsigned c1 = two ? c0 + kEdgeThreads : c0;
+    const int pitch = pitch_of(g.nz);
+    const size_t padded = (size_t)g.nx * g.ny * pitch, from = kOut ? padded : g.plane, to = kOut ? g.plane : padded;
+    const FlatPull p0(g.nx, g.ny, g.nz, c0, kOut ? pitch : g.nz), p1(g.nx, g.ny, g.nz, c1, kOut ? pitch : g.nz);
+    float2 h[kQ];
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+        const float* p = src + (size_t)a * from;
+        h[a] = make_float2(S::dev(__ldg(p + p0.at(a)), a), S::dev(__ldg(p + p1.at(a)), a));
+    }
+    lowp::collide_dev<IMEX_F32, A>(h, cp);
+    if (kOut) {
+#pragma unroll
+        for (int a = 0; a < kQ; ++a) {
+            dst[(size_t)a * to + c0] = S::store(h[a].x, a);
+            if (two) dst[(size_t)a * to + c1] = S::store(h[a].y, a);
+        }
+        return;
+    }
+    auto put = [&](unsigned c, bool second) {
+        const unsigned row = c / (unsigned)g.nz;
+        const int z = (int)(c - row * (unsigned)g.nz);
+        const bool copy = z == 0 && (g.nz & 1);
+        float* const o = dst + (size_t)row * pitch + z;
+#pragma unroll
+        for (int a = 0; a < kQ; ++a) {
+            const float v = S::store(second ? h[a].y : h[a].x, a);
+            o[(size_t)a * to] = v;
+            if (copy) o[(size_t)a * to + g.nz] = v;
+        }
+    };
+    put(c0, false);
+    if (two) put(c1, true);
 }
 
 using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -74,12 +124,13 @@ Plan plan_for(const Geom& g, int sms)
     return best;
 }
 
-cudaError_t encode_maps(const float* buf, const Geom& g, const Plan& p, Maps* out)
+cudaError_t encode_maps(const float* buf, const Geom& g, const Plan& p, bool padded, Maps* out)
 {
     const Encode f = encode_fn();
     if (!f) return cudaErrorNotSupported;
-    const cuuint64_t dims[3] = {(cuuint64_t)g.nz, (cuuint64_t)g.ny, (cuuint64_t)kQ * g.nx};
-    const cuuint64_t strides[2] = {(cuuint64_t)g.nz * 4, (cuuint64_t)g.nz * g.ny * 4};
+    const cuuint64_t row = (cuuint64_t)(padded ? pitch_of(g.nz) : g.nz);
+    const cuuint64_t dims[3] = {row, (cuuint64_t)g.ny, (cuuint64_t)kQ * g.nx};
+    const cuuint64_t strides[2] = {row * 4, row * g.ny * 4};
     const cuuint32_t step[3] = {1, 1, 1};
     for (int q = 0; q < kMaps; ++q) {
         // fewer rows than one: never used, a valid box all the same
@@ -99,6 +150,10 @@ bool eligible(const Geom& g)
     return g.nz % 4 == 0 && g.nz >= kTileZ && g.ny >= 4 && g.nx >= 4 && g.plane < (1ull << 32) / kQ;
 }
 
+bool padded_eligible(const Geom& g)
+{
+    return g.nz % 4 != 0 && g.nz >= kTileZ && g.ny >= 4 && g.nx >= 4 && padded_plane(g) < (1ull << 32) / kQ;
+}
 
 int item_iterations(const Geom& g, const Plan& p) { return (g.nx + p.chunks - 1) / p.chunks + kExtra; }
 
@@ -115,12 +170,17 @@ Plan plan_tiles(const Geom& g, int planes)
 // below 80^3 less, the lattice then stays in L2: 80^3 28 us against 35). So
 // small lattices, whose tiles leave SMs idle or spend most iterations filling
 // the pipeline, and shapes that fit the tiles badly keep one step per launch;
-// the line lies near 85^3.
+// the line lies near 85^3.  Padded layout, single -> two steps, us a step: 255^3
+// 546 -> 357, 131 x 128 x 128 68.8 -> 63.7, 97 x 150 x 121 (four tiles for
+// three and a value) 59.1 -> 55.3, 111^3 48.5 -> 38.8, 85^3 20.3 -> 19.9 (not taken),
+// 65 x 160 x 160 54.1 -> 55.6 (not taken).
 bool worth_alone(const Geom& g, int sms)
 {
-    if (!eligible(g)) return false;
-    const double pair = kLaunchUs + kIterationUs * (double)iterations(g, plan_for(g, sms), sms);
-    const double singles = 2.0 * (double)g.plane * kCellUs;
+    if (!eligible(g) && !padded_eligible(g)) return false;
+    const bool plain = eligible(g);
+    const double pair =
+        kLaunchUs + (plain ? kIterationUs : kPaddedIterationUs) * (double)iterations(g, plan_for(g, sms), sms);
+    const double singles = 2.0 * (double)g.plane * (plain ? kCellUs : kPaddedCellUs);
     return pair < 0.97 * singles;
 }
 
@@ -129,10 +189,12 @@ cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, La
     LatticePtr l(new (std::nothrow) Lattice);
     if (!l) return cudaErrorMemoryAllocation;
     l->plan = plan_for(g, current_sm_count());
-    cudaError_t e = encode_maps(buf0, g, l->plan, &l->maps[0]);
-    if (e == cudaSuccess) e = encode_maps(buf1, g, l->plan, &l->maps[1]);
+    l->padded = !eligible(g);
+    cudaError_t e = encode_maps(buf0, g, l->plan, l->padded, &l->maps[0]);
+    if (e == cudaSuccess) e = encode_maps(buf1, g, l->plan, l->padded, &l->maps[1]);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_two_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+        e = cudaFuncSetAttribute(l->padded ? k_two_f32<true> : k_two_f32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kSmemBytes);
     if (e == cudaSuccess) *out = std::move(l);
     return e;
 }
@@ -140,8 +202,14 @@ cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, La
 cudaError_t launch(const Lattice& l, int from, const float* src, float* dst, const Geom& g, const CollideF32& cp,
                    unsigned* err, cudaStream_t s)
 {
-    return launch_chained(k_two_f32, (unsigned)l.plan.items(), kThreads, kSmemBytes, s, l.maps[from], src, dst, g, l.plan,
-                          cp, make_wait_ctl(err));
+    return launch_chained(l.padded ? k_two_f32<true> : k_two_f32<false>, (unsigned)l.plan.items(), kThreads, kSmemBytes, s,
+                          l.maps[from], src, dst, g, l.plan, cp, make_wait_ctl(err));
+}
+
+cudaError_t launch_edge(bool out, const float* src, float* dst, const Geom& g, const CollideF32& cp, cudaStream_t s)
+{
+    const unsigned grid = (unsigned)((g.plane + 2 * kEdgeThreads - 1) / (2 * kEdgeThreads));
+    return launch_chained(out ? k_edge_f32<true> : k_edge_f32<false>, grid, kEdgeThreads, 0, s, src, dst, g, cp);
 }
 
 }  // namespace two

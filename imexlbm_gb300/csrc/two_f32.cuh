@@ -43,8 +43,15 @@
 // addresses; rows that wrap in y are left out of the box (tensor maps of ty +
 // 2 down to ty - 1 rows) and copied one by one.
 //
-// Requirements (pairs_eligible): nz a multiple of 4 (16-byte pieces and tensor
-// strides), nz >= 32, ny >= 4, nx >= 4, 27 * cells below 2^32.
+// Requirements (eligible): nz a multiple of 4 (16-byte pieces and tensor
+// strides), nz >= 32, ny >= 4, nx >= 4, 27 * cells below 2^32.  Other nz >= 32:
+// the padded layout, in which rows lie a multiple of 8 values apart.  A run's
+// first and last steps are single ones there (k_edge_f32), from the plain layout
+// and back to it.  An odd row's last pair computes z = nz, which is z = 0 once
+// more, and stores it behind the row, where the next launch's boxes read it;
+// of the pieces that wrap, those off a 16-byte boundary come as two values.
+// (Copies of all the cells that wrap, stored behind both ends by B's edge
+// threads, kept every load whole and cost B up to twice its time: 255^3 459 us a step.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -67,6 +74,7 @@ constexpr int kStage = kRows * (kTileZ + 8);  // staged values of a direction: r
 constexpr int kRing = 9 * (1 + 2 + 3);       // ring arrays of kMid values
 constexpr int kSide = 5;                     // side pieces of a loader thread
 constexpr int kLoadWarps = kThreadsL / 32;
+constexpr unsigned kTwoValues = 1u << 29;    // mark of a side piece of two values
 static_assert(kMid / 2 <= kThreadsA && kTileY * kTileZ / 2 <= kThreadsB, "one pair of cells per thread");
 static_assert(36 * kRows <= kSide * kThreadsL, "side pieces");
 static_assert(kStage * 4 % 128 == 0 && kMid % 2 == 0, "128-byte aligned boxes, 8-byte pairs");
@@ -93,7 +101,7 @@ __device__ __forceinline__ Box box_of(const Plan& p, int nx, int ny, int nz, int
     b.y0 = (int)((long long)iy * ny / p.nty);
     b.rows = (int)((long long)(iy + 1) * ny / p.nty) - b.y0;
     b.z0 = iz * p.tz;
-    b.cols = (iz + 1 == p.ntz ? nz : b.z0 + p.tz) - b.z0;
+    b.cols = ((iz + 1 == p.ntz ? nz : b.z0 + p.tz) - b.z0 + 1) & ~1;  // odd: the last one is z = 0 once more
     b.box_rows = p.ty + 2;
     return b;
 }
@@ -141,6 +149,10 @@ __device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int 
         "l"(map), "r"(z), "r"(y), "r"(x), "r"(bulk::smem_u32(mbar))
         : "memory");
 }
+__device__ __forceinline__ void cp4(void* dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(bulk::smem_u32(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp16(void* dst, const void* src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(bulk::smem_u32(dst)), "l"(src) : "memory");
@@ -153,8 +165,9 @@ __device__ __forceinline__ void cp16(void* dst, const void* src)
 // bringing planes, and the CTA runs to its end on what the stages hold (its
 // results are reported invalid).  The set-up before the roles' loops touches
 // no lattice, so each role waits for the kernels before (chain_wait) only then;
-// the caller has let the next kernel in.
-template <bool kMapsInMemory>
+// the caller has let the next kernel in.  kPadded: both buffers in the
+// padded layout (two_f32.hpp), `plane` the values of a direction there.
+template <bool kMapsInMemory, bool kPadded>
 __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const float* __restrict__ src,
                                         float* __restrict__ dst, int nx, int ny, int nz, size_t plane, const Box& b,
                                         const CollideF32& cp, unsigned char* smem, const WaitCtl& wc)
@@ -169,7 +182,8 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
     const int half = b.cols >> 1;                 // destination pairs of a row
     const int W = b.cols + 2, R = b.rows + 2;     // middle cells of a row, middle rows
     const int side0 = b.box_rows * kTileZ;        // a direction's side pieces follow its rows
-    const unsigned sheet = (unsigned)ny * (unsigned)nz;
+    const int pitch = kPadded ? pitch_of(nz) : nz;
+    const unsigned sheet = (unsigned)ny * (unsigned)pitch;
     const int last = b.planes + 2;                // middle planes
     if (threadIdx.x == 0) {
         for (int q = 0; q < 2; ++q) {
@@ -194,7 +208,7 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
         const CUtensorMap* const map = &maps->m[b.box_rows - rows];
         if constexpr (kMapsInMemory)  // written through the generic proxy (an upload before the launch)
             asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
-        const uint32_t row_bytes = (uint32_t)b.cols * 4u;
+        const uint32_t row_bytes = (((uint32_t)b.cols + 3u) & ~3u) * 4u;
         const uint32_t my_bytes = (uint32_t)rows * (kTileZ * 4u) + (uint32_t)(top + bot) * row_bytes;
         unsigned from[kSide], at[kSide];
 #pragma unroll
@@ -207,8 +221,14 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
             const int k = p / R, r = p - k * R, right = k >= 18, kk = k - 18 * right, c9 = kk >> 1;
             const int a = dir_of(c9 / 3 - 1, c9 % 3 - 1, (kk & 1) ? (right ? -1 : 1) : 0);
             const int y = b.y0 - 1 + r - ex_rt(a, 1), z = right ? b.z0 + b.cols : b.z0 - 4;
-            from[q] = (unsigned)(a * plane) + (unsigned)wrap(y, ny) * (unsigned)nz + (unsigned)wrap(z, nz);
+            from[q] = (unsigned)(a * plane) + (unsigned)wrap(y, ny) * (unsigned)pitch + (unsigned)wrap(z, nz);
             at[q] = (unsigned)(a * kStage + side0 + r * 8 + 4 * right) | ((unsigned)(ex_rt(a, 0) + 1) << 30);
+            // a piece that wraps off its 16-byte boundary: only the two values used
+            // of it, z = nz - 2 and nz - 1 on the left, 1 and 2 on the right of an odd row
+            if (kPadded && (z < 0 || z > nz)) {
+                at[q] = (at[q] + (right ? 0 : 2)) | kTwoValues;
+                from[q] += right ? 0 : 2;
+            }
         }
         auto bring = [&](int i) {  // middle plane i into stage i & 1
             const int x = wrap(b.x0 - 1 + i, nx);
@@ -225,9 +245,9 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
                     if (top + bot) {
                         const float* p = src + ((size_t)dir * plane + (size_t)xd * sheet + b.z0);
                         for (int r = 0; r < top; ++r)
-                            bulk::copy_g2s(to + r * kTileZ, p + (size_t)(ylo + r + ny) * nz, row_bytes, mb);
+                            bulk::copy_g2s(to + r * kTileZ, p + (size_t)(ylo + r + ny) * pitch, row_bytes, mb);
                         for (int r = R - bot; r < R; ++r)
-                            bulk::copy_g2s(to + r * kTileZ, p + (size_t)(ylo + r - ny) * nz, row_bytes, mb);
+                            bulk::copy_g2s(to + r * kTileZ, p + (size_t)(ylo + r - ny) * pitch, row_bytes, mb);
                     }
                 }
             }
@@ -236,8 +256,14 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
             for (int q = 0; q < kSide; ++q)
                 if (at[q] != 0xffffffffu) {
                     const unsigned e = at[q] >> 30;
-                    cp16(stage + (at[q] & 0x3fffffffu),
-                         src + ((size_t)from[q] + (size_t)(e == 0 ? xs[0] : e == 1 ? xs[1] : xs[2]) * sheet));
+                    float* const t = stage + (at[q] & (kTwoValues - 1));
+                    const float* const f = src + ((size_t)from[q] + (size_t)(e == 0 ? xs[0] : e == 1 ? xs[1] : xs[2]) * sheet);
+                    if (kPadded && (at[q] & kTwoValues)) {
+                        cp4(t, f);
+                        cp4(t + 1, f + 1);
+                    } else {
+                        cp16(t, f);
+                    }
                 }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bulk::smem_u32(mb)) : "memory");
         };
@@ -321,7 +347,7 @@ __device__ __forceinline__ void run_box(const Maps* __restrict__ maps, const flo
     {
         const int m = on ? tid : 0, r = m / half, q = m - r * half;
         pos = (r + 1) * W + 2 * q;
-        to = (unsigned)(b.y0 + r) * (unsigned)nz + (unsigned)(b.z0 + 2 * q);
+        to = (unsigned)(b.y0 + r) * (unsigned)pitch + (unsigned)(b.z0 + 2 * q);
     }
     chain_wait();
     int s2 = 0, s3 = 0;  // slots of middle planes i - 2 (ex = 0) and i - 3 (ex = +1): those plane i is about to take

@@ -25,17 +25,29 @@ struct Plan {
     int items() const { return nty * ntz * chunks; }
 };
 
+// The padded layout of a lattice whose rows are no multiple of 4 values: within
+// a direction, row (x, y) begins at (x ny + y) pitch_of(nz) values, on a 32-byte
+// sector; where nz is odd a copy of z = 0 follows z = nz - 1, which completes
+// the row's last pair of cells.
+__host__ __device__ constexpr int pitch_of(int nz) { return (nz + 8) / 8 * 8; }
+
 // What a lattice handle keeps: its tiles, cut for the lattice alone, and the
 // maps of its two buffers (the same whatever the cut along x).
 struct Lattice {
     Plan plan;
+    bool padded;
     Maps maps[2];
 };
 using LatticePtr = std::unique_ptr<Lattice>;
 
-// Whether a float32 lattice can take two steps per launch at all.
+// Whether a float32 lattice can take two steps per launch as it lies in
+// memory, or else in the padded layout.
 bool eligible(const Geom& g);
-// Whether two steps per launch beat two launches for one such lattice alone.
+bool padded_eligible(const Geom& g);
+// Values of a direction in the padded layout.
+inline size_t padded_plane(const Geom& g) { return (size_t)g.nx * g.ny * pitch_of(g.nz); }
+// Whether two steps per launch beat two launches for one lattice alone, as it
+// lies or in the padded layout.
 bool worth_alone(const Geom& g, int sms);
 // An eligible lattice's tiles, cut along x into parts of about `planes` planes.
 Plan plan_tiles(const Geom& g, int planes);
@@ -44,11 +56,16 @@ int item_iterations(const Geom& g, const Plan& p);
 // Microseconds: an SM's iteration, a launch, and a float32 cell's step in the
 // one-step kernels on the whole GPU (see worth_alone).
 constexpr double kIterationUs = 1.65, kLaunchUs = 1.5, kCellUs = 1.0 / 31000.0;
+// The same in the padded layout, whose first and last tiles bring twice the
+// side pieces, and of the one-step kernel on such rows.
+constexpr double kPaddedIterationUs = 1.85, kPaddedCellUs = 1.0 / 30000.0;
 
 cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, LatticePtr* out);
 // Two fused steps of one lattice from buffer `from` into the other one.
 cudaError_t launch(const Lattice& l, int from, const float* src, float* dst, const Geom& g, const CollideF32& cp,
                    unsigned* err, cudaStream_t s);
+// One fused step from the plain into the padded layout, or (out) back.
+cudaError_t launch_edge(bool out, const float* src, float* dst, const Geom& g, const CollideF32& cp, cudaStream_t s);
 
 }  // namespace two
 }  // namespace imex

@@ -108,3 +108,20 @@ def test_captured_run_replays(imex, steps):
             outs.append(lat.get_f())
             lat.set_stream(None)
     assert np.array_equal(*outs)
+
+
+@pytest.mark.parametrize("shape", [(121, 150, 98), (121, 150, 97), (90, 125, 131), (400, 19, 126), (650, 9, 157), (40, 160, 127),
+                                   (200, 59, 101), (33, 150, 255), (260, 88, 62), (140, 88, 99)])
+def test_rows_of_any_length(imex, shape):
+    """Rows that are no multiple of 4 values go through the padded layout: last
+    tiles of 1, 2, 3, 5, 29, 30 and 31 columns, odd and even, every number of
+    steps left after the pairs, and a state far from equilibrium."""
+    rng = np.random.default_rng(5)
+    with imex.LBM(*shape, 0.1, 1.0, 0.05, precision=imex.IMEX_F32) as lat:
+        lat.initialize_phase(0.3, 1.1, 2.0)
+        f = lat.get_f() * (1.0 + 0.02 * rng.standard_normal((27,) + shape))
+    for steps, launches in ((9, 1 + 2 + 3), (4, 1 + 3), (5, 1 + 2 + 1), (6, 1 + 2 + 1 + 1)):
+        want, _ = run(imex, shape, steps, True, f)
+        got, n = run(imex, shape, steps, False, f)
+        assert n == launches
+        assert np.array_equal(got, want)
