@@ -3,6 +3,8 @@
 #include <algorithm>
 #include <atomic>
 #include <new>
+#include <utility>
+#include <vector>
 
 #include "two_f32.cuh"
 #include "two_f32.hpp"
@@ -93,16 +95,46 @@ Encode encode_fn()
 
 // Iterations a CTA spends beside its planes: the pipeline's 3 and the set-up.
 constexpr int kExtra = 5;
+// Planes of a brief part at least.
+constexpr int kLeastPart = 4;
 
-// Iterations of the busiest SM (one CTA each at a time).
-long long iterations(const Geom& g, const Plan& p, int sms)
+// Iterations until the last SM is done, one CTA each at a time, taken in order by
+// the SM free first.
+int iterations(const Geom& g, const Plan& p, int sms)
 {
-    return (long long)((p.items() + sms - 1) / sms) * item_iterations(g, p);
+    std::vector<std::pair<int, int>> free{{0, sms}}, next;  // (time, SMs), in order of time
+    int end = 0;
+    for (int c = 0; c < p.chunks; ++c) {
+        const int len = p.begin(c + 1, g.nx) - p.begin(c, g.nx) + kExtra;
+        int left = p.nty * p.ntz;
+        while (left > 0) {
+            const int n = std::min(left, free[0].second), t = free[0].first + len;
+            left -= n;
+            next.clear();
+            if (free[0].second > n) next.emplace_back(free[0].first, free[0].second - n);
+            bool in = false;
+            for (size_t q = 1; q < free.size(); ++q) {
+                if (!in && t <= free[q].first) {
+                    in = true;
+                    if (t == free[q].first) {
+                        next.emplace_back(t, free[q].second + n);
+                        continue;
+                    }
+                    next.emplace_back(t, n);
+                }
+                next.push_back(free[q]);
+            }
+            if (!in) next.emplace_back(t, n);
+            free.swap(next);
+            end = std::max(end, t);
+        }
+    }
+    return end;
 }
 
 Plan tiles_of(const Geom& g)
 {
-    Plan p;
+    Plan p = {};
     // full tiles and one narrower: every full tile's rows are whole 128-byte
     // lines where nz is a multiple of 32 values, and of 16 bytes always (evened
     // out, 4 x 28 for 112, each row took two lines: 112^3 43.2 us a step, now 35.8)
@@ -114,13 +146,32 @@ Plan tiles_of(const Geom& g)
     return p;
 }
 
-// The tiles cut along x so that the busiest SM has least to do.
+// The tiles cut along x so that the last SM is done soonest: in even parts, or in
+// even ones and up to three brief ones that fill the SMs left over in the end.
+// The parts of neighbouring tiles begin and end at the same planes: they share
+// rows and sectors, and read them once while they march together (cut so that
+// every SM has the same number of planes, 256^3 takes 514 us a step).  Even
+// parts alone -> with brief ones: 256^3 (399 iterations, 376) 337 -> 317 us a
+// step, 128^3 (62, 56) 50.9 -> 47.1, 96^3 (25, 25) 20.7 as before.
 Plan plan_for(const Geom& g, int sms)
 {
-    Plan p = tiles_of(g);
-    Plan best = p;
-    for (p.chunks = 2; p.chunks <= g.nx; ++p.chunks)
-        if (iterations(g, p, sms) < iterations(g, best, sms)) best = p;
+    Plan best = tiles_of(g);
+    if (best.nty * best.ntz > 32 * sms) return best;  // no last wave to speak of
+    int least = iterations(g, best, sms);
+    auto offer = [&](const Plan& p) {
+        const int n = iterations(g, p, sms);
+        if (n < least) {
+            least = n;
+            best = p;
+        }
+    };
+    Plan p = best;
+    for (p.chunks = 2; p.chunks <= std::min(g.nx, 32); ++p.chunks) offer(p);
+    for (p.briefs = 1; p.briefs <= 3; ++p.briefs)
+        for (int evens = 1; evens <= 6; ++evens) {
+            p.chunks = evens + p.briefs;
+            for (p.brief = kLeastPart; p.brief * p.chunks < g.nx; ++p.brief) offer(p);
+        }
     return best;
 }
 
@@ -165,15 +216,15 @@ Plan plan_tiles(const Geom& g, int planes)
 }
 
 // Measured: two steps in one launch take 1.5 us and 1.65 us per iteration of
-// the busiest SM (96^3 41 us, 128^3 103, 256^3 676), in two launches of the
+// the busiest SM (96^3 41 us, 128^3 94, 256^3 635), in two launches of the
 // one-step kernel cells / 31 per ns each (96^3 59 us, 128^3 134, 256^3 1034;
 // below 80^3 less, the lattice then stays in L2: 80^3 28 us against 35). So
 // small lattices, whose tiles leave SMs idle or spend most iterations filling
 // the pipeline, and shapes that fit the tiles badly keep one step per launch;
 // the line lies near 85^3.  Padded layout, single -> two steps, us a step: 255^3
-// 546 -> 357, 131 x 128 x 128 68.8 -> 63.7, 97 x 150 x 121 (four tiles for
-// three and a value) 59.1 -> 55.3, 111^3 48.5 -> 38.8, 85^3 20.3 -> 19.9 (not taken),
-// 65 x 160 x 160 54.1 -> 55.6 (not taken).
+// 546 -> 343, 131 x 128 x 128 68.8 -> 57.0, 97 x 150 x 121 (four tiles for
+// three and a value) 59.1 -> 52.4, 111^3 48.5 -> 38.9, 85^3 20.3 -> 19.9 (not taken),
+// 65 x 160 x 160 54.0 -> 53.8.
 bool worth_alone(const Geom& g, int sms)
 {
     if (!eligible(g) && !padded_eligible(g)) return false;

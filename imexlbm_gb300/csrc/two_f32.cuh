@@ -96,8 +96,8 @@ __device__ __forceinline__ Box box_of(const Plan& p, int nx, int ny, int nz, int
     const int tiles = p.nty * p.ntz, chunk = item / tiles, t = item - chunk * tiles;
     const int iy = t / p.ntz, iz = t - iy * p.ntz;
     Box b;  // part i of n balanced parts of a length starts at i * length / n
-    b.x0 = (int)((long long)chunk * nx / p.chunks);
-    b.planes = (int)((long long)(chunk + 1) * nx / p.chunks) - b.x0;
+    b.x0 = p.begin(chunk, nx);
+    b.planes = p.begin(chunk + 1, nx) - b.x0;
     b.y0 = (int)((long long)iy * ny / p.nty);
     b.rows = (int)((long long)(iy + 1) * ny / p.nty) - b.y0;
     b.z0 = iz * p.tz;

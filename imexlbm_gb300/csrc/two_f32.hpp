@@ -19,10 +19,17 @@ struct alignas(64) Maps {
 };
 
 // How a lattice is cut: nty x ntz tiles of at most ty x tz destinations, each
-// marched in `chunks` parts along x.
+// marched in `chunks` parts along x, the last `briefs` of `brief` planes and the
+// others even.
 struct Plan {
-    int ty, tz, nty, ntz, chunks;
+    int ty, tz, nty, ntz, chunks, briefs, brief;
     int items() const { return nty * ntz * chunks; }
+    // Plane at which part i of nx planes begins.
+    __host__ __device__ int begin(int i, int nx) const
+    {
+        const int evens = chunks - briefs;
+        return i > evens ? nx - (chunks - i) * brief : (int)((long long)i * (nx - briefs * brief) / evens);
+    }
 };
 
 // The padded layout of a lattice whose rows are no multiple of 4 values: within
