@@ -166,22 +166,24 @@ __global__ void __launch_bounds__(kUnitThreads) k_batch_units(const BatchHeader*
     void* dst = e.buf[e.cur ^ (s & 1) ^ 1];
     CollideF32 cp = base;
     cp.eps = e.eps;
-    auto run = [&](auto prec, auto near_) {
+    auto run = [&](auto prec, auto even) {
         constexpr int P = decltype(prec)::value;
-        constexpr bool kNear = decltype(near_)::value;
+        constexpr bool kEven = decltype(even)::value;
         using T = typename lowp::Storage<P>::T;
-        const unsigned c = flat::first_cell<kNear>(seg, threadIdx.x);
+        const unsigned c = flat::first_cell<P, kEven>(seg, threadIdx.x);
         if (c < (unsigned)e.plane)
-            flat::step_pair<P, kNear, true>(static_cast<const T*>(src), static_cast<T*>(dst), e.nx, e.ny, e.nz, e.plane, c, cp);
+            flat::step_pair<P, kEven, true>(static_cast<const T*>(src), static_cast<T*>(dst), e.nx, e.ny, e.nz, e.plane, c, cp);
     };
+    const bool even = !(e.plane & 1);
     if (PF != IMEX_F32 && e.prec == IMEX_F16DEV) {
         cp.sr = e.sr;
         cp.seed = e.seed + (uint32_t)s;
-        run(std::integral_constant<int, IMEX_F16DEV>{}, std::true_type{});
-    } else if (e.plane & 1) {
-        run(std::integral_constant<int, IMEX_F32>{}, std::false_type{});
-    } else {
+        if (even) run(std::integral_constant<int, IMEX_F16DEV>{}, std::true_type{});
+        else run(std::integral_constant<int, IMEX_F16DEV>{}, std::false_type{});
+    } else if (even) {
         run(std::integral_constant<int, IMEX_F32>{}, std::true_type{});
+    } else {
+        run(std::integral_constant<int, IMEX_F32>{}, std::false_type{});
     }
 }
 

@@ -13,9 +13,12 @@
 // both; no thread is idle whatever nz is.  The two cells' sources are
 // separate sums of an x, a y and a z offset, so a pair may lie across a
 // row's end.
-// Measured per step, before -> now: float16 131 x 77 x 90 37.0 -> 21.3 us, 107 x
-// 99 x 84 33.0 -> 20.6, 255^3 469 -> 383, 256^3 468 -> 335 (the row-staged kernel:
-// 281); float32 97 x 150 x 121 69.9 -> 61.7, 255^3 575 -> 547, 256^3 527 -> 520
+// Of an odd number of cells the even directions' pairs still lie on a 4-byte
+// boundary and are stored at once; the number's parity is a template argument
+// (255^3 float16 377 -> 350 us, 45^3 4.9 -> 4.0).
+// Measured per step, one cell per thread -> now: float16 131 x 77 x 90 37.0 -> 18.0
+// us, 107 x 99 x 84 33.0 -> 17.3, 255^3 469 -> 350, 256^3 468 -> 335 (the row-staged
+// kernel: 281); float32 97 x 150 x 121 69.9 -> 59.1, 255^3 575 -> 546, 256^3 527 -> 520
 // (memory alone: 543 at the copy rate).  Bound: memory for float32, issue for float16.
 #pragma once
 
@@ -29,30 +32,31 @@ constexpr int kThreads = 128;
 constexpr int kCells = 2 * kThreads;  // cells of a CTA
 
 // A thread's pair is two neighbours, cells 2 t and 2 t + 1 of its CTA's
-// kCells (kNear), or cells t and t + kThreads.  Float32 results of an odd number of
+// kCells (near), or cells t and t + kThreads.  Float32 results of an odd number of
 // cells lie off their 8-byte boundary in every other direction: there the
 // second form keeps lanes on consecutive cells, so that the 4-byte accesses
 // coalesce (61 x 65 x 63: 10.3 us against 12.3; 64^3 8.4 in the first form,
 // 10.3 in the second).
-template <bool kNear>
+template <int P, bool kEven>
+inline constexpr bool kNear = kEven || P == IMEX_F16DEV;
+template <int P, bool kEven>
 __device__ __forceinline__ unsigned first_cell(unsigned block, unsigned t)
 {
-    return block * kCells + (kNear ? 2 * t : t);
+    return block * kCells + (kNear<P, kEven> ? 2 * t : t);
 }
 
 // Fused step of the pair whose first cell is c < plane (the second may lie
-// beyond the last cell) of a lattice of fewer than 2^32 cells.  kNear as
-// above; float16 pairs are neighbours.  Ends its kernel's chain (chain_end).
-template <int P, bool kNear, bool kEarly>
+// beyond the last cell) of a lattice of fewer than 2^32 cells; kEven: of an even
+// number of them.  Ends its kernel's chain (chain_end).
+template <int P, bool kEven, bool kEarly>
 __device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __restrict__ src,
                                           typename lowp::Storage<P>::T* __restrict__ dst, int nx, int ny, int nz,
                                           size_t plane, unsigned c, const CollideF32& cp)
 {
-    static_assert(kNear || P == IMEX_F32, "float16 pairs share a random word");
     using S = lowp::Storage<P>;
     using T = typename S::T;
     using A = lowp::F2;
-    constexpr unsigned kNext = kNear ? 1 : kThreads;
+    constexpr unsigned kNext = kNear<P, kEven> ? 1 : kThreads;  // float16 pairs share a random word
     const bool two = c + kNext < (unsigned)plane;
     const FlatPull p0(nx, ny, nz, c), p1(nx, ny, nz, two ? c + kNext : c);
     float2 h[kQ];
@@ -66,12 +70,11 @@ __device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __
     chain_end<kEarly>();
     T* const o = dst + c;
     if constexpr (P == IMEX_F16DEV) {
-        // an odd number of cells puts every other direction's pairs off their
+        // an odd number of cells puts the odd directions' pairs off their
         // 4-byte boundary
-        const bool whole = two && !(plane & 1);
         auto put = [&](int a, __half2 r) {
             T* const q = o + (size_t)a * plane;
-            if (whole) {
+            if ((kEven || !(a & 1)) && two) {
                 *reinterpret_cast<__half2*>(q) = r;
             } else {
                 q[0] = __low2half(r);
@@ -98,7 +101,7 @@ __device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __
         for (int a = 0; a < kQ; ++a) {
             T* const q = o + (size_t)a * plane;
             const float2 v = make_float2(S::store(h[a].x, a), S::store(h[a].y, a));
-            if (kNear && two) {  // plane even: 8-byte aligned
+            if (kEven && two) {  // plane even: 8-byte aligned
                 *reinterpret_cast<float2*>(q) = v;
             } else {
                 q[0] = v.x;

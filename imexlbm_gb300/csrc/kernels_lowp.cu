@@ -54,16 +54,16 @@ __global__ void __launch_bounds__(kStepBlock) k_step_lowp(const typename Storage
 }
 
 // The fused step over flat cell pairs (flat_lowp.cuh).
-template <int P, bool kNear, bool SR, bool kEarly>
+template <int P, bool kEven, bool SR, bool kEarly>
 __global__ void __launch_bounds__(flat::kThreads) k_flat_lowp(const typename Storage<P>::T* __restrict__ src,
                                                               typename Storage<P>::T* __restrict__ dst, Geom g,
                                                               CollideF32 cp)
 {
     chain_begin<kEarly>();
-    const unsigned c = flat::first_cell<kNear>(blockIdx.x, threadIdx.x);
+    const unsigned c = flat::first_cell<P, kEven>(blockIdx.x, threadIdx.x);
     if (c >= (unsigned)g.plane) return;
     cp.sr = SR;
-    flat::step_pair<P, kNear, kEarly>(src, dst, g.nx, g.ny, g.nz, g.plane, c, cp);
+    flat::step_pair<P, kEven, kEarly>(src, dst, g.nx, g.ny, g.nz, g.plane, c, cp);
 }
 
 // Taylor-Green initial state (float64 equilibrium, src/lbm.cpp:78-108),
@@ -146,13 +146,15 @@ cudaError_t step_impl(int mode, const void* src, void* dst, const Geom& g, const
         const unsigned grid = (unsigned)((g.plane + flat::kCells - 1) / flat::kCells);
         const bool early = chain_early(grid);
         auto go = [&](auto kernel) { return launch_chained(kernel, grid, flat::kThreads, 0, s, a, b, g, cp); };
+        auto of = [&](auto even, auto sr) {
+            constexpr bool kEven = decltype(even)::value, kSr = decltype(sr)::value;
+            return early ? go(k_flat_lowp<P, kEven, kSr, true>) : go(k_flat_lowp<P, kEven, kSr, false>);
+        };
+        const bool even = !(g.plane & 1);
         if constexpr (P == IMEX_F16DEV) {
-            if (cp.sr) return early ? go(k_flat_lowp<P, true, true, true>) : go(k_flat_lowp<P, true, true, false>);
-            return early ? go(k_flat_lowp<P, true, false, true>) : go(k_flat_lowp<P, true, false, false>);
-        } else {
-            if (g.plane & 1) return early ? go(k_flat_lowp<P, false, false, true>) : go(k_flat_lowp<P, false, false, false>);
-            return early ? go(k_flat_lowp<P, true, false, true>) : go(k_flat_lowp<P, true, false, false>);
+            if (cp.sr) return even ? of(std::true_type{}, std::true_type{}) : of(std::false_type{}, std::true_type{});
         }
+        return even ? of(std::true_type{}, std::false_type{}) : of(std::false_type{}, std::false_type{});
     }
     case kModeCollide: k_step_lowp<P, true><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
     case kModeStream: k_step_lowp<P, false><<<step_grid(g), kStepBlock, 0, s>>>(a, b, g, cp); break;
