@@ -114,7 +114,7 @@ __device__ __noinline__ void add_outside(const typename mom::Elem<P>::T* src, Ge
 template <int P, bool PULL, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB)
     k_conserved(const typename mom::Elem<P>::T* __restrict__ src, Geom g, unsigned cells, Partial* __restrict__ part,
-                unsigned* __restrict__ ticket, double* __restrict__ out)
+                unsigned* __restrict__ ticket, const unsigned long long* __restrict__ status, double* __restrict__ out)
 {
     __shared__ BlockSum s;
     __shared__ int s_last;
@@ -190,6 +190,8 @@ __global__ void __launch_bounds__(kThreads, MINB)
                 if (__ldcg(&part[b].any_out))
                     for (int q = 0; q < 5; ++q) r[q] += __ldcg(&part[b].out[q]);
         for (int q = 0; q < 5; ++q) out[q] = r[q];
+        if (status)
+            for (int q = 0; q < 2; ++q) reinterpret_cast<unsigned long long*>(out)[5 + q] = __ldcg(status + q);
         *ticket = 0;  // for the next launch
     }
 }
@@ -204,15 +206,16 @@ inline unsigned blocks_for(size_t cells, int sms, int per_sm)
 constexpr int kMostPerSm = 4;
 
 template <int P, int MINB>
-cudaError_t launch(bool pull, const void* src, const Geom& g, void* part, unsigned* ticket, double* out, cudaStream_t s)
+cudaError_t launch(bool pull, const void* src, const Geom& g, void* part, unsigned* ticket,
+                   const unsigned long long* status, double* out, cudaStream_t s)
 {
     const size_t cells = (size_t)g.nx * g.ny * g.nz;
     if (cells > 0xffffffffull) return cudaErrorInvalidValue;
     const unsigned grid = blocks_for(cells, current_sm_count(), MINB);
     const auto* p = static_cast<const typename mom::Elem<P>::T*>(src);
     auto* pt = static_cast<Partial*>(part);
-    return pull ? launch_chained(k_conserved<P, true, MINB>, grid, kThreads, 0, s, p, g, (unsigned)cells, pt, ticket, out)
-                : launch_chained(k_conserved<P, false, MINB>, grid, kThreads, 0, s, p, g, (unsigned)cells, pt, ticket, out);
+    return pull ? launch_chained(k_conserved<P, true, MINB>, grid, kThreads, 0, s, p, g, (unsigned)cells, pt, ticket, status, out)
+                : launch_chained(k_conserved<P, false, MINB>, grid, kThreads, 0, s, p, g, (unsigned)cells, pt, ticket, status, out);
 }
 
 }  // namespace cons

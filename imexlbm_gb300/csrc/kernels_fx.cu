@@ -500,10 +500,10 @@ cudaError_t launch_fx_to_f64(double* buf, size_t n, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_conserved_fx(bool pull, const double* src, const Geom& g, void* partial, unsigned* ticket, double* out,
-                                cudaStream_t s)
+cudaError_t launch_conserved_fx(bool pull, const double* src, const Geom& g, void* partial, unsigned* ticket,
+                                const unsigned long long* status, double* out, cudaStream_t s)
 {
-    return cons::launch<IMEX_F64, 2>(pull, src, g, partial, ticket, out, s);
+    return cons::launch<IMEX_F64, 2>(pull, src, g, partial, ticket, status, out, s);
 }
 
 }  // namespace imex

@@ -51,8 +51,9 @@ bool rows_fx_eligible(const Geom& g);
 cudaError_t launch_rows_fx(const double* src, double* dst, const Geom& g, const FxParams& fx, const CollideF64& cp,
                            unsigned long long* fallback, const RowConfig& rc, unsigned* err, cudaStream_t s);
 // Conserved sums (conserved.cuh): partial holds conserved_scratch_bytes(),
-// *ticket is 0 before and after the launch.
-cudaError_t launch_conserved_fx(bool pull, const double* src, const Geom& g, void* partial, unsigned* ticket, double* out,
-                                cudaStream_t s);
+// *ticket is 0 before and after the launch; *out takes the 5 sums and, if status
+// is not null, status[0] and status[1] after them.
+cudaError_t launch_conserved_fx(bool pull, const double* src, const Geom& g, void* partial, unsigned* ticket,
+                                const unsigned long long* status, double* out, cudaStream_t s);
 
 }  // namespace imex

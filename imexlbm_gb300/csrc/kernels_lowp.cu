@@ -311,10 +311,10 @@ cudaError_t launch_velocity_diff(int prec_a, const void* fa, bool pull_a, int pr
 }
 
 cudaError_t launch_conserved_lowp(int prec, bool pull, const void* src, const Geom& g, void* partial, unsigned* ticket,
-                                  double* out, cudaStream_t s)
+                                  const unsigned long long* status, double* out, cudaStream_t s)
 {
-    return prec == IMEX_F32 ? cons::launch<IMEX_F32, 3>(pull, src, g, partial, ticket, out, s)
-                            : cons::launch<IMEX_F16DEV, 3>(pull, src, g, partial, ticket, out, s);
+    return prec == IMEX_F32 ? cons::launch<IMEX_F32, 3>(pull, src, g, partial, ticket, status, out, s)
+                            : cons::launch<IMEX_F16DEV, 3>(pull, src, g, partial, ticket, status, out, s);
 }
 
 size_t conserved_scratch_bytes(const Geom& g)

@@ -45,9 +45,10 @@ cudaError_t launch_macro(int prec, bool pull, const void* src, const Geom& g, do
 cudaError_t launch_velocity_diff(int prec_a, const void* fa, bool pull_a, int prec_b, const void* fb, bool pull_b,
                                  const Geom& g, unsigned long long* res, cudaStream_t s);
 // Conserved sums (conserved.cuh): partial holds conserved_scratch_bytes(),
-// *ticket is 0 before and after the launch.
+// *ticket is 0 before and after the launch; *out takes the 5 sums and, if status
+// is not null, status[0] and status[1] after them.
 cudaError_t launch_conserved_lowp(int prec, bool pull, const void* src, const Geom& g, void* partial, unsigned* ticket,
-                                  double* out, cudaStream_t s);
+                                  const unsigned long long* status, double* out, cudaStream_t s);
 size_t conserved_scratch_bytes(const Geom& g);
 
 }  // namespace imex

@@ -187,6 +187,8 @@ std::vector<RowConfig> row_candidates(const imex_lattice* h)
     return out;
 }
 
+constexpr int kNoFailByte = 0x7f;  // of a fixed-point run's flag while no step has failed
+
 std::mutex g_tune_lock;
 std::map<std::tuple<int, int, int, int, int>, RowConfig> g_tune_cache;
 
@@ -258,7 +260,8 @@ int time_fixed_run(imex_lattice* h, int reps, float* ms)
     const int n = reps + 2;  // launches 2 .. n-1 read and write X
     double* x = dbuf(h, 1 - h->cur);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    cudaError_t e = cudaMemsetAsync(h->d_fail, 0x7f, sizeof(int), h->stream);
+    h->fail_clear = false;
+    cudaError_t e = cudaMemsetAsync(h->d_fail, kNoFailByte, sizeof(int), h->stream);
     if (e == cudaSuccess) e = launch_step_fx_run(dbuf(h, h->cur), x, h->g, h->fx, 1, n, h->d_fail, h->stream);
     if (e == cudaSuccess) e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
@@ -280,6 +283,82 @@ int time_fixed_run(imex_lattice* h, int reps, float* ms)
 }
 
 int check_kernel_error(imex_lattice* h);
+
+// Small results on their way to the host: a kernel or a copy writes them to a
+// slot of one page of pinned memory, which the host reads after the synchronisation
+// it makes anyway; a copy into pageable memory costs another 4 to 8 us (a report
+// of a 32^3 float64 lattice, 10 steps and the sums, 98 us so, 87 with the slot).  A slot is held for a call and
+// free again after it; without one (64 calls at once, no page) the call
+// copies.  The page is made by the first imex_create and kept; it is gone
+// after a cudaDeviceReset, which each use finds out, and made anew by the next
+// imex_create.
+constexpr size_t kSlotBytes = 64;
+constexpr int kSlots = 64;
+std::mutex g_page_lock;
+std::atomic<unsigned char*> g_page{nullptr};
+std::atomic<unsigned long long> g_slots_used{0};
+
+// The page's address on the device, or nullptr if it is no pinned memory (any more).
+unsigned char* page_device(unsigned char* page)
+{
+    cudaPointerAttributes at{};
+    if (!page) return nullptr;
+    if (cudaPointerGetAttributes(&at, page) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? static_cast<unsigned char*>(at.devicePointer) : nullptr;
+}
+
+void make_report_page()
+{
+    std::lock_guard<std::mutex> guard(g_page_lock);
+    if (page_device(g_page.load())) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // no concern of another thread's capture
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kSlots * kSlotBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    g_page.store(static_cast<unsigned char*>(p));
+}
+
+class ReportSlot {
+public:
+    explicit ReportSlot(bool want = true)
+    {
+        unsigned char* const page = want ? g_page.load() : nullptr;
+        unsigned char* const dev = page_device(page);
+        if (!dev) return;
+        unsigned long long used = g_slots_used.load();
+        do {
+            index_ = 0;
+            while (index_ < kSlots && (used >> index_ & 1)) ++index_;
+            if (index_ == kSlots) return;
+        } while (!g_slots_used.compare_exchange_weak(used, used | 1ull << index_));
+        host_ = page + index_ * kSlotBytes;
+        dev_ = dev + index_ * kSlotBytes;
+    }
+    ~ReportSlot()
+    {
+        if (host_) g_slots_used.fetch_and(~(1ull << index_));
+    }
+    ReportSlot(const ReportSlot&) = delete;
+    ReportSlot& operator=(const ReportSlot&) = delete;
+    explicit operator bool() const { return host_ != nullptr; }
+    void* device() const { return dev_; }
+    void* host() const { return host_; }
+    void read(void* to, size_t n) const { std::memcpy(to, host_, n); }
+
+private:
+    int index_ = 0;
+    unsigned char* host_ = nullptr;
+    unsigned char* dev_ = nullptr;
+};
+
+bool capturing(imex_lattice* h);
 
 // Resources of the two-steps-per-launch kernel (per handle, grown to the
 // deepest ring a launch shape asks for): the ticket counter, 2 nx ny row
@@ -420,8 +499,10 @@ int check_ready(imex_lattice* h, const char* what)
 int check_kernel_error(imex_lattice* h)
 {
     unsigned v = 0;
-    IMEX_CUDA(h, cudaMemcpyAsync(&v, h->d_err, sizeof v, cudaMemcpyDeviceToHost, h->stream), "cudaMemcpy");
+    const ReportSlot slot(!capturing(h));
+    IMEX_CUDA(h, cudaMemcpyAsync(slot ? slot.host() : &v, h->d_err, sizeof v, cudaMemcpyDeviceToHost, h->stream), "cudaMemcpy");
     IMEX_CUDA(h, cudaStreamSynchronize(h->stream), "kernel status");
+    if (slot) slot.read(&v, sizeof v);
     if (v) {
         IMEX_CUDA(h, cudaMemsetAsync(h->d_err, 0, sizeof v, h->stream), "cudaMemset");
         return fail(h, IMEX_ERR_CUDA, "a kernel's asynchronous copy did not complete in time; its results are invalid");
@@ -569,6 +650,7 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     h->d_err = reinterpret_cast<unsigned*>(h->d_fallback + 1);
     h->d_fail = reinterpret_cast<int*>(h->d_fallback + 2);
     h->d_ticket = reinterpret_cast<unsigned*>(h->d_fallback + 3);
+    make_report_page();
     e = cudaMemsetAsync(h->d_fallback, 0, 4 * sizeof(unsigned long long), h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);  // usable from any stream from here on
     if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "imex_create"));
@@ -703,7 +785,8 @@ int step_fixed_run(imex_lattice* h, int n)
         int rc = ensure_two_step(h, h->rows.rows);
         if (rc) return rc;
     }
-    IMEX_CUDA(h, cudaMemsetAsync(h->d_fail, 0x7f, sizeof(int), h->stream), "cudaMemset");
+    if (!h->fail_clear) IMEX_CUDA(h, cudaMemsetAsync(h->d_fail, kNoFailByte, sizeof(int), h->stream), "cudaMemset");
+    h->fail_clear = false;  // until the run has come to its end
     for (int j = 1; j <= n;) {
         PhaseScope timed(h->prof, IMEX_PHASE_COLLISION, h->stream);
         runs.emplace_back(j, h->cur);
@@ -720,8 +803,12 @@ int step_fixed_run(imex_lattice* h, int n)
         j += k;
     }
     int failed = 0;
-    IMEX_CUDA(h, cudaMemcpyAsync(&failed, h->d_fail, sizeof failed, cudaMemcpyDeviceToHost, h->stream), "cudaMemcpy");
+    const ReportSlot slot;
+    void* const to = slot ? slot.host() : &failed;
+    IMEX_CUDA(h, cudaMemcpyAsync(to, h->d_fail, sizeof failed, cudaMemcpyDeviceToHost, h->stream), "cudaMemcpy");
     IMEX_CUDA(h, cudaStreamSynchronize(h->stream), "fixed-point run");
+    if (slot) slot.read(&failed, sizeof failed);
+    h->fail_clear = failed > n;
     if (two) {
         int rc = check_kernel_error(h);  // a bounded wait of the two-step kernel ran out
         if (rc) return rc;
@@ -838,23 +925,29 @@ int imex_conserved(imex_lattice* h, double out[5])
     if (rc) return rc;
     if (!out) return fail(h, IMEX_ERR_ARG, "imex_conserved: null output");
     const bool pull = h->tag == kPendingStream;
-    int timed = h->prof.start(IMEX_PHASE_CONSERVED, h->stream);
-    cudaError_t e =
-        is_lowp(h) ? launch_conserved_lowp(h->precision, pull, h->buf[h->cur], h->g, h->d_partial, h->d_ticket, h->d_out,
-                                           h->stream)
-        : use_fixed(h)
-            ? launch_conserved_fx(pull, dbuf(h, h->cur), h->g, h->d_partial, h->d_ticket, h->d_out, h->stream)
-            : launch_conserved_f64(pull, dbuf(h, h->cur), h->g, h->d_partial, h->d_out, h->stream);
-    h->prof.stop(timed, h->stream);
-    if (e != cudaSuccess) return cuda_fail(h, e, "conserved kernel launch");
-    h->launches += is_lowp(h) || use_fixed(h) ? 1 : 2;
-    // the 5 sums, the fallback counter and the error flag lie in a row: one copy
+    // the 5 sums, the fallback counter and the error flag, in a row
     struct {
         double sums[5];
         unsigned long long fallback, err;
     } res;
-    IMEX_CUDA(h, cudaMemcpyAsync(&res, h->d_out, sizeof res, cudaMemcpyDeviceToHost, h->stream), "cudaMemcpy");
+    const bool single = is_lowp(h) || use_fixed(h);  // one launch, which can write to the host itself
+    const ReportSlot slot(single && !capturing(h));
+    double* const out_dev = slot ? static_cast<double*>(slot.device()) : h->d_out;
+    const unsigned long long* const status = slot ? h->d_fallback : nullptr;
+    int timed = h->prof.start(IMEX_PHASE_CONSERVED, h->stream);
+    cudaError_t e =
+        is_lowp(h) ? launch_conserved_lowp(h->precision, pull, h->buf[h->cur], h->g, h->d_partial, h->d_ticket, status,
+                                           out_dev, h->stream)
+        : use_fixed(h)
+            ? launch_conserved_fx(pull, dbuf(h, h->cur), h->g, h->d_partial, h->d_ticket, status, out_dev, h->stream)
+            : launch_conserved_f64(pull, dbuf(h, h->cur), h->g, h->d_partial, h->d_out, h->stream);
+    h->prof.stop(timed, h->stream);
+    if (e != cudaSuccess) return cuda_fail(h, e, "conserved kernel launch");
+    h->launches += single ? 1 : 2;
+    if (!slot)
+        IMEX_CUDA(h, cudaMemcpyAsync(&res, h->d_out, sizeof res, cudaMemcpyDeviceToHost, h->stream), "cudaMemcpy");
     IMEX_CUDA(h, cudaStreamSynchronize(h->stream), "imex_conserved");
+    if (slot) slot.read(&res, sizeof res);
     if (res.err) {
         rc = check_kernel_error(h);  // reports it and clears the flag
         if (rc) return rc;

@@ -50,6 +50,7 @@ struct imex_lattice {
     bool fx_ok = false;  // fixed-point engine usable for this lattice
     unsigned* d_err = nullptr;  // set by kernels whose bounded waits ran out
     int* d_fail = nullptr;      // first failing step of a fixed-point run (imex_step)
+    bool fail_clear = false;    // *d_fail is as a run needs it
     int64_t fx_reruns = 0;      // fixed-point runs redone from a failing step
     int fx_skip = 0;            // imex_step calls left that step one at a time after a failed run
     // two fused steps per launch (launch_two_step_fx): ticket counter, row
