@@ -54,8 +54,18 @@ __global__ void __launch_bounds__(kStepBlock) k_step_lowp(const typename Storage
 }
 
 // The fused step over flat cell pairs (flat_lowp.cuh).
+// CTAs per SM the registers are held to; 0: as the compiler has it (90 at most,
+// 5 CTAs).  Six fit without a spill where nothing is drawn at random (float16 to
+// nearest: 107 x 99 x 84 17.25 -> 17.08 us a step, 64 x 64 x 63 6.50 -> 6.00, 45^3 4.24 ->
+// 3.51; float32 with 6: 64^3 6.44 -> 6.92); a lattice whose CTAs all run at once
+// gains from room for its loads' addresses instead (1; stochastic 64 x 64 x 63
+// 6.55 -> 6.16, 45^3 3.87 -> 3.57; float32 61 x 65 x 63 7.79 -> 7.44, but 64^3 6.44 -> 6.62).
 template <int P, bool kEven, bool SR, bool kEarly>
-__global__ void __launch_bounds__(flat::kThreads) k_flat_lowp(const typename Storage<P>::T* __restrict__ src,
+inline constexpr int kFlatCtas = P == IMEX_F16DEV && !SR                      ? 6
+                                 : !kEarly && (P == IMEX_F16DEV || !kEven) ? 1
+                                                                              : 0;
+template <int P, bool kEven, bool SR, bool kEarly>
+__global__ void __launch_bounds__(flat::kThreads, kFlatCtas<P, kEven, SR, kEarly>) k_flat_lowp(const typename Storage<P>::T* __restrict__ src,
                                                               typename Storage<P>::T* __restrict__ dst, Geom g,
                                                               CollideF32 cp)
 {
