@@ -285,7 +285,7 @@ def extended_precision(hbm: float):
     500 steps."""
     from imexlbm_gb300 import sweep
     r = sweep.run(size=512, steps=2000, report=500, log=lambda _: None)
-    bpc = {"f64": 432, "f32": 216, "f16dev": 108, "f16dev_sr": 108}
+    bpc = {"f64": 432, "f32": 108, "f16dev": 108, "f16dev_sr": 108}  # float32: two steps per read and write
     out = {"workload": "taylor-green 512^3, Re=1600, u0=0.05, 2000 steps, errors vs the float64 run every 500 steps",
            "runs": {}}
     for name, mlups in r["mlups"].items():
@@ -431,19 +431,22 @@ def run_ours(a):
     # launches read / write float64)
     hbm, peak_kind = load_peaks()
     bpc = BYTES_PER_CELL[a.precision]
-    # algorithmic bytes per step over the time per step (a launch is one step,
-    # or two for the pinned two-steps-per-launch shape)
-    achieved = bpc * cells * a.steps / (ms * 1e-3) / 1e9
     kname = {"fixed": "step_fxs", "native": "step_f64", "float32": "step_lowp_" + a.precision}[eng_name]
+    # algorithmic bytes per step over the time per step (a launch is one step,
+    # or two for the pinned float64 two-steps-per-launch shape)
+    per_launch = bpc * cells
     if eng_name == "fixed" and launch_shape[0] == 1:
-        kname = "two_fxs"
+        kname, per_launch = "two_fxs", 2 * bpc * cells
+    elif a.precision == "f32" and gpu_launches < a.steps:
+        kname, bpc = "two_f32", bpc / 2  # one read and one write per two steps
+    achieved = bpc * cells * a.steps / (ms * 1e-3) / 1e9
     tr, tr_size = load_traffic(kname)
     roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
             "frac": round(achieved / hbm, 4), "peak_kind": peak_kind,
             "traffic": round(tr * cells, 0) if tr is not None else None,
             "traffic_from": (f"ncu dram bytes per cell of a {tr_size} capture ({tr} B), times this launch's "
                              f"{cells} cells (profiles/dram_traffic.json)") if tr is not None else None,
-            "kernel": kname, "algorithmic_bytes_per_launch": bpc * cells * (2 if kname == "two_fxs" else 1)}
+            "kernel": kname, "algorithmic_bytes_per_launch": per_launch}
 
     # end-to-end through the public API with host buffers
     e2e = None

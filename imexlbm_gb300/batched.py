@@ -5,11 +5,11 @@ Default workload (seeded, numpy PCG64 seed 20261203): 64 cubic lattices,
 edges uniform over {32, 48, 64, 96, 128}, Re uniform in [100, 3200] cast to
 int as the deck does, u0 uniform in [0.02, 0.08], a phase offset uniform in
 [0, 2 pi)^3 added to x, y, z of the Taylor-Green field, 500 steps each,
-float32 storage, one persistent launch per step (captured in CUDA graphs,
-launch shape from the autotuner).
+float32 storage, a few launches per step or per two steps (captured in CUDA
+graphs).
 
 Reported: the batch's aggregate MLUPS (sum of cells x steps / wall time of
-the batched steps, after one warm-up step that includes the autotuner), the
+the batched steps, after one warm-up step), the
 plain float64 path's aggregate MLUPS on the same lattices (one lattice per
 launch, one after the other), their ratio, and per lattice the kinetic-
 energy error against its float64 run, mass drift and momentum.
@@ -72,7 +72,7 @@ def run(n=64, steps=500, precision="f32", seed=20261203, log=print, check_fp64=T
     m0 = [lat.Conserved()[0] for lat in lats]
     launches0 = batch.kernel_launches()
     t0 = time.perf_counter()
-    batch.step(1)          # autotuner + first (in-place) collision of every member
+    batch.step(1)          # first (in-place) collision of every member
     batch.synchronize()
     t_warm = time.perf_counter() - t0
     launches1 = batch.kernel_launches()
@@ -123,9 +123,9 @@ def main(argv=None) -> int:
     ap.add_argument("--seed", type=int, default=20261203)
     ap.add_argument("--no-fp64", action="store_true")
     ap.add_argument("--row-launch", default=None, metavar="STAGES,KB,CTAS",
-                    help="pin the row kernel's shape (-1,0,0: off) instead of autotuning it")
+                    help="pin the row kernel's shape (-1,0,0: off)")
     ap.add_argument("--launch", default=None, metavar="THREADS,CPT,CTAS",
-                    help="pin the one-thread-per-cell kernel's shape instead of autotuning it")
+                    help="pin the one-thread-per-cell kernel's shape")
     ap.add_argument("--json", default=None)
     a = ap.parse_args(argv)
     rl = tuple(int(v) for v in a.row_launch.split(",")) if a.row_launch else None

@@ -1,26 +1,27 @@
-// Batched step: many reduced-precision lattices of any sizes advance in one
-// persistent launch over a packed cell index.
+// Batched step: many reduced-precision lattices of any sizes advance together
+// in a few launches per step, whatever their number.
 //
 // A batch holds member lattice handles (float32 or float16-deviation
-// storage).  Their cells are numbered consecutively - lattice after
-// lattice, each in its own f[a][x][y][z] order - and every launch of the
-// persistent kernel walks that packed index: a thread finds its lattice by
-// binary search over the members' first-cell indices, decodes (x, y, z),
-// pulls the 27 values from that lattice's buffer with periodic wrap,
-// collides in float32 (lowp_math.cuh, the same arithmetic as the
-// one-lattice kernels, so results are bit-identical) and writes the other
-// buffer.  Lattices of different sizes, viscosities and storage formats mix
-// in one launch; no launch is spent on a small lattice alone.
+// storage); lattices of different sizes, viscosities and storage formats mix,
+// each in its own f[a][x][y][z] order.  The arithmetic is the one-lattice
+// kernels' (lowp_math.cuh), so results are bit-identical to stepping alone.
 //
-// The member table lives in device memory and the kernel reads it at every
-// launch, so a CUDA graph of K launches (step index s = 0..K-1 baked in)
+// The member tables live in device memory and the kernels read them at every
+// launch, so a CUDA graph of K steps' launches (step index s = 0..K-1 baked in)
 // stays valid while members join, leave or finish: a member runs at step s
 // only while s < its step count for the tick, and within a tick it reads
 // buf[cur ^ (s & 1)] and writes the other buffer.
 //
-// Members whose rows suit asynchronous bulk copies (nz * element size a
-// multiple of 16 bytes) run instead in a second persistent kernel, the
-// batched form of the row-staged step (rows.cuh): its work items are blocks
+// Float32 members whose rows suit tensor copies step twice per launch, in the
+// batched form of two_f32.cuh, when the batch holds enough
+// of them to fill the GPU with its tiles (pick_pairs).  At step s = 0, 2, ..
+// of a tick they read buf[cur ^ (s / 2 & 1)] and write the other buffer; a
+// member with an odd number of steps takes the last one in the segment kernel
+// after the tick.
+//
+// Float16 members whose rows suit asynchronous bulk copies (nz * element size a
+// multiple of 16 bytes) run in a persistent kernel, the
+// batched form of the row-staged step (rows_lowp.cuh): its work items are blocks
 // of B consecutive y-rows of one member, B chosen per member so that an
 // item's 27 source runs fill one stage of a shared-memory ring; the copies
 // of later items are in flight while an item is collided, and the item's
@@ -28,12 +29,9 @@
 // Items of members whose step count for the tick is exhausted are armed
 // with no bytes and skipped, keeping the ring's phases uniform.
 //
-// Float32 members whose rows suit tensor copies step twice per launch in a
-// third kernel, the batched form of two_f32.cuh, when the batch holds enough
-// of them to fill the GPU with its tiles (pick_pairs).  At step s = 0, 2, ..
-// of a tick they read buf[cur ^ (s / 2 & 1)] and write the other buffer; a
-// member with an odd number of steps takes the last one in the cell kernel's
-// one-CTA-per-segment form after the tick.
+// The others run in the segment kernel, one CTA per 256 cells of a member's
+// flat order (k_batch_units), or, with a pinned shape, in a persistent kernel over
+// a packed cell index (k_batch).
 //
 // Launch shapes (cell kernel: threads per CTA, cells per thread, CTAs per
 // SM; row kernel: stages, stage size, CTAs per SM) follow from the members

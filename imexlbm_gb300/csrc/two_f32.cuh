@@ -4,8 +4,8 @@
 // cell, 102% of the copy bandwidth at 256^3 with the float32 pipe 30% busy.
 // Here a CTA marches along x over a (y, z) tile and keeps the state between
 // the two steps in shared memory, so memory moves one read and one write per
-// two steps.  256^3: 1048 us per two steps -> 716 (46.9 GLUPS where the copy
-// bandwidth allows 31 of one step); 128^3: 141 -> 110.  Bound now: 80% of the
+// two steps.  256^3: 1048 us per two steps -> 635 (52.8 GLUPS where the copy
+// bandwidth allows 31 of one step); 128^3: 134 -> 94.  Bound now: 85% of the
 // copy bandwidth, then the packed float32 pipe (304 two-cell operations a
 // pair of cells and step) and the latency of a plane's phases.
 //

@@ -226,8 +226,8 @@ class LBM:
 
 
 class Batch:
-    """Float32 / float16-deviation lattices advanced together by one
-    persistent launch per step (include/imexlbm.h, imex_batch_*)."""
+    """Float32 / float16-deviation lattices advanced together in a
+    few launches per step (include/imexlbm.h, imex_batch_*)."""
 
     def __init__(self, max_members: int = 256):
         self._L = _lib.load()

@@ -113,7 +113,9 @@ int imex_streaming(imex_lattice *h);
  * the state in fixed point between its kernel launches (the same numbers,
  * bit for bit); such a call returns after the run has finished on the
  * device (it reads whether every cell stayed in the exact range), except
- * while the handle's stream is being captured. */
+ * while the handle's stream is being captured.  Large float32 lattices take
+ * two steps per launch in a call of nsteps >= 3 (the same numbers), except
+ * with a pinned launch shape, with the per-phase profile on or under capture. */
 int imex_step(imex_lattice *h, int nsteps);
 
 /* Global diagnostics of the current distributions: out = {mass, px, py, pz,
@@ -301,7 +303,7 @@ const char *imex_last_error(const imex_lattice *h);
 /* ---------------------------------------------------------------- batch -- */
 
 /* Many float32 / float16-deviation lattices of any sizes, advanced together
- * by one persistent kernel launch per step over a packed cell index (no
+ * in a few kernel launches per step (no
  * counterpart in the reference, which runs one lattice per process).  The
  * batch holds handles created by imex_create; each member keeps its own
  * buffers, state, diagnostics (imex_conserved, imex_get_f ...) and
