@@ -248,9 +248,9 @@ int imex_conserved_noalloc(const double *f_dev, int nx, int ny, int nz, double *
  * arrive by asynchronous bulk copies - with ctas_per_sm resident CTAs per
  * SM; it needs nz * element size a multiple of 16 bytes and the fixed-point
  * or a reduced-precision engine.  stages < 0: back to automatic.  By
- * default the first fused step of a handle times every eligible shape on
- * the handle's own lattice (without changing its state) and keeps the
- * fastest, cached per lattice shape for the process; while the handle's
+ * default the first fused step of a handle (that steps once per launch)
+ * times every eligible shape on the handle's own lattice (without changing
+ * its state) and keeps the fastest, cached per lattice shape for the process; while the handle's
  * stream is being captured into a CUDA graph it takes the first eligible
  * shape instead.  No counterpart in the reference (Kokkos picks its own
  * tiles, src/lbm.cpp:135-139). */
