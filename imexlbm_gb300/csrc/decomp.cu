@@ -338,12 +338,12 @@ __device__ __forceinline__ void load_cell(const double* __restrict__ src, const 
 // cell lo + (i, j, k); per-axis tables of the whole lattice.
 __global__ void __launch_bounds__(kThreads) k_dom_init(double* __restrict__ f, PadGeom b, int lo0, int lo1, int lo2,
                                                       const double* __restrict__ tx, const double* __restrict__ ty,
-                                                      const double* __restrict__ tz, double rho0, double u0)
+                                                      const double* __restrict__ tz, TgParams tg)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
     if (k >= b.L[2]) return;
     double fe[kQ];
-    tg_init_cell(fe, tx, ty, tz, lo0 + i, lo1 + j, lo2 + k, rho0, u0);
+    tg_init_cell(fe, tx, ty, tz, lo0 + i, lo1 + j, lo2 + k, tg);
     const size_t c = pad_index(b, i + 1, j + 1, k + 1);
 #pragma unroll
     for (int a = 0; a < kQ; ++a) f[(size_t)a * b.plane + c] = fe[a];
@@ -824,8 +824,8 @@ int imex_domain_initialize(imex_domain* d)
     for (size_t r = 0; r < d->dev.size() && e == cudaSuccess; ++r) {
         const imex_block& b = d->blocks[r];
         k_dom_init<<<block_grid(d->dev[r]), kThreads, 0, d->stream>>>(d->dev[r].buf[0], d->dev[r].g, b.lo[0], b.lo[1], b.lo[2],
-                                                                     dt + offs[0], dt + offs[1], dt + offs[2], d->rho0,
-                                                                     d->u0);
+                                                                     dt + offs[0], dt + offs[1], dt + offs[2],
+                                                                     tg_params(d->rho0, d->u0));
         e = cudaGetLastError();
         ++d->launches;
     }

@@ -17,13 +17,13 @@ namespace imex {
 // ------------------------------------------------------------------- init --
 __global__ void __launch_bounds__(kStepBlock) k_init_f64(double* __restrict__ f, Geom g, const double* __restrict__ tx,
                                                          const double* __restrict__ ty, const double* __restrict__ tz,
-                                                         double rho0, double u0)
+                                                         TgParams tg)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, i = blockIdx.z;
     if (k >= g.nz) return;
     double fe[kQ];
-    tg_init_cell(fe, tx, ty, tz, i, j, k, rho0, u0);
+    tg_init_cell(fe, tx, ty, tz, i, j, k, tg);
     const size_t cell = ((size_t)i * g.ny + j) * g.nz + k;
 #pragma unroll
     for (int a = 0; a < kQ; ++a) f[(size_t)a * g.plane + cell] = fe[a];
@@ -133,7 +133,7 @@ size_t conserved_partials(const Geom& g)
 cudaError_t launch_init_f64(double* f, const Geom& g, const double* tx, const double* ty, const double* tz, double rho0,
                             double u0, cudaStream_t s)
 {
-    k_init_f64<<<step_grid(g), kStepBlock, 0, s>>>(f, g, tx, ty, tz, rho0, u0);
+    k_init_f64<<<step_grid(g), kStepBlock, 0, s>>>(f, g, tx, ty, tz, tg_params(rho0, u0));
     return cudaGetLastError();
 }
 

@@ -81,13 +81,13 @@ __global__ void __launch_bounds__(flat::kThreads, kFlatCtas<P, kEven, SR, kEarly
 template <int P>
 __global__ void __launch_bounds__(kStepBlock) k_init_lowp(typename Storage<P>::T* __restrict__ f, Geom g,
                                                           const double* __restrict__ tx, const double* __restrict__ ty,
-                                                          const double* __restrict__ tz, double rho0, double u0)
+                                                          const double* __restrict__ tz, TgParams tg)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, i = blockIdx.z;
     if (k >= g.nz) return;
     double fe[kQ];
-    tg_init_cell(fe, tx, ty, tz, i, j, k, rho0, u0);
+    tg_init_cell(fe, tx, ty, tz, i, j, k, tg);
     const size_t cell = ((size_t)i * g.ny + j) * g.nz + k;
 #pragma unroll
     for (int a = 0; a < kQ; ++a) f[(size_t)a * g.plane + cell] = Storage<P>::from_f64(fe[a], a);
@@ -201,9 +201,9 @@ cudaError_t launch_init_lowp(int prec, void* f, const Geom& g, const double* tx,
                              double rho0, double u0, cudaStream_t s)
 {
     if (prec == IMEX_F32)
-        k_init_lowp<IMEX_F32><<<step_grid(g), kStepBlock, 0, s>>>(static_cast<float*>(f), g, tx, ty, tz, rho0, u0);
+        k_init_lowp<IMEX_F32><<<step_grid(g), kStepBlock, 0, s>>>(static_cast<float*>(f), g, tx, ty, tz, tg_params(rho0, u0));
     else
-        k_init_lowp<IMEX_F16DEV><<<step_grid(g), kStepBlock, 0, s>>>(static_cast<__half*>(f), g, tx, ty, tz, rho0, u0);
+        k_init_lowp<IMEX_F16DEV><<<step_grid(g), kStepBlock, 0, s>>>(static_cast<__half*>(f), g, tx, ty, tz, tg_params(rho0, u0));
     return cudaGetLastError();
 }
 

@@ -11,27 +11,32 @@
 // alone: 0, +-u, +-v, +-(u + v), +-(u - v), and adding ez w = +-0 changes no
 // bit of 3p + 3 e.u.  Negation is exact, so the two members of +-e.u share
 // 3 e.u and 4.5 (e.u)^2, and one bracket serves the ez = 0 direction (its
-// weight) and the ez = +-1 pair (theirs): 74 operations, the same bits.
-// imex_initialize at 256^3: float64 8.21 -> 2.50 ms, float32 8.94 -> 2.98,
-// float16 deviations 10.65 -> 3.54 (memory alone would take 0.54 / 0.27 / 0.14).
+// weight) and the ez = +-1 pair (theirs): 70 operations, the same bits.
+// imex_initialize at 256^3: float64 8.21 -> 2.38 ms, float32 8.94 -> 2.37,
+// float16 deviations 10.65 -> 2.37 (memory alone would take 0.54 / 0.27 / 0.14).
 #pragma once
 
 #include "d3q27.cuh"
 
 namespace imex {
 
+// What does not depend on the cell, formed on the host (the same roundings;
+// 2.50 -> 2.38 ms).
+struct TgParams {
+    double u0, amp, p0;  // rho0 u0^2 / 16, rho0 / 3
+};
+inline TgParams tg_params(double rho0, double u0) { return TgParams{u0, rho0 * u0 * u0 / 16.0, rho0 * (1.0 / 3.0)}; }
+
 __device__ __forceinline__ void tg_init_cell(double (&fe)[kQ], const double* __restrict__ tx,
                                              const double* __restrict__ ty, const double* __restrict__ tz, int i,
-                                             int j, int k, double rho0, double u0)
+                                             int j, int k, const TgParams& tg)
 {
     const double sx = tx[3 * i], cx = tx[3 * i + 1], c2x = tx[3 * i + 2];
     const double sy = ty[3 * j], cy = ty[3 * j + 1], c2y = ty[3 * j + 2];
     const double cz = tz[3 * k + 1], c2z = tz[3 * k + 2];
-    const double cs2 = 1.0 / 3.0;
-    const double u = __dmul_rn(__dmul_rn(__dmul_rn(u0, sx), cy), cz);
-    const double v = __dmul_rn(__dmul_rn(__dmul_rn(-u0, cx), sy), cz);
-    const double amp = __ddiv_rn(__dmul_rn(__dmul_rn(rho0, u0), u0), 16.0);
-    const double p = __dadd_rn(__dmul_rn(rho0, cs2), __dmul_rn(__dmul_rn(amp, __dadd_rn(c2x, c2y)), __dadd_rn(c2z, 2.0)));
+    const double u = __dmul_rn(__dmul_rn(__dmul_rn(tg.u0, sx), cy), cz);
+    const double v = __dmul_rn(__dmul_rn(__dmul_rn(-tg.u0, cx), sy), cz);
+    const double p = __dadd_rn(tg.p0, __dmul_rn(__dmul_rn(tg.amp, __dadd_rn(c2x, c2y)), __dadd_rn(c2z, 2.0)));
     const double udu = __dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v));
     const double p3 = __dmul_rn(3.0, p), u15 = __dmul_rn(1.5, udu);
     // e.u by (|ex|, |ey|) and the relative sign of ex and ey: x, y, same, opposite
