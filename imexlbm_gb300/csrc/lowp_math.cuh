@@ -153,7 +153,20 @@ struct Storage<IMEX_F32> {
     static __device__ __forceinline__ float store(float h, int a) { return (float)weight(a) + h; }
     static __device__ __forceinline__ double to_f64(float v, int) { return (double)v; }
     static __device__ __forceinline__ double to_f64_exact(float v, int, bool&) { return (double)v; }
-    static __device__ __forceinline__ float from_f64(double f, int) { return __double2float_rn(f); }
+    // Rounded to nearest, ties to even, by adding just under half of the 29
+    // bits that go (one more where the bit that stays is odd): a conversion is
+    // an operation of the float64 pipe, 18 a cell beside the initialisation's
+    // 70 on it (256^3 2.86 -> 2.37 ms).  Below 2^-126, from 2^127 on, NaN: that operation.
+    static __device__ __forceinline__ float from_f64(double f, int)
+    {
+        const uint64_t b = (uint64_t)__double_as_longlong(f);
+        const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
+        if ((hi & 0x7FFFFFFFu) - 0x38100000u >= 0x47E00000u - 0x38100000u) return from_f64_wide(f);
+        const uint64_t t = b + (0x0FFFFFFFu + ((lo >> 29) & 1u));
+        // exponent 1023 to 127: 896 << 23 less, modulo 2^32
+        return __uint_as_float((((uint32_t)(t >> 29) + 0x40000000u) & 0x7FFFFFFFu) | (hi & 0x80000000u));
+    }
+    static __device__ __noinline__ float from_f64_wide(double f) { return __double2float_rn(f); }
 };
 
 template <>
