@@ -592,9 +592,10 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     // scratch: conserved partials (the native engine's: 5 doubles per
     // 128-cell row segment), 5 reduced values, fallback counter, error flag,
     // fixed-point run flag, the conserved kernel's ticket
-    // (the min/max report's chunks lie in the partials' place)
+    // (the min/max report's chunks and the initial field's tables lie in the
+    // partials' place)
     const size_t parts = std::max({conserved_partials(h->g) * 5 * sizeof(double), conserved_scratch_bytes(h->g),
-                                   minmax_scratch_bytes(h->g)});
+                                   minmax_scratch_bytes(h->g), 3 * sizeof(double) * ((size_t)nx + ny + nz)});
     const size_t scratch = parts + 5 * sizeof(double) + 4 * sizeof(unsigned long long);
     size_t need = 2 * arr + scratch;
     // Device memory comes from the device's stream-ordered pool: creating
@@ -708,9 +709,10 @@ int imex_initialize_phase(imex_lattice* h, double phx, double phy, double phz)
             host[off++] = std::cos(2.0 * xx);
         }
     }
-    double* dev = nullptr;
-    cudaError_t e = cudaMallocAsync(&dev, tot * sizeof(double), h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dev, host, tot * sizeof(double), cudaMemcpyHostToDevice, h->stream);
+    // in the conserved partials' place: an allocation whose memory the pool has
+    // given back to the driver takes 100 us
+    double* const dev = h->d_partial;
+    cudaError_t e = cudaMemcpyAsync(dev, host, tot * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess)
         e = is_lowp(h) ? launch_init_lowp(h->precision, h->buf[0], h->g, dev + offs[0], dev + offs[1], dev + offs[2], h->rho0,
                                        h->u0, h->stream)
@@ -718,9 +720,8 @@ int imex_initialize_phase(imex_lattice* h, double phx, double phy, double phz)
                                       h->stream);
     if (e == cudaSuccess) {
         ++h->launches;
-        e = cudaFreeAsync(dev, h->stream);
+        e = cudaStreamSynchronize(h->stream);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "imex_initialize");
     h->cur = 0;
     h->tag = kExact;

@@ -182,7 +182,7 @@ struct Storage<IMEX_F16DEV> {
     // float64 arithmetic they took 1.67 ms (two operations a value on a pipe
     // of 1.67 a clock and SM) and 3.66 ms per 256^3 lattice; in integers, on
     // the exact grid of fx_math.cuh, 1.09 and 1.11 (memory alone: 0.68), and
-    // the initialisation that ends in the second fell from 3.54 to 2.49.
+    // the initialisation that ends in the second fell from 3.54 to 2.37.
     // Values off the grid (f outside [2^-9, 1), |f - w| >= 1, NaN, Inf)
     // clear ok and go through float64, a cell at a time or out of line: with
     // the float64 form inline the compiler computes it for every value.
