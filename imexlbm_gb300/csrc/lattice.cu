@@ -852,6 +852,7 @@ int step_pairs(imex_lattice* h, int n, int* done)
     if (!h->pairs)
         IMEX_CUDA(h, two::make_lattice(static_cast<float*>(h->buf[0]), static_cast<float*>(h->buf[1]), h->g, &h->pairs),
                   "two-step kernel set-up");
+    if (!h->pairs->cut) two::cut_alone(h->pairs.get(), h->g);
     const bool padded = h->pairs->padded;
     *done = padded && n < 4 ? 0 : n & ~1;
     for (int s = 0; s < *done;) {

@@ -235,11 +235,17 @@ bool worth_alone(const Geom& g, int sms)
     return pair < 0.97 * singles;
 }
 
+void cut_alone(Lattice* l, const Geom& g)
+{
+    l->plan = plan_for(g, current_sm_count());
+    l->cut = true;
+}
+
 cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, LatticePtr* out)
 {
     LatticePtr l(new (std::nothrow) Lattice);
     if (!l) return cudaErrorMemoryAllocation;
-    l->plan = plan_for(g, current_sm_count());
+    l->plan = tiles_of(g);
     l->padded = !eligible(g);
     cudaError_t e = encode_maps(buf0, g, l->plan, l->padded, &l->maps[0]);
     if (e == cudaSuccess) e = encode_maps(buf1, g, l->plan, l->padded, &l->maps[1]);

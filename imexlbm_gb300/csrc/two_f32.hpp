@@ -38,10 +38,11 @@ struct Plan {
 // the row's last pair of cells.
 __host__ __device__ constexpr int pitch_of(int nz) { return (nz + 8) / 8 * 8; }
 
-// What a lattice handle keeps: its tiles, cut for the lattice alone, and the
-// maps of its two buffers (the same whatever the cut along x).
+// What a lattice handle keeps: its tiles, once it has stepped alone cut for
+// that, and the maps of its two buffers (the same whatever the cut along x).
 struct Lattice {
     Plan plan;
+    bool cut = false;
     bool padded;
     Maps maps[2];
 };
@@ -67,6 +68,9 @@ constexpr double kIterationUs = 1.65, kLaunchUs = 1.5, kCellUs = 1.0 / 31000.0;
 // side pieces, and of the one-step kernel on such rows.
 constexpr double kPaddedIterationUs = 1.85, kPaddedCellUs = 1.0 / 30000.0;
 
+// The tiles cut along x for the lattice alone (0.1 ms on the host: not for a
+// batch's members, which are cut together).
+void cut_alone(Lattice* l, const Geom& g);
 cudaError_t make_lattice(const float* buf0, const float* buf1, const Geom& g, LatticePtr* out);
 // Two fused steps of one lattice from buffer `from` into the other one.
 cudaError_t launch(const Lattice& l, int from, const float* src, float* dst, const Geom& g, const CollideF32& cp,
