@@ -548,7 +548,11 @@ int imex_test_set_fault(int kind, long long value)
 
 const char* imex_last_error(const imex_lattice* h) { return h ? h->err.c_str() : thread_error(); }
 
-int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int precision, imex_lattice** out)
+}  // extern "C"
+
+namespace imex {
+
+int lattice_create(int nx, int ny, int nz, double tau, double rho0, double u0, int precision, bool alone, imex_lattice** out)
 {
     if (!out) return set_thread_error(IMEX_ERR_ARG, "imex_create: null output pointer");
     *out = nullptr;
@@ -587,7 +591,7 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     // float32 rows that are no multiple of 4 values: room for the layout of two
     // steps per launch, where there is any and the lattice is worth it
     const size_t plain = arr;
-    if (precision == IMEX_F32 && two::padded_eligible(h->g) && two::worth_alone(h->g, current_sm_count()))
+    if (alone && precision == IMEX_F32 && two::padded_eligible(h->g) && two::worth_alone(h->g, current_sm_count()))
         arr = kQ * two::padded_plane(h->g) * sizeof(float);
     // scratch: conserved partials (the native engine's: 5 doubles per
     // 128-cell row segment), 5 reduced values, fallback counter, error flag,
@@ -658,6 +662,15 @@ int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int 
     h->bytes = need;
     *out = h;
     return IMEX_OK;
+}
+
+}  // namespace imex
+
+extern "C" {
+
+int imex_create(int nx, int ny, int nz, double tau, double rho0, double u0, int precision, imex_lattice** out)
+{
+    return imex::lattice_create(nx, ny, nz, tau, rho0, u0, precision, true, out);
 }
 
 void imex_destroy(imex_lattice* h)

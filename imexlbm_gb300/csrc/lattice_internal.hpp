@@ -73,9 +73,12 @@ struct imex_lattice {
 
 namespace imex {
 
-// Both defined in lattice.cu.
+// Defined in lattice.cu unless said.
 int lattice_fail(imex_lattice* h, int code, const std::string& msg);
 size_t lattice_elem_size(int precision);
 size_t minmax_scratch_bytes(const Geom& g);  // fields.cu
+// imex_create; alone false: a lattice that only steps in batches, with no room
+// for the padded layout (two_f32.hpp) of a lattice that steps alone.
+int lattice_create(int nx, int ny, int nz, double tau, double rho0, double u0, int precision, bool alone, imex_lattice** out);
 
 }  // namespace imex

@@ -120,7 +120,7 @@ void admit(imex_server* s, std::vector<Pending>& incoming)
     for (Pending& p : incoming) {
         Active a{p.id, p.req, nullptr, request_bytes(p.req), p.t_submit, s->now()};
         const imex_request& q = p.req;
-        int rc = imex_create(q.nx, q.ny, q.nz, q.tau, q.rho0, q.u0, q.precision, &a.h);
+        int rc = imex::lattice_create(q.nx, q.ny, q.nz, q.tau, q.rho0, q.u0, q.precision, false, &a.h);
         if (!rc && q.precision == IMEX_F16DEV) rc = imex_set_rounding(a.h, q.rounding);
         if (!rc)
             rc = q.resume_path[0] ? imex_checkpoint_load(a.h, q.resume_path)

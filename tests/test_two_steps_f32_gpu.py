@@ -125,3 +125,13 @@ def test_rows_of_any_length(imex, shape):
         got, n = run(imex, shape, steps, False, f)
         assert n == launches
         assert np.array_equal(got, want)
+
+
+def test_padded_room_is_counted(imex):
+    """The larger buffers of a lattice with odd rows are at most 7 values a row more."""
+    shape = (96, 128, 129)
+    with imex.LBM(*shape, 0.05, 1.0, 0.05, precision=imex.IMEX_F32) as lat, \
+            imex.LBM(96, 128, 128, 0.05, 1.0, 0.05, precision=imex.IMEX_F32) as even:
+        per_value = lat.device_bytes() / (2 * 27 * 4 * 96 * 128)
+        assert 129 < per_value < 129 + 8
+        assert 128 <= even.device_bytes() / (2 * 27 * 4 * 96 * 128) < 129
