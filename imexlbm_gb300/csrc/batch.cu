@@ -633,7 +633,8 @@ void pick_pairs(imex_batch* b)
     std::vector<size_t> cand;
     for (size_t m = 0; m < n; ++m) {
         const imex_lattice* h = b->members[m];
-        if (h->precision != IMEX_F32 || !two::eligible(h->g)) continue;
+        // (a captured one: pairs would leave its state in the buffer its graph does not read)
+        if (h->precision != IMEX_F32 || h->captured || !two::eligible(h->g)) continue;
         const two::Plan p = two::plan_tiles(h->g, h->g.nx);
         const double one = 2.0 * (double)h->ncells * two::kCellUs;
         if ((double)p.items() * two::item_iterations(h->g, p) * two::kIterationUs / b->sms > 0.97 * one) continue;

@@ -742,28 +742,61 @@ int imex_initialize_phase(imex_lattice* h, double phx, double phy, double phz)
     return IMEX_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+bool capturing(imex_lattice* h)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+// Notes that steps of the handle go into a graph (see step_pairs); other
+// formats flip the buffers once a step whatever they do.
+void note_capture(imex_lattice* h)
+{
+    if (h->precision == IMEX_F32 && !h->captured) h->captured = capturing(h);
+}
+
+int collide(imex_lattice* h)
+{
+    if (h->tag == kExact) return launch_mode(h, kModeCollide);
+    int rc = launch_mode(h, kModeFused);
+    if (rc) return rc;
+    h->tag = kExact;
+    return IMEX_OK;
+}
+
+int stream(imex_lattice* h)
+{
+    if (h->tag == kPendingStream) {
+        int rc = launch_mode(h, kModeStream);
+        if (rc) return rc;
+    }
+    h->tag = kPendingStream;
+    ++h->steps;
+    return IMEX_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 int imex_collision(imex_lattice* h)
 {
     int rc = check_ready(h, "imex_collision");
     if (rc) return rc;
-    if (h->tag == kExact) return launch_mode(h, kModeCollide);
-    rc = launch_mode(h, kModeFused);
-    if (rc) return rc;
-    h->tag = kExact;
-    return IMEX_OK;
+    note_capture(h);
+    return collide(h);
 }
 
 int imex_streaming(imex_lattice* h)
 {
     int rc = check_ready(h, "imex_streaming");
     if (rc) return rc;
-    if (h->tag == kPendingStream) {
-        rc = launch_mode(h, kModeStream);
-        if (rc) return rc;
-    }
-    h->tag = kPendingStream;
-    ++h->steps;
-    return IMEX_OK;
+    note_capture(h);
+    return stream(h);
 }
 
 }  // extern "C"
@@ -774,9 +807,9 @@ namespace {
 int step_each(imex_lattice* h, int nsteps)
 {
     for (int s = 0; s < nsteps; ++s) {
-        int rc = imex_collision(h);
+        int rc = collide(h);
         if (rc) return rc;
-        rc = imex_streaming(h);
+        rc = stream(h);
         if (rc) return rc;
     }
     return IMEX_OK;
@@ -857,9 +890,12 @@ bool use_pairs(imex_lattice* h)
     return h->pairs_worth != 0;
 }
 
-// Fused float32 steps, n or n - 1 of them, two per launch from the steady
+// Fused float32 steps, as many of n as go two per launch, from the steady
 // state; rows that are no multiple of 4 values: a single step into the padded
-// layout first and one out of it last.  *done: the steps taken.
+// layout first and one out of it last.  *done: the steps taken.  A graph of
+// the handle's steps reads the buffer that held the state when it was captured, and
+// an even number of single steps leaves the state there; so once there is
+// one, the steps taken flip the buffers as often, modulo 2, as there are steps.
 int step_pairs(imex_lattice* h, int n, int* done)
 {
     if (!h->pairs)
@@ -867,7 +903,8 @@ int step_pairs(imex_lattice* h, int n, int* done)
                   "two-step kernel set-up");
     if (!h->pairs->cut) two::cut_alone(h->pairs.get(), h->g);
     const bool padded = h->pairs->padded;
-    *done = padded && n < 4 ? 0 : n & ~1;
+    if (h->captured) *done = !padded ? n & ~3 : n < 6 ? 0 : ((n - 2) & ~3) + 2;
+    else *done = padded && n < 4 ? 0 : n & ~1;
     for (int s = 0; s < *done;) {
         const float* src = static_cast<const float*>(h->buf[h->cur]);
         float* dst = static_cast<float*>(h->buf[1 - h->cur]);
@@ -884,12 +921,6 @@ int step_pairs(imex_lattice* h, int n, int* done)
     return IMEX_OK;
 }
 
-bool capturing(imex_lattice* h)
-{
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
-}
-
 }  // namespace
 
 extern "C" {
@@ -899,6 +930,7 @@ int imex_step(imex_lattice* h, int nsteps)
     if (nsteps < 0) return fail(h, IMEX_ERR_ARG, "imex_step: nsteps < 0");
     int rc = check_ready(h, "imex_step");
     if (rc) return rc;
+    note_capture(h);
     if (use_fixed(h) && nsteps >= 3) {
         // reach the steady state (buffer pending a streaming) and the
         // launch shape, then run the rest as one fixed-point run when the

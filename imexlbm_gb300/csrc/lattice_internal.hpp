@@ -66,6 +66,7 @@ struct imex_lattice {
     bool shape_pinned = false;  // shape set by imex_set_launch rather than the autotuner
     imex::two::LatticePtr pairs;  // two float32 steps per launch (two_f32.hpp), made on first use
     int pairs_worth = -1;         // whether they pay for this lattice alone (-1: not asked yet)
+    bool captured = false;        // float32: steps of this handle were captured into a graph
     bool padded_room = false;     // the buffers hold the padded layout too (two_f32.hpp)
     imex::PhaseTimer prof;      // per-phase device time (imex_profile_*)
     std::string err;

@@ -115,7 +115,10 @@ int imex_streaming(imex_lattice *h);
  * device (it reads whether every cell stayed in the exact range), except
  * while the handle's stream is being captured.  Large float32 lattices take
  * two steps per launch in a call of nsteps >= 3 (the same numbers), except
- * with a pinned launch shape, with the per-phase profile on or under capture. */
+ * with a pinned launch shape, with the per-phase profile on or under capture.
+ * A captured run reads and writes the buffers as they were when it was
+ * captured: an even number of steps returns the state to the buffer it was
+ * in, and so does every even number of eager steps between two replays. */
 int imex_step(imex_lattice *h, int nsteps);
 
 /* Global diagnostics of the current distributions: out = {mass, px, py, pz,
