@@ -78,9 +78,11 @@ __global__ void __launch_bounds__(kThreads) k_velocity_diff(const typename mom::
         if (oka && okb) {
 #pragma unroll
             for (int d = 1; d < 4; ++d) {
-                const long long x = ca.M[d] - cb.M[d], y = cb.M[d];
-                take(0, (unsigned long long)(x < 0 ? -x : x));
-                take(1, (unsigned long long)(y < 0 ? -y : y));
+                // a component is below 2.25 (18 values below 1/8), so a difference can pass
+                // the 4 at which the signed form ends
+                const int64_t x = ca.M[d], y = cb.M[d];
+                take(0, x < y ? (uint64_t)y - (uint64_t)x : (uint64_t)x - (uint64_t)y);
+                take(1, (uint64_t)(y < 0 ? -y : y));
             }
         } else {
             double ma[4], mb[4];

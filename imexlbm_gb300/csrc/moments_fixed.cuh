@@ -12,8 +12,11 @@
 //                     multiples of 2^-37 or more for stored values of the
 //                     weights' size, so their conversion drops nothing.
 //
-// Outside the range (|u| >= 1, 3p outside (0, 2), a float64 value not in
-// [2^-9, 1), NaN, Inf) `ok` is false and the caller uses moments_f64_of.
+// Outside the range `ok` is false and the caller uses moments_f64_of.  In the
+// range are: float64 values in [2^-9, 1) for f_0 and [2^-9, 1/8) for the others
+// with 3p < 2; float32 sums below 1 in magnitude (sum h, and each of sum h e);
+// EXACT, stored values (or deviations, in units of f) below 1/2 and 1/8 in
+// magnitude, whose sums may reach 3.75 (3p) and 2.25 (u, v, w).
 #pragma once
 
 #include "fx_math.cuh"
