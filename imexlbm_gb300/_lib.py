@@ -34,6 +34,7 @@ IMEX_ENGINE_FIXED = 2
 IMEX_TEST_FAULT_NONE = 0
 IMEX_TEST_FAULT_STARVE_STAGE = 1
 IMEX_TEST_FAULT_BATCH_TABLE = 2
+IMEX_TEST_FAULT_BATCH_UPLOAD = 3
 
 # Every symbol include/imexlbm.h declares, with (restype, argtypes).
 _dp = ctypes.POINTER(ctypes.c_double)

@@ -425,7 +425,7 @@ struct imex_batch {
     Table<PairHeader> phdr;
     Table<PairEntry> ptab;
     Table<two::Maps> pmaps;
-    size_t pmaps_up = 0;             // maps of pmaps.h the device holds
+    size_t pmaps_up = 0;             // maps of pmaps.h the device holds (0: none is known to)
     Table<int> pgroup;
     Table<BatchHeader> thdr;         // the members' odd last step, in the cell kernel
     Table<BatchEntry> ttab;
@@ -686,7 +686,10 @@ int upload_pairs(imex_batch* b, const std::vector<int>& steps)
     }
     if (items > 0x7fffffffu || units > 0x7fffffffu)
         return bfail(b, IMEX_ERR_ARG, "imex_batch_step: too many work items for one launch");
-    const void* maps_at = b->pmaps.d;
+    // Until this tick's maps are on their way the staging no longer tells what
+    // the device holds: a return in between leaves none known.
+    const size_t maps_up = b->pmaps.cap >= 2 * n ? b->pmaps_up : 0;  // a larger table is a new one
+    b->pmaps_up = 0;
     const size_t pgroups = (items + kPairGroup - 1) / kPairGroup, tgroups = (units + kUnitGroup - 1) / kUnitGroup;
     cudaError_t e = b->phdr.reserve(1, b->stream);
     if (e == cudaSuccess) e = b->ptab.reserve(n, b->stream);
@@ -696,10 +699,9 @@ int upload_pairs(imex_batch* b, const std::vector<int>& steps)
     if (e == cudaSuccess) e = b->ttab.reserve(n, b->stream);
     if (e == cudaSuccess) e = b->tgroup.reserve(tgroups, b->stream);
     if (e != cudaSuccess) return bcuda(b, e, "batch tables");
-    if (b->pmaps.d != maps_at) b->pmaps_up = 0;
     size_t begin = 0, ubegin = 0;
     int tails = 0;
-    bool new_maps = b->pmaps_up < 2 * n;
+    bool new_maps = maps_up < 2 * n;
     for (size_t q = 0; q < n; ++q) {
         imex_lattice* h = b->members[order[q]];
         if (!h->pairs)
@@ -749,7 +751,7 @@ int upload_pairs(imex_batch* b, const std::vector<int>& steps)
     *b->thdr.h = BatchHeader{ubegin, tails, 0};
     b->pair_items = (unsigned)begin;
     b->tail_units = (unsigned)ubegin;
-    e = b->phdr.upload(1, b->stream);
+    e = test_fault_kind() == IMEX_TEST_FAULT_BATCH_UPLOAD ? cudaErrorUnknown : b->phdr.upload(1, b->stream);
     if (e == cudaSuccess) e = b->ptab.upload(n, b->stream);
     if (e == cudaSuccess && new_maps) e = b->pmaps.upload(2 * n, b->stream);
     if (e == cudaSuccess) e = b->pgroup.upload(pgroups, b->stream);
@@ -757,7 +759,7 @@ int upload_pairs(imex_batch* b, const std::vector<int>& steps)
     if (e == cudaSuccess && tails) e = b->ttab.upload(tails, b->stream);
     if (e == cudaSuccess && tails) e = b->tgroup.upload(tgroups, b->stream);
     if (e != cudaSuccess) return bcuda(b, e, "batch tables");
-    b->pmaps_up = std::max(b->pmaps_up, 2 * n);
+    b->pmaps_up = std::max(maps_up, 2 * n);
     return IMEX_OK;
 }
 
@@ -1107,7 +1109,10 @@ int imex_batch_step(imex_batch* b, int nsteps)
         for (size_t m = 0; m < left.size(); ++m) tick[m] = (int)std::min<int64_t>(left[m], k);
         rc = upload_pairs(b, tick);
         if (!rc) rc = upload_table(b, tick, b->rshape, b->shape);
-        if (rc) return rc;
+        if (rc) {  // copies already queued read the staging, which the next call writes
+            cudaStreamSynchronize(b->stream);
+            return rc;
+        }
         if (b->graph_steps > 0 && k == b->graph_steps) {
             if (!graph_valid(b, k)) {
                 rc = capture_graph(b, k);

@@ -539,7 +539,7 @@ int imex_test_set_fault(int kind, long long value)
     }
     if (kind == IMEX_TEST_FAULT_STARVE_STAGE && (value < 1000 || value > bulk::kWaitCycles))
         return set_thread_error(IMEX_ERR_ARG, "imex_test_set_fault: the wait limit must be in [1000, 2^31] SM clocks");
-    if (kind != IMEX_TEST_FAULT_STARVE_STAGE && kind != IMEX_TEST_FAULT_BATCH_TABLE)
+    if (kind != IMEX_TEST_FAULT_STARVE_STAGE && kind != IMEX_TEST_FAULT_BATCH_TABLE && kind != IMEX_TEST_FAULT_BATCH_UPLOAD)
         return set_thread_error(IMEX_ERR_ARG, "imex_test_set_fault: unknown fault");
     g_fault_value.store(value);
     g_fault_kind.store(kind);

@@ -547,10 +547,14 @@ const char *imex_version(void);
  *   IMEX_TEST_FAULT_BATCH_TABLE   the batch row kernel is launched with a
  *       member-table capacity one below its member count, so it refuses the
  *       table; imex_batch_synchronize returns IMEX_ERR_CUDA.
+ *   IMEX_TEST_FAULT_BATCH_UPLOAD  imex_batch_step returns IMEX_ERR_CUDA once
+ *       it has laid out the tables of the members that step twice per launch,
+ *       before it uploads them; nothing is launched.
  * The results of the steps run under a fault are invalid. */
 #define IMEX_TEST_FAULT_NONE 0
 #define IMEX_TEST_FAULT_STARVE_STAGE 1
 #define IMEX_TEST_FAULT_BATCH_TABLE 2
+#define IMEX_TEST_FAULT_BATCH_UPLOAD 3
 int imex_test_set_fault(int kind, long long value);
 
 #ifdef __cplusplus
