@@ -113,7 +113,7 @@ __device__ __noinline__ void add_outside(const typename mom::Elem<P>::T* src, Ge
 
 template <int P, bool PULL, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB)
-    k_conserved(const typename mom::Elem<P>::T* __restrict__ src, Geom g, unsigned cells, Partial* __restrict__ part,
+    k_conserved(const typename mom::Elem<P>::T* src, Geom g, unsigned cells, Partial* __restrict__ part,
                 unsigned* __restrict__ ticket, const unsigned long long* __restrict__ status, double* __restrict__ out)
 {
     __shared__ BlockSum s;

@@ -49,7 +49,7 @@ __device__ __forceinline__ unsigned first_cell(unsigned block, unsigned t)
 // beyond the last cell) of a lattice of fewer than 2^32 cells; kEven: of an even
 // number of them.  Ends its kernel's chain (chain_end).
 template <int P, bool kEven, bool kEarly>
-__device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __restrict__ src,
+__device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* src,
                                           typename lowp::Storage<P>::T* __restrict__ dst, int nx, int ny, int nz,
                                           size_t plane, unsigned c, const CollideF32& cp)
 {
@@ -63,7 +63,7 @@ __device__ __forceinline__ void step_pair(const typename lowp::Storage<P>::T* __
 #pragma unroll
     for (int a = 0; a < kQ; ++a) {
         const T* p = src + (size_t)a * plane;
-        const T v0 = __ldg(p + p0.at(a)), v1 = __ldg(p + p1.at(a));
+        const T v0 = load_state(p + p0.at(a)), v1 = load_state(p + p1.at(a));
         h[a] = make_float2(S::dev(v0, a), S::dev(v1, a));
     }
     lowp::collide_dev<P, A>(h, cp);

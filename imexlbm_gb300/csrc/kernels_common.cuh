@@ -42,7 +42,9 @@ inline int current_sm_count()
 // Every thread of such a kernel calls chain_begin before its first access to
 // memory and before any return: it waits until the kernels before have
 // completed and their stores are visible (a kernel that completed without
-// waiting would let the one after it overtake the one before).  chain_end
+// waiting would let the one after it overtake the one before).  The kernel
+// exists while the one before still writes, so what it reads of a lattice it
+// reads by load_state, tensor or bulk copies.  chain_end
 // comes once its sources are read.  Where the CTAs take turns on the SMs
 // (early) the next kernel is let in at the beginning: its CTAs come up as
 // these finish.  Where all CTAs run at once it is let in at the end: let in
@@ -81,6 +83,15 @@ template <bool EARLY>
 __device__ __forceinline__ void chain_end()
 {
     if (!EARLY) chain_next();
+}
+
+// Load of lattice state.  An ordinary cached load: the read-only path (__ldg, and what the
+// compiler may take for a const __restrict__ pointer) is for memory that nothing
+// writes as long as the kernel exists, which does not hold for a chained one.
+template <class T>
+__device__ __forceinline__ T load_state(const T* p)
+{
+    return __ldca(p);
 }
 
 // Source indices of the pull for cell (i, j, k): the value streaming into
@@ -149,18 +160,12 @@ struct FlatPull {
     __device__ __forceinline__ unsigned at(int a) const { return x[ex(a, 0) + 1] + y[ex(a, 1) + 1] + z[ex(a, 2) + 1]; }
 };
 
-template <int A, typename T>
-__device__ __forceinline__ T ldg_pull(const T* __restrict__ src, const Geom& g, const PullIndex& p)
-{
-    return __ldg(src + p.at<A>(g));
-}
-
 // Unrolled gather of the 27 pulled (or in-place) values.
 template <typename T, int A = 0>
-__device__ __forceinline__ void gather27(const T* __restrict__ src, const Geom& g, const PullIndex& p, T (&f)[kQ])
+__device__ __forceinline__ void gather27(const T* src, const Geom& g, const PullIndex& p, T (&f)[kQ])
 {
     if constexpr (A < kQ) {
-        f[A] = ldg_pull<A>(src, g, p);
+        f[A] = load_state(src + p.at<A>(g));
         gather27<T, A + 1>(src, g, p, f);
     }
 }

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kStepBlock, 5) k_collide_fx(double* __restrict
 // of a place in the CTA's row segment.
 template <bool OM_GE1, bool IN_FX, bool OUT_FX, bool FLAT, bool EARLY>
 __global__ void __launch_bounds__(kStepBlock, 5)
-    k_step_fxs(const unsigned long long* __restrict__ src, unsigned long long* __restrict__ dst, Geom g, FxConst c,
+    k_step_fxs(const unsigned long long* src, unsigned long long* __restrict__ dst, Geom g, FxConst c,
                int j, int* __restrict__ fail)
 {
     chain_begin<EARLY>();
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kStepBlock, 5)
         if (q >= (unsigned)g.plane) return;
         const FlatPull pi(g.nx, g.ny, g.nz, q);
 #pragma unroll
-        for (int a = 0; a < kQ; ++a) in[a] = __ldg(src + (size_t)a * g.plane + pi.at(a));
+        for (int a = 0; a < kQ; ++a) in[a] = load_state(src + (size_t)a * g.plane + pi.at(a));
         cell = q;
     } else {
         const int k = blockIdx.x * blockDim.x + threadIdx.x;

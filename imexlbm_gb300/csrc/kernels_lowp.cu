@@ -65,7 +65,7 @@ inline constexpr int kFlatCtas = P == IMEX_F16DEV && !SR                      ? 
                                  : !kEarly && (P == IMEX_F16DEV || !kEven) ? 1
                                                                               : 0;
 template <int P, bool kEven, bool SR, bool kEarly>
-__global__ void __launch_bounds__(flat::kThreads, kFlatCtas<P, kEven, SR, kEarly>) k_flat_lowp(const typename Storage<P>::T* __restrict__ src,
+__global__ void __launch_bounds__(flat::kThreads, kFlatCtas<P, kEven, SR, kEarly>) k_flat_lowp(const typename Storage<P>::T* src,
                                                               typename Storage<P>::T* __restrict__ dst, Geom g,
                                                               CollideF32 cp)
 {

@@ -98,7 +98,7 @@ __device__ __forceinline__ unsigned long long block_largest(unsigned long long (
 }
 
 template <int P, bool PULL>
-__global__ void __launch_bounds__(kThreads) k_extremes(const typename mom::Elem<P>::T* __restrict__ src, Geom g, Split s,
+__global__ void __launch_bounds__(kThreads) k_extremes(const typename mom::Elem<P>::T* src, Geom g, Split s,
                                                        Chunk* __restrict__ chunks, Result* __restrict__ res)
 {
     __shared__ unsigned long long red[kThreads / 32][8];
@@ -134,8 +134,9 @@ __global__ void __launch_bounds__(kThreads) k_extremes(const typename mom::Elem<
 template <int P>
 __device__ __forceinline__ double value_of(const typename mom::Elem<P>::T* src, const Geom& g, const PullIndex& pi, int a)
 {
-    if constexpr (P == IMEX_F64) return __ldg(src + pi.at_dyn(g, a));
-    else return lowp::Storage<P>::to_f64(src[pi.at_dyn(g, a)], a);
+    const auto v = load_state(src + pi.at_dyn(g, a));
+    if constexpr (P == IMEX_F64) return v;
+    else return lowp::Storage<P>::to_f64(v, a);
 }
 
 // The float64 sums of a cell in the reference's order: x[0] = 3p, x[1..3] = u, v, w.
@@ -189,13 +190,13 @@ __device__ __noinline__ bool sums_exact(const typename mom::Elem<P>::T* src, con
     else {
         float least = 1.f;
 #pragma unroll
-        for (int a = 0; a < kQ; ++a) least = fminf(least, fabsf(src[pi.at_dyn(g, a)]));
+        for (int a = 0; a < kQ; ++a) least = fminf(least, fabsf(load_state(src + pi.at_dyn(g, a))));
         return least >= 0x1p-27f;
     }
 }
 
 template <int P, bool PULL>
-__global__ void __launch_bounds__(kThreads) k_pick(const typename mom::Elem<P>::T* __restrict__ src, Geom g, Split s,
+__global__ void __launch_bounds__(kThreads) k_pick(const typename mom::Elem<P>::T* src, Geom g, Split s,
                                                    const Chunk* __restrict__ chunks, Result* __restrict__ res)
 {
     __shared__ unsigned long long red[kThreads / 32][8];

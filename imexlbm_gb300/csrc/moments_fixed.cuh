@@ -68,7 +68,7 @@ inline constexpr int kVelBits = P == IMEX_F64 ? kBits : P == IMEX_F16DEV ? 12 : 
 // EXACT (reduced precision): the stored values summed exactly instead of in
 // float32; the velocities in units of 2^-61.
 template <int P, bool EXACT>
-__device__ __forceinline__ bool moments(const typename Elem<P>::T* __restrict__ src, const Geom& g, const PullIndex& pi,
+__device__ __forceinline__ bool moments(const typename Elem<P>::T* src, const Geom& g, const PullIndex& pi,
                                         Cell<P>& c)
 {
     bool ok = true;
@@ -98,7 +98,7 @@ __device__ __forceinline__ bool moments(const typename Elem<P>::T* __restrict__ 
         int64_t S = 0, U[3] = {0, 0, 0};
 #pragma unroll
         for (int a = 0; a < kQ; ++a) {
-            const auto v = __ldg(src + pi.at_dyn(g, a));
+            const auto v = load_state(src + pi.at_dyn(g, a));
             constexpr int S2 = P == IMEX_F32 ? 0 : Elem<P>::kScaleLog2;
             float x;
             if constexpr (P == IMEX_F32) x = v;
@@ -130,7 +130,7 @@ __device__ __forceinline__ bool moments(const typename Elem<P>::T* __restrict__ 
         constexpr int S = Elem<P>::kScaleLog2;
         float h[kQ];
 #pragma unroll
-        for (int a = 0; a < kQ; ++a) h[a] = lowp::Storage<P>::dev(src[pi.at_dyn(g, a)], a);
+        for (int a = 0; a < kQ; ++a) h[a] = lowp::Storage<P>::dev(load_state(src + pi.at_dyn(g, a)), a);
         float d[kPairs + 1], sig = h[0];
 #pragma unroll
         for (int q = 1; q <= kPairs; ++q) {
@@ -164,8 +164,9 @@ __device__ __noinline__ void moments_f64_of(const typename Elem<P>::T* src, Geom
 #pragma unroll
     for (int a = 0; a < kQ; ++a) {
         double f;
-        if constexpr (P == IMEX_F64) f = src[pi.at_dyn(g, a)];
-        else f = lowp::Storage<P>::to_f64(src[pi.at_dyn(g, a)], a);
+        const auto v = load_state(src + pi.at_dyn(g, a));
+        if constexpr (P == IMEX_F64) f = v;
+        else f = lowp::Storage<P>::to_f64(v, a);
         out[0] += f;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {

@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // separate pairs: neither layout's rows are 8-byte aligned in every direction).
 constexpr int kEdgeThreads = 128;
 template <bool kOut>
-__global__ void __launch_bounds__(kEdgeThreads) k_edge_f32(const float* __restrict__ src, float* __restrict__ dst, Geom g,
+__global__ void __launch_bounds__(kEdgeThreads) k_edge_f32(const float* src, float* __restrict__ dst, Geom g,
                                                            CollideF32 cp)
 {
     using S = lowp::Storage<IMEX_F32>;
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_f32(const float* __restri
 #pragma unroll
     for (int a = 0; a < kQ; ++a) {
         const float* p = src + (size_t)a * from;
-        h[a] = make_float2(S::dev(__ldg(p + p0.at(a)), a), S::dev(__ldg(p + p1.at(a)), a));
+        h[a] = make_float2(S::dev(load_state(p + p0.at(a)), a), S::dev(load_state(p + p1.at(a)), a));
     }
     lowp::collide_dev<IMEX_F32, A>(h, cp);
     if (kOut) {
