@@ -288,49 +288,43 @@ int check_kernel_error(imex_lattice* h);
 // slot of one page of pinned memory, which the host reads after the synchronisation
 // it makes anyway; a copy into pageable memory costs another 4 to 8 us (a report
 // of a 32^3 float64 lattice, 10 steps and the sums, 98 us so, 87 with the slot).  A slot is held for a call and
-// free again after it; without one (64 calls at once, no page) the call
-// copies.  The page is made by the first imex_create and kept; it is gone
-// after a cudaDeviceReset, which each use finds out, and made anew by the next
-// imex_create.
+// free again after it; without one (64 calls at once, page not pinned) the call
+// copies.  The page is storage of this library, so that its address is never another
+// allocation's; imex_create has it pinned.  A cudaDeviceReset undoes that, which each use
+// finds out, and the next imex_create pins it again.
 constexpr size_t kSlotBytes = 64;
 constexpr int kSlots = 64;
 std::mutex g_page_lock;
-std::atomic<unsigned char*> g_page{nullptr};
+alignas(4096) unsigned char g_page[kSlots * kSlotBytes];
 std::atomic<unsigned long long> g_slots_used{0};
 
-// The page's address on the device, or nullptr if it is no pinned memory (any more).
-unsigned char* page_device(unsigned char* page)
+// The page's address on the device, or nullptr if it is not pinned (any more).
+unsigned char* page_device()
 {
     cudaPointerAttributes at{};
-    if (!page) return nullptr;
-    if (cudaPointerGetAttributes(&at, page) != cudaSuccess) {
+    if (cudaPointerGetAttributes(&at, g_page) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
     return at.type == cudaMemoryTypeHost ? static_cast<unsigned char*>(at.devicePointer) : nullptr;
 }
 
-void make_report_page()
+void pin_report_page()
 {
     std::lock_guard<std::mutex> guard(g_page_lock);
-    if (page_device(g_page.load())) return;
+    if (page_device()) return;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // no concern of another thread's capture
     cudaThreadExchangeStreamCaptureMode(&mode);
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, kSlots * kSlotBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    if (cudaHostRegister(g_page, sizeof g_page, cudaHostRegisterPortable | cudaHostRegisterMapped) != cudaSuccess)
         cudaGetLastError();
-        p = nullptr;
-    }
     cudaThreadExchangeStreamCaptureMode(&mode);
-    g_page.store(static_cast<unsigned char*>(p));
 }
 
 class ReportSlot {
 public:
     explicit ReportSlot(bool want = true)
     {
-        unsigned char* const page = want ? g_page.load() : nullptr;
-        unsigned char* const dev = page_device(page);
+        unsigned char* const dev = want ? page_device() : nullptr;
         if (!dev) return;
         unsigned long long used = g_slots_used.load();
         do {
@@ -338,7 +332,7 @@ public:
             while (index_ < kSlots && (used >> index_ & 1)) ++index_;
             if (index_ == kSlots) return;
         } while (!g_slots_used.compare_exchange_weak(used, used | 1ull << index_));
-        host_ = page + index_ * kSlotBytes;
+        host_ = g_page + index_ * kSlotBytes;
         dev_ = dev + index_ * kSlotBytes;
     }
     ~ReportSlot()
@@ -655,7 +649,7 @@ int lattice_create(int nx, int ny, int nz, double tau, double rho0, double u0, i
     h->d_err = reinterpret_cast<unsigned*>(h->d_fallback + 1);
     h->d_fail = reinterpret_cast<int*>(h->d_fallback + 2);
     h->d_ticket = reinterpret_cast<unsigned*>(h->d_fallback + 3);
-    make_report_page();
+    pin_report_page();
     e = cudaMemsetAsync(h->d_fallback, 0, 4 * sizeof(unsigned long long), h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);  // usable from any stream from here on
     if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "imex_create"));
