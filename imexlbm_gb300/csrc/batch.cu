@@ -1155,8 +1155,8 @@ int imex_batch_synchronize(imex_batch* b)
 int imex_batch_set_launch(imex_batch* b, int threads, int cells_per_thread, int ctas_per_sm)
 {
     if (!b) return set_thread_error(IMEX_ERR_ARG, "imex_batch_set_launch: null batch");
-    b->cells_pinned = threads != 0;
     if (threads == 0) {
+        b->cells_pinned = false;
         b->shape = BatchShape{};
         return IMEX_OK;
     }
@@ -1164,6 +1164,7 @@ int imex_batch_set_launch(imex_batch* b, int threads, int cells_per_thread, int 
         if (threads != kUnitThreads)
             return bfail(b, IMEX_ERR_ARG, "imex_batch_set_launch: cells_per_thread 0 (one CTA per segment) "
                                           "takes 128 threads");
+        b->cells_pinned = true;
         b->shape = BatchShape{kUnitThreads, 0, 0};
         return IMEX_OK;
     }
@@ -1171,6 +1172,7 @@ int imex_batch_set_launch(imex_batch* b, int threads, int cells_per_thread, int 
         ctas_per_sm < 1 || ctas_per_sm * threads > 2048)
         return bfail(b, IMEX_ERR_ARG, "imex_batch_set_launch: threads 128|256, cells_per_thread 0|1|2|4, "
                                       "ctas_per_sm*threads <= 2048");
+    b->cells_pinned = true;
     b->shape.threads = threads;
     b->shape.cpt = cells_per_thread;
     b->shape.ctas_per_sm = ctas_per_sm;
@@ -1189,8 +1191,8 @@ int imex_batch_get_launch(imex_batch* b, int out[3])
 int imex_batch_set_row_launch(imex_batch* b, int stages, int dir_kb, int ctas_per_sm, int float32_members)
 {
     if (!b) return set_thread_error(IMEX_ERR_ARG, "imex_batch_set_row_launch: null batch");
-    b->rows_pinned = stages != 0;
     if (stages == 0 || stages == -1) {  // 0: by rule, -1: row kernel off
+        b->rows_pinned = stages != 0;
         b->rshape = RowShape{stages, 0, 0, 1};
         return IMEX_OK;
     }
@@ -1199,6 +1201,7 @@ int imex_batch_set_row_launch(imex_batch* b, int stages, int dir_kb, int ctas_pe
         ctas_per_sm > 4 || !rows_fit(rs, b->capacity))
         return bfail(b, IMEX_ERR_ARG, "imex_batch_set_row_launch: 2 <= stages <= 8, dir_kb 1, 2 or 4, 1 <= "
                                       "ctas_per_sm <= 4, and the CTAs' rings must fit an SM's shared memory");
+    b->rows_pinned = true;
     b->rshape = rs;
     return IMEX_OK;
 }
