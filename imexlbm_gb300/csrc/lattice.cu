@@ -354,6 +354,28 @@ private:
 
 bool capturing(imex_lattice* h);
 
+// Float32 lattices of odd rows get buffers with room for the padded layout
+// (two_f32.hpp) when they are created, since later it costs two allocations and a copy (a first run
+// of 20 steps at 121 x 150 x 97 1.19 ms, 1.89 so); but only while at most
+// kIdleRoomMost of it lies unused in the process, because a lattice that steps in
+// batches never uses it (7% of it at nz = 97).  Beyond that a lattice gets it at its first run.
+constexpr size_t kIdleRoomMost = (size_t)1 << 30;
+std::atomic<size_t> g_idle_room{0};
+
+bool claim_idle_room(size_t bytes)
+{
+    if (g_idle_room.fetch_add(bytes) + bytes <= kIdleRoomMost) return true;
+    g_idle_room.fetch_sub(bytes);
+    return false;
+}
+
+// The handle's room is in use, or gone.
+void release_idle_room(imex_lattice* h)
+{
+    g_idle_room.fetch_sub(h->idle_room);
+    h->idle_room = 0;
+}
+
 // Resources of the two-steps-per-launch kernel (per handle, grown to the
 // deepest ring a launch shape asks for): the ticket counter, 2 nx ny row
 // flags (zero: no epoch yet) and the ring of `ring` + 2 x-planes.
@@ -582,11 +604,14 @@ int lattice_create(int nx, int ny, int nz, double tau, double rho0, double u0, i
     if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaGetDevice"));
 
     size_t arr = (size_t)kQ * h->ncells * elem_size(precision);
-    // float32 rows that are no multiple of 4 values: room for the layout of two
-    // steps per launch, where there is any and the lattice is worth it
     const size_t plain = arr;
-    if (alone && precision == IMEX_F32 && two::padded_eligible(h->g) && two::worth_alone(h->g, current_sm_count()))
-        arr = kQ * two::padded_plane(h->g) * sizeof(float);
+    if (alone && precision == IMEX_F32 && two::padded_eligible(h->g) && two::worth_alone(h->g, current_sm_count())) {
+        const size_t padded = kQ * two::padded_plane(h->g) * sizeof(float);
+        if (claim_idle_room(2 * (padded - plain))) {
+            h->idle_room = 2 * (padded - plain);
+            arr = padded;
+        }
+    }
     // scratch: conserved partials (the native engine's: 5 doubles per
     // 128-cell row segment), 5 reduced values, fallback counter, error flag,
     // fixed-point run flag, the conserved kernel's ticket
@@ -609,10 +634,12 @@ int lattice_create(int nx, int ny, int nz, double tau, double rho0, double u0, i
     cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
     cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
     const size_t avail = free_b + (reserved > used ? (size_t)(reserved - used) : 0);
-    if (need > avail && arr > plain) {
+    auto no_room = [&] {
+        need -= h->idle_room;
         arr = plain;
-        need = 2 * arr + scratch;
-    }
+        release_idle_room(h);
+    };
+    if (need > avail && arr > plain) no_room();
     if (need > avail) {
         char msg[160];
         std::snprintf(msg, sizeof msg, "imex_create: needs %.3f GB of device memory, %.3f GB free", need / 1e9,
@@ -622,20 +649,16 @@ int lattice_create(int nx, int ny, int nz, double tau, double rho0, double u0, i
     e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(nullptr, e, "cudaStreamCreate"));
     h->stream = h->own_stream;
-    h->padded_room = arr > plain;
-    auto buffers = [&](size_t bytes) {
-        for (int b = 0; b < 2 && e == cudaSuccess; ++b) e = cudaMallocAsync(&h->buf[b], bytes, h->stream);
-    };
-    buffers(arr);
-    if (e != cudaSuccess && h->padded_room) {
+    for (int tries = arr > plain ? 2 : 1; tries > 0; --tries) {
+        for (int b = 0; b < 2 && e == cudaSuccess; ++b) e = cudaMallocAsync(&h->buf[b], arr, h->stream);
+        if (e == cudaSuccess || tries == 1) break;
         cudaGetLastError();
         if (h->buf[0]) cudaFreeAsync(h->buf[0], h->stream);
         h->buf[0] = h->buf[1] = nullptr;
-        h->padded_room = false;
-        need -= 2 * (arr - plain);
+        no_room();
         e = cudaSuccess;
-        buffers(plain);
     }
+    h->padded_room = arr > plain;
     unsigned char* s = nullptr;
     if (e == cudaSuccess) e = cudaMallocAsync((void**)&s, scratch, h->stream);
     if (e != cudaSuccess) {
@@ -687,6 +710,7 @@ void imex_destroy(imex_lattice* h)
         if (h->two_mem) cudaFreeAsync(h->two_mem, h->own_stream);
         cudaStreamDestroy(h->own_stream);
     }
+    release_idle_room(h);
     delete h;
 }
 
@@ -880,8 +904,34 @@ bool use_pairs(imex_lattice* h)
 {
     if (h->precision != IMEX_F32 || h->shape_pinned || h->prof.enabled()) return false;
     if (h->pairs_worth < 0)
-        h->pairs_worth = (two::eligible(h->g) || h->padded_room) && two::worth_alone(h->g, current_sm_count());
+        h->pairs_worth = two::worth_alone(h->g, current_sm_count());
     return h->pairs_worth != 0;
+}
+
+// Buffers with room for the padded layout, for a lattice that has none and takes two
+// steps per launch in it: one after the other, so that no more than three
+// exist at once.  A lattice whose steps are captured keeps the buffers its graph reads, one
+// that finds no memory those it has: both go on by single steps.
+int make_padded_room(imex_lattice* h)
+{
+    const size_t plain = kQ * h->ncells * sizeof(float), padded = kQ * two::padded_plane(h->g) * sizeof(float);
+    h->pairs_worth = 0;  // until it is done
+    if (h->captured) return IMEX_OK;
+    for (const int b : {1 - h->cur, h->cur}) {
+        void* p = nullptr;
+        if (cudaMallocAsync(&p, padded, h->stream) != cudaSuccess) {
+            cudaGetLastError();
+            return IMEX_OK;
+        }
+        cudaError_t e = b == h->cur ? cudaMemcpyAsync(p, h->buf[b], plain, cudaMemcpyDeviceToDevice, h->stream) : cudaSuccess;
+        std::swap(p, h->buf[b]);
+        h->bytes += padded - plain;
+        if (e == cudaSuccess) e = cudaFreeAsync(p, h->stream);
+        IMEX_CUDA(h, e, "buffers of the padded layout");
+    }
+    h->padded_room = true;
+    h->pairs_worth = 1;
+    return IMEX_OK;
 }
 
 // Fused float32 steps, as many of n as go two per launch, from the steady
@@ -892,13 +942,22 @@ bool use_pairs(imex_lattice* h)
 // one, the steps taken flip the buffers as often, modulo 2, as there are steps.
 int step_pairs(imex_lattice* h, int n, int* done)
 {
+    *done = 0;
+    if (!two::eligible(h->g)) {
+        if (n < 4) return IMEX_OK;
+        if (!h->padded_room) {
+            int rc = make_padded_room(h);
+            if (rc || !h->padded_room) return rc;
+        }
+        release_idle_room(h);
+    }
     if (!h->pairs)
         IMEX_CUDA(h, two::make_lattice(static_cast<float*>(h->buf[0]), static_cast<float*>(h->buf[1]), h->g, &h->pairs),
                   "two-step kernel set-up");
     if (!h->pairs->cut) two::cut_alone(h->pairs.get(), h->g);
     const bool padded = h->pairs->padded;
     if (h->captured) *done = !padded ? n & ~3 : n < 6 ? 0 : ((n - 2) & ~3) + 2;
-    else *done = padded && n < 4 ? 0 : n & ~1;
+    else *done = n & ~1;
     for (int s = 0; s < *done;) {
         const float* src = static_cast<const float*>(h->buf[h->cur]);
         float* dst = static_cast<float*>(h->buf[1 - h->cur]);

@@ -48,14 +48,14 @@ def captured(lat, steps, way):
 @pytest.mark.parametrize("way", ["step", "calls"])
 def test_eager_steps_between_replays(imex, shape, eager, way):
     with make(imex, shape) as lat:
-        lat.step(1)
+        lat.step(9)                     # pairs: rows of 97 values get their larger buffers here
         replay = captured(lat, 4, way)
         replay()
         lat.step(eager)
         replay()
         got = lat.get_f()
         lat.set_stream(None)
-    assert np.array_equal(got, single_steps(imex, shape, 1 + 4 + eager + 4))
+    assert np.array_equal(got, single_steps(imex, shape, 9 + 4 + eager + 4))
 
 
 @pytest.mark.parametrize("eager", [6, 8])
@@ -82,11 +82,11 @@ def test_batch_steps_between_replays(imex, eager):
 def test_eager_steps_still_pair_once_captured(imex, shape):
     """Steps of a captured lattice go two per launch where that keeps the buffer."""
     with make(imex, shape) as lat:
-        lat.step(1)
+        lat.step(9)
         captured(lat, 4, "step")
         before = lat.kernel_launches()
         lat.step(22)
         assert lat.kernel_launches() - before < 22
         got = lat.get_f()
         lat.set_stream(None)
-        assert np.array_equal(got, single_steps(imex, shape, 23))
+        assert np.array_equal(got, single_steps(imex, shape, 31))
