@@ -50,7 +50,7 @@ struct Int128 {
 };
 
 // Sums over the block's threads, valid in thread 0.  The integers go down
-// the warp by shuffles; the float64 values through shared memory, where
+// the warp by shuffles; a float64 value through shared memory, where
 // warp 0 adds a fixed eight per lane before its own shuffles (1.6 float64
 // additions a thread instead of 5).
 struct BlockSum {
@@ -58,6 +58,20 @@ struct BlockSum {
     long long hi[kWarps][4];
     double ke[kThreads];
 };
+__device__ __forceinline__ double block_sum(double v, BlockSum& s)
+{
+    const int lane = threadIdx.x & 31;
+    s.ke[threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        v = s.ke[lane];
+#pragma unroll
+        for (int w = 1; w < kWarps; ++w) v += s.ke[w * 32 + lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    }
+    return v;
+}
 __device__ __forceinline__ void block_sum(Int128 (&m)[4], double& ke, BlockSum& s)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -66,26 +80,17 @@ __device__ __forceinline__ void block_sum(Int128 (&m)[4], double& ke, BlockSum& 
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
             m[q].add(__shfl_down_sync(0xffffffffu, m[q].lo, o), __shfl_down_sync(0xffffffffu, m[q].hi, o));
-    s.ke[threadIdx.x] = ke;
     if (lane == 0)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             s.lo[warp][q] = m[q].lo;
             s.hi[warp][q] = m[q].hi;
         }
-    __syncthreads();
-    if (warp == 0) {
-        double v = s.ke[lane];
+    ke = block_sum(ke, s);
+    if (threadIdx.x == 0)
 #pragma unroll
-        for (int w = 1; w < kWarps; ++w) v += s.ke[w * 32 + lane];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        ke = v;
-        if (lane == 0)
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                for (int w = 1; w < kWarps; ++w) m[q].add(s.lo[w][q], s.hi[w][q]);
-    }
+        for (int q = 0; q < 4; ++q)
+            for (int w = 1; w < kWarps; ++w) m[q].add(s.lo[w][q], s.hi[w][q]);
 }
 
 // value * 2^-61, rounded twice at most (the high word is exact).
@@ -100,15 +105,43 @@ __device__ __forceinline__ double to_double(Int128 v)
     return neg ? -d : d;
 }
 
-// A cell outside the fixed-point range: its float64 sums (src/lbm.cpp:271-294).
+// Sums of a thread's cells outside the fixed-point range, in local memory: those of
+// reduced precision in the wider range (moments_wide) as integers, the kinetic energy in
+// the other cells' units; the rest in float64.  Written from the first such cell on:
+// cleared at the start, by every thread, they cost 3 us at 128^3 (of 93).
+struct Outside {
+    Int128 m[4];
+    double ke, sums[5];
+    int any;  // float64 sums
+};
+
+// Adds such a cell (src/lbm.cpp:271-294).  The wider range covers lattices of densities of 2 to
+// thousands: in float64, on the pipe that the integers are there to leave alone, 256^3
+// float32 of density 1000 takes 3.9 ms, in integers 1.12.
 template <int P>
 __device__ __noinline__ void add_outside(const typename mom::Elem<P>::T* src, Geom g, int i, int j, int k, bool pull,
-                                         double* sums)
+                                         Outside* o, bool first)
 {
+    if (first) *o = Outside{};
+    if constexpr (P != IMEX_F64) {
+        const mom::WideMoments w = mom::moments_wide<P>(src, g, i, j, k, pull);
+        if (w.ok) {
+            constexpr double kVel = (double)(1ull << (mom::kWide + mom::kVelBits<P>)) * 0x1p-61;
+            for (int d = 0; d < 4; ++d)
+                o->m[d].add((unsigned long long)w.M[d] << mom::kWide, (long long)w.M[d] >> (64 - mom::kWide));
+            if (P == IMEX_F16DEV) o->m[0].add((long long)mom::weights_fixed());
+            for (int d = 1; d < 4; ++d) {
+                const double v = __ll2double_rn(w.M[d]) * kVel;
+                o->ke = fma(v, v, o->ke);
+            }
+            return;
+        }
+    }
     double m[4];
     mom::moments_f64_of<P>(src, g, i, j, k, pull, m);
-    for (int q = 0; q < 4; ++q) sums[q] += m[q];
-    sums[4] += 0.5 * (m[1] * m[1] + m[2] * m[2] + m[3] * m[3]);
+    for (int q = 0; q < 4; ++q) o->sums[q] += m[q];
+    o->sums[4] += 0.5 * (m[1] * m[1] + m[2] * m[2] + m[3] * m[3]);
+    o->any = 1;
 }
 
 template <int P, bool PULL, int MINB>
@@ -120,8 +153,9 @@ __global__ void __launch_bounds__(kThreads, MINB)
     __shared__ int s_last;
     chain_begin<true>();
     Int128 m[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-    double ke = 0.0, sums[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    int any = 0;
+    double ke = 0.0;
+    Outside outside;
+    bool met = false;  // a cell for it
     for (unsigned long long q = (unsigned long long)blockIdx.x * kThreads + threadIdx.x; q < cells;
          q += (unsigned long long)gridDim.x * kThreads) {
         int i, j, k;
@@ -134,25 +168,24 @@ __global__ void __launch_bounds__(kThreads, MINB)
 #pragma unroll
             for (int d = 0; d < 3; ++d) ke = fma(c.vel[d], c.vel[d], ke);
         } else {
-            any = 1;
-            add_outside<P>(src, g, i, j, k, PULL, sums);
+            add_outside<P>(src, g, i, j, k, PULL, &outside, !met);
+            met = true;
         }
+    }
+    if (P != IMEX_F64 && met) {
+#pragma unroll
+        for (int d = 0; d < 4; ++d) m[d].add(outside.m[d].lo, outside.m[d].hi);
+        ke += outside.ke;
     }
     block_sum(m, ke, s);
-    any = __syncthreads_or(any);
+    int any = __syncthreads_or(met && outside.any);
     Partial& mine = part[blockIdx.x];
-    if (any) {  // rare: the threads' float64 sums one after the other
+    if (any)
         for (int q = 0; q < 5; ++q) {
-            s.ke[threadIdx.x] = sums[q];
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double v = 0.0;
-                for (int t = 0; t < kThreads; ++t) v += s.ke[t];
-                mine.out[q] = v;
-            }
-            __syncthreads();
+            __syncthreads();  // s is read
+            const double v = block_sum(met ? outside.sums[q] : 0.0, s);
+            if (threadIdx.x == 0) mine.out[q] = v;
         }
-    }
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -180,16 +213,20 @@ __global__ void __launch_bounds__(kThreads, MINB)
     }
     block_sum(m, ke, s);
     any = __syncthreads_or(any);
+    double sums[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if (any)
+        for (int q = 0; q < 5; ++q) {
+            for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads)
+                if (__ldcg(&part[b].any_out)) sums[q] += __ldcg(&part[b].out[q]);
+            __syncthreads();  // s is read
+            sums[q] = block_sum(sums[q], s);
+        }
     if (threadIdx.x == 0) {
         constexpr double kUnit = 1.0 / (double)(1ull << mom::kVelBits<P>);
         double r[5];
         for (int q = 0; q < 4; ++q) r[q] = to_double(m[q]);
         r[4] = 0.5 * ((ke * kUnit) * kUnit);
-        if (any)
-            for (unsigned b = 0; b < gridDim.x; ++b)
-                if (__ldcg(&part[b].any_out))
-                    for (int q = 0; q < 5; ++q) r[q] += __ldcg(&part[b].out[q]);
-        for (int q = 0; q < 5; ++q) out[q] = r[q];
+        for (int q = 0; q < 5; ++q) out[q] = any ? r[q] + sums[q] : r[q];
         if (status)
             for (int q = 0; q < 2; ++q) reinterpret_cast<unsigned long long*>(out)[5 + q] = __ldcg(status + q);
         *ticket = 0;  // for the next launch

@@ -65,6 +65,14 @@ struct Cell {
 template <int P>
 inline constexpr int kVelBits = P == IMEX_F64 ? kBits : P == IMEX_F16DEV ? 12 : 0;
 
+// Sum of the 27 weights.
+__device__ __forceinline__ constexpr uint64_t weights_fixed()
+{
+    uint64_t w = 0;
+    for (int a = 0; a < kQ; ++a) w += lowp::weight_fixed(a);
+    return w;
+}
+
 // EXACT (reduced precision): the stored values summed exactly instead of in
 // float32; the velocities in units of 2^-61.
 template <int P, bool EXACT>
@@ -113,11 +121,8 @@ __device__ __forceinline__ bool moments(const typename Elem<P>::T* src, const Ge
             }
         }
         if constexpr (P == IMEX_F16DEV) {
-            uint64_t w = 0;
-#pragma unroll
-            for (int a = 0; a < kQ; ++a) w += lowp::weight_fixed(a);
             ok = ok && S < (int64_t)3 << 61;  // the weights' 2^61 more stays below 2^63
-            S += (int64_t)w;
+            S += (int64_t)weights_fixed();
         }
         c.M[0] = S;
 #pragma unroll
@@ -174,6 +179,47 @@ __device__ __noinline__ void moments_f64_of(const typename Elem<P>::T* src, Geom
             if (ex(a, d) == -1) out[1 + d] -= f;
         }
     }
+}
+
+// Reduced precision again with a wider range: the exact sums of the values (float16: of
+// the deviations, without the weights' part of 3p) in units of 2^-(61 - kWide), for densities up
+// to several thousand.  ok: every value is below 2^(kWide - 1) (rest) or
+// 2^(kWide - 3) in magnitude and a multiple of the unit (a float16 / 2^12 always is).
+constexpr int kWide = 12;
+struct WideMoments {
+    int64_t M[4];
+    bool ok;
+};
+template <int S, int LIM>
+__device__ __forceinline__ int64_t exact_of_float(float x, bool& ok)
+{
+    const uint32_t b = __float_as_uint(x), mant = (b & 0x007FFFFFu) | 0x00800000u;
+    const int over = 89 + S - (int)((b >> 23) & 255u);  // bits of the mantissa below the unit
+    ok = ok && (over <= 0 || (b << 1) == 0 || (over < 24 && (mant & ((1u << over) - 1u)) == 0));
+    return fixed_of_float<S, LIM>(x, ok);
+}
+template <int P>
+__device__ __forceinline__ WideMoments moments_wide(const typename Elem<P>::T* src, Geom g, int i, int j, int k, bool pull)
+{
+    constexpr int S = Elem<P>::kScaleLog2 + kWide;
+    const PullIndex pi(g, i, j, k, pull);
+    WideMoments w = {{0, 0, 0, 0}, true};
+#pragma unroll
+    for (int a = 0; a < kQ; ++a) {
+        float x;
+        if constexpr (P == IMEX_F32) x = load_state(src + pi.at_dyn(g, a));
+        else x = __half2float(load_state(src + pi.at_dyn(g, a)));
+        int64_t X;
+        if constexpr (P == IMEX_F32) X = a == 0 ? exact_of_float<S, 1>(x, w.ok) : exact_of_float<S, 3>(x, w.ok);
+        else X = a == 0 ? fixed_of_float<S, 1>(x, w.ok) : fixed_of_float<S, 3>(x, w.ok);
+        w.M[0] += X;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (ex(a, d) == 1) w.M[1 + d] += X;
+            if (ex(a, d) == -1) w.M[1 + d] -= X;
+        }
+    }
+    return w;
 }
 
 // (x, y, z) of a flat cell index (z fastest); lattices in device memory
