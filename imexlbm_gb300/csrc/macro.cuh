@@ -11,7 +11,7 @@
 // all: the difference of exact integers is exact, and largest among integers.
 // One kernel reads both lattices; two field kernels, 6 arrays between and a
 // float64 maximum took 7.3 / 8.9 / 10.3 ms at 256^3 (float64 / float32 / float16
-// against itself), this takes 0.89 / 1.07 / 1.07 (memory: 1.08 / 0.54 / 0.27).
+// against itself), this takes 1.09 / 1.03 / 1.07 (memory: 1.08 / 0.54 / 0.27).
 #pragma once
 
 #include "moments_fixed.cuh"
@@ -56,12 +56,19 @@ cudaError_t launch(bool pull, const void* src, const Geom& g, double* p, double*
     return cudaGetLastError();
 }
 
+// CTAs an SM holds, with the registers that two cells' sums and loads take, and a
+// grid of four turns of them. (Six CTAs an SM where four or five fit left a second
+// turn nearly empty, for one pair of formats or another as their registers came out:
+// 256^3 1.08 to 2.46 ms; now 0.96 to 1.09.  One turn 1.03 to 1.18,
+// four CTAs and four turns 0.98 to 1.12.)
+constexpr int kDiffCtas = 3;
+
 // max over cells and components of |u_a - u_b| and of |u_b|: res[0], res[1]
 // as integers in units of 2^-61; res[2], res[3] as float64 bit patterns over
 // the cells where either lattice is outside the fixed-point range (NaN
 // skipped, as fmax skips it).
 template <int PA, int PB>
-__global__ void __launch_bounds__(kThreads) k_velocity_diff(const typename mom::Elem<PA>::T* __restrict__ fa, bool pull_a,
+__global__ void __launch_bounds__(kThreads, kDiffCtas) k_velocity_diff(const typename mom::Elem<PA>::T* __restrict__ fa, bool pull_a,
                                                             const typename mom::Elem<PB>::T* __restrict__ fb, bool pull_b,
                                                             Geom g, unsigned cells, unsigned long long* __restrict__ res)
 {
@@ -81,7 +88,8 @@ __global__ void __launch_bounds__(kThreads) k_velocity_diff(const typename mom::
                 // a component is below 2.25 (18 values below 1/8), so a difference can pass
                 // the 4 at which the signed form ends
                 const int64_t x = ca.M[d], y = cb.M[d];
-                take(0, x < y ? (uint64_t)y - (uint64_t)x : (uint64_t)x - (uint64_t)y);
+                const uint64_t diff = (uint64_t)x - (uint64_t)y;
+                take(0, x < y ? 0 - diff : diff);
                 take(1, (uint64_t)(y < 0 ? -y : y));
             }
         } else {
@@ -108,7 +116,7 @@ cudaError_t launch_diff(const void* fa, bool pull_a, const void* fb, bool pull_b
                         cudaStream_t s)
 {
     if (g.plane > 0xffffffffull) return cudaErrorInvalidValue;
-    const unsigned need = (unsigned)((g.plane + kThreads - 1) / kThreads), most = (unsigned)current_sm_count() * 6;
+    const unsigned need = (unsigned)((g.plane + kThreads - 1) / kThreads), most = (unsigned)current_sm_count() * 4 * kDiffCtas;
     k_velocity_diff<PA, PB><<<need < most ? need : most, kThreads, 0, s>>>(
         static_cast<const typename mom::Elem<PA>::T*>(fa), pull_a, static_cast<const typename mom::Elem<PB>::T*>(fb), pull_b, g,
         (unsigned)g.plane, res);
