@@ -94,8 +94,11 @@ __global__ void __launch_bounds__(kThreads, kDiffCtas) k_velocity_diff(const typ
             }
         } else {
             double ma[4], mb[4];
-            mom::moments_f64_of<PA>(fa, g, i, j, k, pull_a, ma);
-            mom::moments_f64_of<PB>(fb, g, i, j, k, pull_b, mb);
+            // velocities alone: the float64 pipe bounds a lattice of such cells (256^3
+            // float32 of density 1000 against float64 4.8 ms; with the mass, and six CTAs an
+            // SM, 8.7; two field kernels and a maximum 8.1)
+            mom::moments_f64_of<PA, false>(fa, g, i, j, k, pull_a, ma);
+            mom::moments_f64_of<PB, false>(fb, g, i, j, k, pull_b, mb);
             for (int d = 1; d < 4; ++d) {
                 const double x = fabs(ma[d] - mb[d]), y = fabs(mb[d]);
                 if (x >= 0.0) take(2, (unsigned long long)__double_as_longlong(x));

@@ -159,8 +159,8 @@ __device__ __forceinline__ bool moments(const typename Elem<P>::T* src, const Ge
     return ok;
 }
 
-// The same moments in float64, for a cell outside the range.
-template <int P>
+// The same moments in float64, for a cell outside the range; out[0] only if MASS.
+template <int P, bool MASS = true>
 __device__ __noinline__ void moments_f64_of(const typename Elem<P>::T* src, Geom g, int i, int j, int k, bool pull,
                                             double* out)
 {
@@ -172,7 +172,7 @@ __device__ __noinline__ void moments_f64_of(const typename Elem<P>::T* src, Geom
         const auto v = load_state(src + pi.at_dyn(g, a));
         if constexpr (P == IMEX_F64) f = v;
         else f = lowp::Storage<P>::to_f64(v, a);
-        out[0] += f;
+        if (MASS) out[0] += f;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             if (ex(a, d) == 1) out[1 + d] += f;
