@@ -10,10 +10,13 @@
 // sums of a cell differ by less than kSlack, so no other cell can hold the
 // float64 extreme.  The cells are taken in chunks; a chunk with no such cell
 // ends at once, so k_pick is a few chunks' work unless a component is constant
-// to the last bits.  0.90 / 0.72 / 0.71 ms at 256^3 (memory: 0.54 / 0.27 / 0.14);
+// to the last bits.  0.62 / 0.67 / 0.67 ms at 256^3 (memory: 0.54 / 0.27 / 0.14);
 // with w = 0 everywhere, as in an initial flow in x and y, that one component
-// is summed again everywhere: 1.36 / 1.16 / 1.64.  A lattice uniform in all four is the
-// one slower for it in float64 (3.72).
+// is summed again everywhere: 1.33 / 1.20 / 1.81.  Of cells that repeat, as in a fluid at
+// rest, the first is summed (1.91 / 1.39 / 1.54; each of them 3.73 / 1.33 / 3.69, more
+// than the float64 sums of all in one kernel).  Cells outside the integers' range are
+// summed by k_extremes, where they are met: a lattice of density 1000 3.32 / 4.16 / 4.47
+// (in k_pick 3.94 / 4.58 / 5.26).
 #pragma once
 
 #include <cfloat>
@@ -43,9 +46,9 @@ __device__ __forceinline__ unsigned long long up(double d)
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 
-// Extremes of one chunk of cells, and whether it has cells outside the range.
+// Integer extremes of one chunk of cells.
 struct Chunk {
-    unsigned long long key[8], outside;
+    unsigned long long key[8];
 };
 // The whole lattice's: the integer extremes, and the float64 ones as keys.
 struct Result {
@@ -95,40 +98,6 @@ __device__ __forceinline__ unsigned long long block_largest(unsigned long long (
     if (threadIdx.x < 8)
         for (int w = 0; w < kThreads / 32; ++w) v = red[w][threadIdx.x] > v ? red[w][threadIdx.x] : v;
     return v;
-}
-
-template <int P, bool PULL>
-__global__ void __launch_bounds__(kThreads) k_extremes(const typename mom::Elem<P>::T* src, Geom g, Split s,
-                                                       Chunk* __restrict__ chunks, Result* __restrict__ res)
-{
-    __shared__ unsigned long long red[kThreads / 32][8];
-    chain_begin<false>();
-    unsigned long long best[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int outside = 0;
-    const unsigned begin = blockIdx.x * s.chunk, end = s.cells - begin < s.chunk ? s.cells : begin + s.chunk;
-    for (unsigned cell = begin + threadIdx.x; cell < end && cell >= begin; cell += kThreads) {
-        int i, j, k;
-        mom::cell_of(g, cell, i, j, k);
-        mom::Cell<P> c;
-        if (mom::moments<P, true>(src, g, PullIndex(g, i, j, k, PULL), c)) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const unsigned long long v = up(c.M[q]);
-                best[q] = v > best[q] ? v : best[q];
-                best[4 + q] = ~v > best[4 + q] ? ~v : best[4 + q];
-            }
-        } else {
-            outside = 1;
-        }
-    }
-    const unsigned long long v = block_largest(best, red);
-    outside = __syncthreads_or(outside);
-    if (threadIdx.x < 8) {
-        chunks[blockIdx.x].key[threadIdx.x] = v;
-        lift(&res->whole[threadIdx.x], v);
-    }
-    if (threadIdx.x == 0) chunks[blockIdx.x].outside = outside;
-    chain_end<false>();
 }
 
 template <int P>
@@ -195,6 +164,95 @@ __device__ __noinline__ bool sums_exact(const typename mom::Elem<P>::T* src, con
     }
 }
 
+// Whether cells c and d hold the same 27 values, so that their sums are the same:
+// in a fluid at rest all do.  Ends at the first difference.
+constexpr unsigned kNoCell = 0xffffffffu;
+template <int P>
+__device__ __noinline__ bool same_values(const typename mom::Elem<P>::T* src, Geom g, unsigned c, unsigned d, bool pull)
+{
+    int i, j, k;
+    mom::cell_of(g, c, i, j, k);
+    const PullIndex pc(g, i, j, k, pull);
+    mom::cell_of(g, d, i, j, k);
+    const PullIndex pd(g, i, j, k, pull);
+    bool same = true;
+#pragma unroll
+    for (int a = 0; a < kQ && same; ++a) {
+        const auto v = load_state(src + pc.at_dyn(g, a)), w = load_state(src + pd.at_dyn(g, a));
+        if constexpr (P == IMEX_F64) same = __double_as_longlong(v) == __double_as_longlong(w);
+        else if constexpr (P == IMEX_F32) same = __float_as_uint(v) == __float_as_uint(w);
+        else same = __half_as_ushort(v) == __half_as_ushort(w);
+    }
+    return same;
+}
+
+// Component q of a cell by the reference's comparisons: from -DBL_MAX and DBL_MAX on,
+// NaN skipped.
+__device__ __forceinline__ void take(unsigned long long* best, int q, double x)
+{
+    if (x > -DBL_MAX && up(x) > best[q]) best[q] = up(x);
+    if (x < DBL_MAX && ~up(x) > best[4 + q]) best[4 + q] = ~up(x);
+}
+
+// The float64 sums of a cell outside the range, for k_extremes, unless the thread's last such
+// cell (kNoCell: none yet) has the same; best lies in local memory, cleared by the first.
+template <int P>
+__device__ __noinline__ void take_outside(const typename mom::Elem<P>::T* src, Geom g, unsigned cell, unsigned last,
+                                          bool pull, unsigned long long* best)
+{
+    if (last == kNoCell) {
+        for (int q = 0; q < 8; ++q) best[q] = 0;
+    } else if (same_values<P>(src, g, cell, last, pull)) {
+        return;
+    }
+    double x[4];
+    int i, j, k;
+    mom::cell_of(g, cell, i, j, k);
+    mom::moments_f64_of<P>(src, g, i, j, k, pull, x);
+    x[0] *= 1.0 / 3.0;
+    for (int q = 0; q < 4; ++q) take(best, q, x[q]);
+}
+
+template <int P, bool PULL>
+__global__ void __launch_bounds__(kThreads) k_extremes(const typename mom::Elem<P>::T* src, Geom g, Split s,
+                                                       Chunk* __restrict__ chunks, Result* __restrict__ res)
+{
+    __shared__ unsigned long long red[kThreads / 32][8];
+    chain_begin<false>();
+    unsigned long long best[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    unsigned long long summed[8];  // of cells outside the range
+    unsigned last = kNoCell;       // the last of them
+    const unsigned begin = blockIdx.x * s.chunk, end = s.cells - begin < s.chunk ? s.cells : begin + s.chunk;
+    for (unsigned cell = begin + threadIdx.x; cell < end && cell >= begin; cell += kThreads) {
+        int i, j, k;
+        mom::cell_of(g, cell, i, j, k);
+        mom::Cell<P> c;
+        if (mom::moments<P, true>(src, g, PullIndex(g, i, j, k, PULL), c)) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const unsigned long long v = up(c.M[q]);
+                best[q] = v > best[q] ? v : best[q];
+                best[4 + q] = ~v > best[4 + q] ? ~v : best[4 + q];
+            }
+        } else {
+            take_outside<P>(src, g, cell, last, PULL, summed);
+            last = cell;
+        }
+    }
+    const unsigned long long v = block_largest(best, red);
+    if (threadIdx.x < 8) {
+        chunks[blockIdx.x].key[threadIdx.x] = v;
+        lift(&res->whole[threadIdx.x], v);
+    }
+    if (__syncthreads_or(last != kNoCell)) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) best[q] = last != kNoCell ? summed[q] : 0;
+        const unsigned long long w = block_largest(best, red);
+        if (threadIdx.x < 8) lift(&res->picked[threadIdx.x], w);
+    }
+    chain_end<false>();
+}
+
 template <int P, bool PULL>
 __global__ void __launch_bounds__(kThreads) k_pick(const typename mom::Elem<P>::T* src, Geom g, Split s,
                                                    const Chunk* __restrict__ chunks, Result* __restrict__ res)
@@ -204,7 +262,7 @@ __global__ void __launch_bounds__(kThreads) k_pick(const typename mom::Elem<P>::
     // least key of a cell to be summed; keys are far above 2 kSlack or 0 (no
     // in-range cell at all: none is compared)
     unsigned long long least[8];
-    bool any = __ldcg(&chunks[blockIdx.x].outside) != 0;
+    bool any = false;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const unsigned long long w = __ldcg(&res->whole[q]);
@@ -212,6 +270,9 @@ __global__ void __launch_bounds__(kThreads) k_pick(const typename mom::Elem<P>::
         any = any || __ldcg(&chunks[blockIdx.x].key[q]) >= least[q];
     }
     if (!any) return;  // the same in every thread
+    unsigned last = kNoCell;  // the last cell summed
+    int last_need = 0;
+    bool differ = false;      // a comparison failed: no more of them in this chunk (16 cells a thread)
     unsigned long long best[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const unsigned begin = blockIdx.x * s.chunk, end = s.cells - begin < s.chunk ? s.cells : begin + s.chunk;
     for (unsigned cell = begin + threadIdx.x; cell < end && cell >= begin; cell += kThreads) {
@@ -219,32 +280,36 @@ __global__ void __launch_bounds__(kThreads) k_pick(const typename mom::Elem<P>::
         mom::cell_of(g, cell, i, j, k);
         const PullIndex pi(g, i, j, k, PULL);
         mom::Cell<P> c;
-        const bool ok = mom::moments<P, true>(src, g, pi, c);
+        if (!mom::moments<P, true>(src, g, pi, c)) continue;  // k_extremes has summed it
         int need = 0;  // components to be summed
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const unsigned long long v = up(c.M[q]);
-            if (!ok || v >= least[q] || ~v >= least[4 + q]) need |= 1 << q;
+            if (v >= least[q] || ~v >= least[4 + q]) need |= 1 << q;
         }
         if (!need) continue;
         double x[4];
-        if (ok && sums_exact<P>(src, g, pi)) {
+        if (sums_exact<P>(src, g, pi)) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) x[q] = (double)c.M[q] * 0x1p-61;
-        } else if (need & (need - 1)) {
-            sum_all<P>(src, g, pi, x);
         } else {
-            x[0] = sum_one<P>(src, g, pi, __ffs(need) - 1);
-            x[1] = x[2] = x[3] = x[0];
+            if (need == last_need && !differ) {
+                if (same_values<P>(src, g, cell, last, PULL)) continue;
+                differ = true;
+            }
+            last = cell;
+            last_need = need;
+            if (need & (need - 1)) {
+                sum_all<P>(src, g, pi, x);
+            } else {
+                x[0] = sum_one<P>(src, g, pi, __ffs(need) - 1);
+                x[1] = x[2] = x[3] = x[0];
+            }
         }
         x[0] *= 1.0 / 3.0;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            if (need >> q & 1) {
-                // the reference's comparisons: from -DBL_MAX and DBL_MAX on, NaN skipped
-                if (x[q] > -DBL_MAX && up(x[q]) > best[q]) best[q] = up(x[q]);
-                if (x[q] < DBL_MAX && ~up(x[q]) > best[4 + q]) best[4 + q] = ~up(x[q]);
-            }
+            if (need >> q & 1) take(best, q, x[q]);
     }
     const unsigned long long v = block_largest(best, red);
     if (threadIdx.x < 8) lift(&res->picked[threadIdx.x], v);
