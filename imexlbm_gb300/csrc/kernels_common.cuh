@@ -35,7 +35,7 @@ inline int current_sm_count()
 // Chained launches: the kernels of a run of steps are launched with
 // programmatic stream serialization, so that a kernel's CTAs may take their
 // places while the one before it in the stream still runs, and only the
-// launch's own latency overlaps: about 3 us a step, whatever the size (float32
+// launch's own latency overlaps: 1.5 to 3 us a step (float32
 // 32^3 4.1 -> 2.3 us, 64^3 8.4 -> 6.5; float64 32^3 6.2 -> 4.6, 64^3 22.6 -> 20.0,
 // 131 x 77 x 90 69.5 -> 66.3; float16 64^3 8.8 -> 6.6).
 //
@@ -68,8 +68,11 @@ inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 blo
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
-// Whether a grid of `ctas` CTAs of the step kernels (5 to 7 per SM) runs in turns.
-inline bool chain_early(unsigned long long ctas) { return ctas > 8ull * (unsigned)current_sm_count(); }
+// Whether a grid of `threads` threads runs in turns on SMs that hold `resident` of them.
+inline bool chain_early(unsigned long long threads, unsigned resident)
+{
+    return threads > (unsigned long long)resident * (unsigned)current_sm_count();
+}
 
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

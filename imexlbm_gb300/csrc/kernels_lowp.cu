@@ -154,7 +154,7 @@ cudaError_t step_impl(int mode, const void* src, void* dst, const Geom& g, const
     case kModeFused: {
         if (g.plane > 0xffffffffull - flat::kCells) return cudaErrorInvalidValue;  // above device memory
         const unsigned grid = (unsigned)((g.plane + flat::kCells - 1) / flat::kCells);
-        const bool early = chain_early(grid);
+        const bool early = chain_early((unsigned long long)grid * flat::kThreads, 8 * flat::kThreads);  // five to seven CTAs an SM
         auto go = [&](auto kernel) { return launch_chained(kernel, grid, flat::kThreads, 0, s, a, b, g, cp); };
         auto of = [&](auto even, auto sr) {
             constexpr bool kEven = decltype(even)::value, kSr = decltype(sr)::value;
