@@ -956,7 +956,7 @@ bool graph_pairs_valid(const imex_batch* b)
 // Whether the captured graph still describes the launches: the same shapes
 // and kernels, and for the segment kernel the same segment count (its grid)
 // and the same group table (a pointer baked into the graph; upload_table
-// moves the table when a tick or a tuning candidate needs a larger one).
+// moves the table when a tick needs a larger one).
 bool graph_valid(const imex_batch* b, int K)
 {
     return b->graph && b->graph_k == K && graph_pairs_valid(b) && b->graph_shape.threads == b->shape.threads &&
