@@ -1,0 +1,37 @@
+"""Many tiny members in one segment kernel: a CTA finds its member among more
+than the 32 that a warp looks at together, with sizes that share segments' group
+entries or span several, members that stop early, and both formats."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def make(imex, q, f16):
+    shape = [(3, 2, 5), (8, 8, 8), (1, 7, 40), (6, 5, 4), (16, 9, 8)][q % 5] if q != 70 else (40, 41, 43)
+    lat = imex.LBM(*shape, 0.01 + 0.001 * (q % 7), 1.0, 0.05, precision=imex.IMEX_F16DEV if f16 and q % 3 == 0 else imex.IMEX_F32)
+    lat.initialize_phase(0.1 * q, 0.2, 0.3 * q)
+    return lat
+
+
+@pytest.mark.parametrize("members", [2, 33, 34, 66, 140])
+@pytest.mark.parametrize("f16", [False, True])
+def test_tiny_members(imex, members, f16):
+    lats = [make(imex, q, f16) for q in range(members)]
+    with imex.Batch(160) as b:
+        b.set_launch(128, 0, 0)
+        b.set_row_launch(-1)
+        for q, lat in enumerate(lats):
+            b.add(lat, -1 if q % 4 else 3)
+        b.step(2)
+        b.step(4)
+        b.synchronize()
+        for q, lat in enumerate(lats):
+            steps = 6 if q % 4 else 3
+            with make(imex, q, f16) as alone:
+                alone.set_launch(0, 1, 1)
+                alone.step(steps)
+                assert lat.steps_done() == steps
+                assert np.array_equal(lat.get_f(), alone.get_f()), q
+    for lat in lats:
+        lat.close()
