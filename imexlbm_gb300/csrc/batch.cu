@@ -132,7 +132,10 @@ __device__ __forceinline__ void batch_cell(const BatchEntry& e, unsigned local, 
 
 // Cells per segment of the one-CTA-per-segment cell kernel.
 constexpr int kUnitCells = flat::kCells, kUnitThreads = flat::kThreads;
-constexpr int kUnitGroup = 256;  // segments per entry of the member lookup table
+// Segments per entry of the member lookup table: few, since a CTA steps from the entry's member to
+// its own one load at a time, and tiny members share entries (64 of 8^3 with 256: 15.4 us a step,
+// with 8: 5.6; a warp looking at 32 members at once 5.7, but large members 0.3% slower).
+constexpr int kUnitGroup = 8;
 
 // Segments of a member.
 __host__ __device__ inline unsigned long long unit_count(unsigned long long cells)
@@ -144,9 +147,8 @@ __host__ __device__ inline unsigned long long unit_count(unsigned long long cell
 // cells per thread (flat_lowp.cuh, the one-lattice kernel's cell pairs).
 // Segment u belongs to the member whose first segment index `begin` is the
 // largest not above u; the member is found from group[u / kUnitGroup] (the
-// member holding segment u - u mod kUnitGroup) by looking forward, the same
-// for every thread of the CTA (one member after the other, 64 of 8^3 took 15 us a
-// step, now 5.7).  The grid covers the segments of the tick's
+// member holding segment u - u mod kUnitGroup) by stepping forward, the same
+// for every thread of the CTA.  The grid covers the segments of the tick's
 // members; a CUDA graph of these launches is captured again when that count
 // changes.  PF = IMEX_F32: every member is float32.
 template <int PF>
@@ -157,12 +159,7 @@ __global__ void __launch_bounds__(kUnitThreads) k_batch_units(const BatchHeader*
     const unsigned u = blockIdx.x;
     const int count = hdr->count;
     int m = group[u / kUnitGroup];
-    // 32 members at a time where it is not that one or the next
-    for (unsigned later = ~0u; later == ~0u && m + 1 < count && tab[m + 1].begin <= u;) {
-        const int q = m + 1 + (int)(threadIdx.x & 31);
-        later = __ballot_sync(~0u, q < count && tab[q].begin <= u);
-        m += __popc(later);
-    }
+    while (m + 1 < count && tab[m + 1].begin <= u) ++m;
     const BatchEntry& e = tab[m];
     if (s >= e.steps) return;
     const unsigned seg = u - (unsigned)e.begin;
