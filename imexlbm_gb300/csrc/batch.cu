@@ -251,13 +251,13 @@ __host__ __device__ inline size_t rows_table_bytes(int members)
 // the stage), ahead of the CTA barrier that ends the item before it; a
 // CTA's consecutive items usually belong to one member, so the entry is
 // looked up and loaded from global memory only when the member changes.
-template <int kDirBytes, int kMinBlocks>
+template <int kDirBytes, int kMinBlocks, bool kEarly = true>
 __global__ void __launch_bounds__(rowslp::kThreads, kMinBlocks)
     k_batch_rows(const RowsHeader* __restrict__ hdr, const BatchEntry* __restrict__ tab, int s, CollideF32 base,
                  int stages, int table_cap, WaitCtl wc)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    chain_begin<true>();
+    chain_begin<kEarly>();  // not early: the next launch comes in as the CTAs end
     const int count = hdr->count;
     if (count > table_cap) {  // the table would not fit the shared memory the launch has
         if (threadIdx.x == 0) atomicOr(wc.err, 2u);
@@ -443,6 +443,7 @@ struct imex_batch {
     RowShape rshape;
     int n_cell = 0, n_row = 0;  // members in each kernel (last uploaded table)
     int n_cell_f16 = 0;         // float16-deviation members in the cell kernel
+    unsigned long long row_cells = 0;  // cells of the row kernel's members
     int graph_steps = 0;  // K of the captured graph (0: no graph)
     cudaGraphExec_t graph = nullptr;
     int graph_k = 0;
@@ -573,8 +574,13 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
         // capacity below the member count, so that its refusal fires
         const int cap = test_fault_kind() == IMEX_TEST_FAULT_BATCH_TABLE ? b->n_row - 1 : b->capacity;
         const WaitCtl wc = make_wait_ctl(b->d_err);
-#define IMEX_BATCH_ROWS(D, M) \
-    return launch_chained(k_batch_rows<D, M>, grid, rowslp::kThreads, smem, b->stream, b->d_rhdr, b->d_rtab, s, base, \
+        // Let in early, the next launch's CTAs pile up on the SMs done first, which costs more
+        // than it brings while a CTA has few items: us a step early and not, float16 4 of 48^3 14.0,
+        // 13.1; 4 of 64^3 25.6, 22.3; 8 of 80^3 (4.1 M cells) 86.0, 85.2; 16 of 64^3 (4.2 M) 83.7, 84.3;
+        // 2 of 256^3 550.7, 557.6.  (The shape of the rule for such batches has the form.)
+        const bool early = b->row_cells >= 4150000;
+#define IMEX_BATCH_ROWS(...) \
+    return launch_chained(k_batch_rows<__VA_ARGS__>, grid, rowslp::kThreads, smem, b->stream, b->d_rhdr, b->d_rtab, s, base, \
                           rs.stages, cap, wc)
         switch (rs.dir_kb) {
         case 1:
@@ -583,7 +589,8 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
             break;
         case 2:
             if (one) IMEX_BATCH_ROWS(2048, 1);
-            else IMEX_BATCH_ROWS(2048, 2);
+            else if (early) IMEX_BATCH_ROWS(2048, 2);
+            else IMEX_BATCH_ROWS(2048, 2, false);
             break;
         case 4: IMEX_BATCH_ROWS(4096, 1); break;
         default: return cudaErrorInvalidValue;
@@ -796,6 +803,7 @@ int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& r
     const unsigned long long chunk = (unsigned long long)(sh.threads > 0 ? sh.threads : 256) * (sh.cpt > 0 ? sh.cpt : 1);
     unsigned long long begin = 0;
     unsigned ibegin = 0;
+    unsigned long long row_cells = 0;
     int n = 0, nr = 0, n16 = 0;
     for (size_t m = 0; m < b->members.size(); ++m) {
         if (!single(b, m)) continue;
@@ -818,6 +826,7 @@ int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& r
         e.B = B;
         e.pad = 0;
         if (B) {
+            row_cells += h->ncells;
             e.begin = 0;
             e.ibegin = ibegin;
             ibegin += (unsigned)((size_t)h->g.nx * rowslp::y_blocks(h->g.ny, B));
@@ -859,6 +868,7 @@ int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& r
     b->h_rhdr->count = nr;
     b->n_cell = n;
     b->n_row = nr;
+    b->row_cells = row_cells;
     b->n_cell_f16 = n16;
     B_CUDA(b, cudaMemcpyAsync(b->d_tab, b->h_tab, sizeof(BatchEntry) * (n ? n : 1), cudaMemcpyHostToDevice, b->stream),
            "cudaMemcpyAsync");
@@ -1006,6 +1016,8 @@ int imex_batch_create(int max_members, imex_batch** out)
         e = cudaFuncSetAttribute(k_batch_rows<2048, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_batch_rows<2048, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_batch_rows<2048, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_batch_rows<4096, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) {
