@@ -929,6 +929,19 @@ RowShape pick_rows(const imex_batch* b)
     return rows_fit(small, b->capacity) ? small : RowShape{-1, 0, 0, 1};
 }
 
+// The cell kernel's shape for the members left to it: one CTA per segment, two cells a thread; below a
+// cell for each thread of a CTA per SM the persistent kernel with one cell a thread, whose threads have
+// less to do one after the other.  us a step, segments and persistent: one float32 lattice of 16^3 4.40,
+// 3.63, 4 of 8^3 4.50, 3.98, 16 of 8^3 5.08, 4.18, 4 of 16^3 4.45, 4.33; float16 one 16^3 4.46, 4.30, 4 of 16^3
+// 4.39, 4.45; but float32 4 of 24^3 (55,000 cells) 5.29, 5.67.
+BatchShape pick_cells(const imex_batch* b)
+{
+    unsigned long long cells = 0;
+    for (size_t m = 0; m < b->members.size(); ++m)
+        if (single(b, m) && !rows_per_item(b->members[m], b->rshape)) cells += b->members[m]->ncells;
+    return cells && cells <= 128ull * b->sms ? BatchShape{128, 1, 8} : BatchShape{kUnitThreads, 0, 0};
+}
+
 // Capture K steps (s = 0..K-1) of the current shapes into a graph.
 int capture_graph(imex_batch* b, int K)
 {
@@ -1112,8 +1125,8 @@ int imex_batch_step(imex_batch* b, int nsteps)
     int rc = join_members(b);
     if (rc) return rc;
     pick_pairs(b);
-    if (!b->cells_pinned) b->shape = BatchShape{kUnitThreads, 0, 0};
     if (!b->rows_pinned) b->rshape = pick_rows(b);
+    if (!b->cells_pinned) b->shape = pick_cells(b);
     std::vector<int> tick(b->members.size());
     for (;;) {
         int64_t most = 0;
