@@ -781,16 +781,20 @@ int64_t owed(const imex_batch* b, size_t m, int64_t want)
     return left < 0 ? 0 : (left < want ? left : want);
 }
 
+// Whether the row kernel takes a member under row shape rs.
+bool takes_rows(const imex_lattice* h, const RowShape& rs)
+{
+    if (rs.stages <= 0 || (h->precision == IMEX_F32 && !rs.f32)) return false;
+    const size_t row_bytes = (size_t)h->g.nz * lattice_elem_size(h->precision);
+    return row_bytes % 16 == 0 && row_bytes <= (size_t)rs.dir_kb * 1024 && (size_t)h->g.nx * h->g.ny < 0x7fffffffu;
+}
+
 // Rows per work item of a member in the row kernel under shape rs
 // (rowslp::item_rows); 0 if the member stays in the cell kernel.
 int rows_per_item(const imex_lattice* h, const RowShape& rs)
 {
-    if (rs.stages <= 0 || (h->precision == IMEX_F32 && !rs.f32)) return 0;
-    const size_t row_bytes = (size_t)h->g.nz * lattice_elem_size(h->precision);
-    const size_t cap = (size_t)rs.dir_kb * 1024;
-    if (row_bytes % 16 || row_bytes > cap) return 0;
-    if ((size_t)h->g.nx * h->g.ny >= 0x7fffffffu) return 0;
-    return rowslp::item_rows(h->g.ny, h->g.nz, (int)lattice_elem_size(h->precision), (int)cap);
+    if (!takes_rows(h, rs)) return 0;
+    return rowslp::item_rows(h->g.ny, h->g.nz, (int)lattice_elem_size(h->precision), rs.dir_kb * 1024);
 }
 
 // Write the member tables for a tick where member m runs steps[m] fused
@@ -870,15 +874,18 @@ int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& r
     b->n_row = nr;
     b->row_cells = row_cells;
     b->n_cell_f16 = n16;
-    B_CUDA(b, cudaMemcpyAsync(b->d_tab, b->h_tab, sizeof(BatchEntry) * (n ? n : 1), cudaMemcpyHostToDevice, b->stream),
-           "cudaMemcpyAsync");
-    B_CUDA(b, cudaMemcpyAsync(b->d_hdr, b->h_hdr, sizeof(BatchHeader), cudaMemcpyHostToDevice, b->stream),
-           "cudaMemcpyAsync");
-    B_CUDA(b, cudaMemcpyAsync(b->d_rtab, b->h_rtab, sizeof(BatchEntry) * (nr ? nr : 1), cudaMemcpyHostToDevice,
-                              b->stream),
-           "cudaMemcpyAsync");
-    B_CUDA(b, cudaMemcpyAsync(b->d_rhdr, b->h_rhdr, sizeof(RowsHeader), cudaMemcpyHostToDevice, b->stream),
-           "cudaMemcpyAsync");
+    if (n) {  // (a kernel without members is not launched)
+        B_CUDA(b, cudaMemcpyAsync(b->d_tab, b->h_tab, sizeof(BatchEntry) * n, cudaMemcpyHostToDevice, b->stream),
+               "cudaMemcpyAsync");
+        B_CUDA(b, cudaMemcpyAsync(b->d_hdr, b->h_hdr, sizeof(BatchHeader), cudaMemcpyHostToDevice, b->stream),
+               "cudaMemcpyAsync");
+    }
+    if (nr) {
+        B_CUDA(b, cudaMemcpyAsync(b->d_rtab, b->h_rtab, sizeof(BatchEntry) * nr, cudaMemcpyHostToDevice, b->stream),
+               "cudaMemcpyAsync");
+        B_CUDA(b, cudaMemcpyAsync(b->d_rhdr, b->h_rhdr, sizeof(RowsHeader), cudaMemcpyHostToDevice, b->stream),
+               "cudaMemcpyAsync");
+    }
     // the pinned staging is reused next tick: wait until the copies are done
     B_CUDA(b, cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
     return IMEX_OK;
@@ -919,7 +926,7 @@ RowShape pick_rows(const imex_batch* b)
     unsigned long long cells = 0, wide = 0;
     for (size_t m = 0; m < b->members.size(); ++m) {
         const imex_lattice* h = b->members[m];
-        if (!single(b, m) || h->precision != IMEX_F16DEV || !rows_per_item(h, RowShape{2, 4, 1, 0})) continue;
+        if (!single(b, m) || h->precision != IMEX_F16DEV || !takes_rows(h, RowShape{2, 4, 1, 0})) continue;
         cells += h->ncells;
         if (h->g.nz >= 96) wide += h->ncells;
     }
@@ -938,7 +945,7 @@ BatchShape pick_cells(const imex_batch* b)
 {
     unsigned long long cells = 0;
     for (size_t m = 0; m < b->members.size(); ++m)
-        if (single(b, m) && !rows_per_item(b->members[m], b->rshape)) cells += b->members[m]->ncells;
+        if (single(b, m) && !takes_rows(b->members[m], b->rshape)) cells += b->members[m]->ncells;
     return cells && cells <= 128ull * b->sms ? BatchShape{128, 1, 8} : BatchShape{kUnitThreads, 0, 0};
 }
 
