@@ -605,7 +605,8 @@ int lattice_create(int nx, int ny, int nz, double tau, double rho0, double u0, i
 
     size_t arr = (size_t)kQ * h->ncells * elem_size(precision);
     const size_t plain = arr;
-    if (alone && precision == IMEX_F32 && two::padded_eligible(h->g) && two::worth_alone(h->g, current_sm_count())) {
+    if (alone && precision == IMEX_F32 && two::padded_eligible(h->g)) h->pairs_worth = two::worth_alone(h->g, current_sm_count());
+    if (h->pairs_worth > 0) {
         const size_t padded = kQ * two::padded_plane(h->g) * sizeof(float);
         if (claim_idle_room(2 * (padded - plain))) {
             h->idle_room = 2 * (padded - plain);

@@ -229,10 +229,14 @@ bool worth_alone(const Geom& g, int sms)
 {
     if (!eligible(g) && !padded_eligible(g)) return false;
     const bool plain = eligible(g);
-    const double pair =
-        kLaunchUs + (plain ? kIterationUs : kPaddedIterationUs) * (double)iterations(g, plan_for(g, sms), sms);
     const double singles = 2.0 * (double)g.plane * (plain ? kCellUs : kPaddedCellUs);
-    return pair < 0.97 * singles;
+    auto beats = [&](double its) {
+        return kLaunchUs + (plain ? kIterationUs : kPaddedIterationUs) * its < 0.97 * singles;
+    };
+    // no plan has fewer iterations than all the tiles' spread evenly (imex_create asks: the plan takes 40 us)
+    const Plan t = tiles_of(g);
+    const double least = std::max<double>(1 + kExtra, (double)t.nty * t.ntz * (g.nx + kExtra) / sms);
+    return beats(least) && beats((double)iterations(g, plan_for(g, sms), sms));
 }
 
 void cut_alone(Lattice* l, const Geom& g)
