@@ -574,11 +574,12 @@ cudaError_t launch_step(imex_batch* b, const BatchShape& sh, const RowShape& rs,
         // capacity below the member count, so that its refusal fires
         const int cap = test_fault_kind() == IMEX_TEST_FAULT_BATCH_TABLE ? b->n_row - 1 : b->capacity;
         const WaitCtl wc = make_wait_ctl(b->d_err);
-        // Let in early, the next launch's CTAs pile up on the SMs done first, which costs more
+        // Let in early, the next step's CTAs pile up on the SMs done first, which costs more
         // than it brings while a CTA has few items: us a step early and not, float16 4 of 48^3 14.0,
         // 13.1; 4 of 64^3 25.6, 22.3; 8 of 80^3 (4.1 M cells) 86.0, 85.2; 16 of 64^3 (4.2 M) 83.7, 84.3;
-        // 2 of 256^3 550.7, 557.6.  (The shape of the rule for such batches has the form.)
-        const bool early = b->row_cells >= 4150000;
+        // 2 of 256^3 550.7, 557.6.  (The shape of the rule for such batches has the form.)  What comes
+        // in is the two-step kernel where there is one: early, its set-up overlaps.
+        const bool early = b->row_cells >= 4150000 || b->n_pair > 0;
 #define IMEX_BATCH_ROWS(...) \
     return launch_chained(k_batch_rows<__VA_ARGS__>, grid, rowslp::kThreads, smem, b->stream, b->d_rhdr, b->d_rtab, s, base, \
                           rs.stages, cap, wc)

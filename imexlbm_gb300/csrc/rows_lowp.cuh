@@ -315,9 +315,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
                 int stages, WaitCtl wc)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    // the next launch comes in as this one's CTAs end, not before: its CTAs would pile up on the
-    // SMs done first (112^3 early 31.0 us, 30.0 so; 128^3 42.3, 41.9; 192^3 130.2, 129.0; 256^3 276.9, 277.0)
-    chain_wait();
+    chain_begin<true>();  // the ring leaves the next launch's CTAs no room before this one's end
     const int yblocks = y_blocks(g.ny, B);
     const int items = g.nx * yblocks;
     const int G = gridDim.x;
