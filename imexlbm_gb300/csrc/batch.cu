@@ -860,11 +860,10 @@ int upload_table(imex_batch* b, const std::vector<int>& steps, const RowShape& r
             B_CUDA(b, cudaMallocHost((void**)&b->h_group, cap * sizeof(int)), "cudaMallocHost");
             b->group_cap = cap;
         }
-        int m = 0;
-        for (size_t q = 0; q < groups; ++q) {
-            const unsigned long long u = (unsigned long long)q * kUnitGroup;
-            while (m + 1 < n && b->h_tab[m + 1].begin <= u) ++m;
-            b->h_group[q] = m;
+        for (int m = 0; m < n; ++m) {  // the entries whose first segment is member m's
+            const size_t from = (size_t)((b->h_tab[m].begin + kUnitGroup - 1) / kUnitGroup),
+                         to = m + 1 < n ? (size_t)((b->h_tab[m + 1].begin + kUnitGroup - 1) / kUnitGroup) : groups;
+            std::fill(b->h_group + from, b->h_group + to, m);
         }
         B_CUDA(b, cudaMemcpyAsync(b->d_group, b->h_group, groups * sizeof(int), cudaMemcpyHostToDevice, b->stream),
                "cudaMemcpyAsync");
