@@ -128,7 +128,10 @@ int imex_conserved(imex_lattice *h, double out[5]);
 
 /* Per-cell macroscopic fields p = sum f / 3 and (u, v, w) = sum f e, each
  * nx*ny*nz float64 on the host.  Replaces LBM::ComputeMacroscopic()
- * (src/lbm.cpp:213-240).  Any output pointer may be NULL. */
+ * (src/lbm.cpp:213-240).  Any output pointer may be NULL.  The sums are exact
+ * and rounded once; imex_minmax_uvwp and imex_write_tecplot keep the
+ * reference's order of float64 sums, so that their values can differ from
+ * these in the last place. */
 int imex_macroscopic(imex_lattice *h, double *p, double *u, double *v, double *w);
 
 /* Largest velocity difference between two lattices of the same size on
@@ -160,10 +163,10 @@ int imex_profile_read(imex_lattice *h, imex_phase_stats out[IMEX_NPHASE], int re
 
 /* Extremes of the macroscopic fields: out = {umax, vmax, wmax, pmax, umin,
  * vmin, wmin, pmin} over all cells, with p = sum f / 3 and (u, v, w) =
- * sum f e as ComputeMacroscopic forms them.  The "minmax_uvwp" reduction of
+ * sum f e in the reference's order of float64 sums (imex_macroscopic).  The "minmax_uvwp" reduction of
  * LBM::MPIoutput (src/lbm.cpp:351-372), in its reducer order; NaN values
  * are skipped and an all-NaN field gives -DBL_MAX / DBL_MAX, the
- * reduction's identities.  One fused pass over f, no field arrays.
+ * reduction's identities.  No field arrays.
  * Synchronises. */
 int imex_minmax_uvwp(imex_lattice *h, double out[8]);
 
@@ -340,7 +343,10 @@ int imex_batch_synchronize(imex_batch *b);
  * cells_per_thread 0 with threads 128 - one CTA per 256-cell segment of
  * every member, the one-lattice kernel's grid over the whole batch (its
  * CUDA graph is captured again when the members' segment count changes).
- * threads = 0 leaves it to the rule again. */
+ * threads = 0 leaves it to the rule again.  The rule takes {128, 1, 8} while
+ * the kernel's members have fewer than 128 cells per SM and {128, 0, 0}
+ * otherwise; the other shapes, at best a few percent faster on some batches and
+ * slower on most, are for callers who compare them.  A refused call changes nothing. */
 int imex_batch_set_launch(imex_batch *b, int threads, int cells_per_thread, int ctas_per_sm);
 int imex_batch_get_launch(imex_batch *b, int out[3]);
 
@@ -351,7 +357,10 @@ int imex_batch_get_launch(imex_batch *b, int out[3]);
  * fits), resident CTAs per SM, and whether float32 members join it
  * (float32_members != 0) or stay in the cell kernel.  stages 0 leaves
  * it to the rule (default); -1 turns the row kernel off, so every member runs in the cell
- * kernel.  With either shape pinned no member steps twice per launch.
+ * kernel.  With either shape pinned no member steps twice per launch.  The
+ * rule takes {2, 2, 2} or {2, 4, 1}, and float16 members only; the other
+ * shapes, and float32 members in this kernel, are for callers who compare
+ * them.  A refused call changes nothing.
  * imex_batch_get_row_launch gives {stages, dir_kb, ctas_per_sm,
  * float32_members} (stages -1 when the rule keeps every member in the cell
  * kernel). */
@@ -362,7 +371,8 @@ int imex_batch_get_row_launch(imex_batch *b, int out[4]);
  * directly). */
 int imex_batch_set_graph(imex_batch *b, int steps_per_graph);
 
-/* Kernel launches issued by the batch (one per batched step). */
+/* Kernel launches issued by the batch (each of its kernels one per step, or
+ * per two steps). */
 int64_t imex_batch_kernel_launches(const imex_batch *b);
 const char *imex_batch_last_error(const imex_batch *b);
 
