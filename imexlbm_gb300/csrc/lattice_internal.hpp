@@ -66,7 +66,8 @@ struct imex_lattice {
     bool shape_pinned = false;  // shape set by imex_set_launch rather than the autotuner
     imex::two::LatticePtr pairs;  // two float32 steps per launch (two_f32.hpp), made on first use
     int pairs_worth = -1;         // whether they pay for this lattice alone (-1: not asked yet)
-    bool captured = false;        // float32: steps of this handle were captured into a graph
+    bool may_pair = false;        // alone or in a batch it may take two steps per launch
+    bool captured = false;        // may_pair: steps of this handle were captured into a graph
     bool padded_room = false;     // the buffers have room for the padded layout (two_f32.hpp)
     size_t idle_room = 0;         // bytes of it while it was never used
     imex::PhaseTimer prof;      // per-phase device time (imex_profile_*)
